@@ -39,27 +39,27 @@ def listed():
 
     return [
         # the smallest step there is: three tiny layers in float32, bound by launches and latency
-        case("tiny decode, 4 requests", kind="qwen3", model="tiny", layers=3, dtype="float32", decodes=4, low=17, high=40, prompts=0, tokens=0, start=0),
+        case("tiny decode 4", kind="qwen3", model="tiny", layers=3, dtype="float32", decodes=4, low=17, high=40, prompts=0, tokens=0, start=0),
         # one person's chat: one request decoding on the whole 8B model
-        case("8B decode, 1 request", kind="qwen3", model="8b", layers=36, dtype="bfloat16", decodes=1, low=2048, high=2048, prompts=0, tokens=0, start=0),
+        case("8B decode 1", kind="qwen3", model="8b", layers=36, dtype="bfloat16", decodes=1, low=2048, high=2048, prompts=0, tokens=0, start=0),
         # the engine's headline: eight requests at one context
-        case("8B decode, 8 requests", kind="qwen3", model="8b", layers=36, dtype="bfloat16", decodes=8, low=2048, high=2048, prompts=0, tokens=0, start=0),
+        case("8B decode 8", kind="qwen3", model="8b", layers=36, dtype="bfloat16", decodes=8, low=2048, high=2048, prompts=0, tokens=0, start=0),
         # a full server: 64 requests of all lengths
-        case("8B decode, 64 requests", kind="qwen3", model="8b", layers=36, dtype="bfloat16", decodes=64, low=300, high=3000, prompts=0, tokens=0, start=0),
+        case("8B decode 64", kind="qwen3", model="8b", layers=36, dtype="bfloat16", decodes=64, low=300, high=3000, prompts=0, tokens=0, start=0),
         # long conversations on the largest shape: eight query heads a kv head, the cache as large as the weights
-        case("32B decode, long contexts", kind="qwen3", model="32b", layers=6, dtype="bfloat16", decodes=13, low=6000, high=12000, prompts=0, tokens=0, start=0),
+        case("32B decode long", kind="qwen3", model="32b", layers=6, dtype="bfloat16", decodes=13, low=6000, high=12000, prompts=0, tokens=0, start=0),
         # a whole prompt in one step
-        case("8B prompt of 2,048", kind="qwen3", model="8b", layers=36, dtype="bfloat16", decodes=0, low=0, high=0, prompts=1, tokens=2048, start=0),
+        case("8B prompt 2048", kind="qwen3", model="8b", layers=36, dtype="bfloat16", decodes=0, low=0, high=0, prompts=1, tokens=2048, start=0),
         # short questions arriving together
-        case("8B, 3 short prompts", kind="qwen3", model="8b", layers=36, dtype="bfloat16", decodes=0, low=0, high=0, prompts=3, tokens=117, start=0),
+        case("8B short prompts", kind="qwen3", model="8b", layers=36, dtype="bfloat16", decodes=0, low=0, high=0, prompts=3, tokens=117, start=0),
         # chunked prefill: a portion of a long prompt beside 32 decoding requests, the budget of 512 full
-        case("14B portion and 32 decodes", kind="qwen3", model="14b", layers=12, dtype="bfloat16", decodes=32, low=400, high=1800, prompts=1, tokens=480, start=960),
+        case("14B portion and decodes", kind="qwen3", model="14b", layers=12, dtype="bfloat16", decodes=32, low=400, high=1800, prompts=1, tokens=480, start=960),
         # a portion deep in a long prompt, at the default budget, with nothing beside it
-        case("8B portion of 512 at 7,000", kind="qwen3", model="8b", layers=36, dtype="bfloat16", decodes=0, low=0, high=0, prompts=1, tokens=512, start=7000),
+        case("8B portion at 7000", kind="qwen3", model="8b", layers=36, dtype="bfloat16", decodes=0, low=0, high=0, prompts=1, tokens=512, start=7000),
         # the float32 path that checks the other one, at full width
-        case("8B layers in float32", kind="qwen3", model="8b", layers=2, dtype="float32", decodes=0, low=0, high=0, prompts=1, tokens=300, start=0),
+        case("8B float32", kind="qwen3", model="8b", layers=2, dtype="float32", decodes=0, low=0, high=0, prompts=1, tokens=300, start=0),
         # drawing the next token of 48 requests whose clients ask for different settings
-        case("sampling, 48 requests", kind="sample", vocab=151936, rows=48, settings="default nucleus greedy"),
+        case("sampling 48", kind="sample", vocab=151936, rows=48, settings="default nucleus greedy"),
     ]
 
 
