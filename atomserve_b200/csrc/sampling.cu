@@ -1,4 +1,4 @@
-// Sampling on the device, one block per row of float32 logits [B, V].
+// Sampling on the device: a cluster of eight blocks per row of float32 logits [B, V].
 //
 // The rules are the reference sampler's (atomserve/sampler.py:82-129): top-k on the raw
 // logits (0 or >= V keeps all; temperature 0 is the single best), divide by the temperature,
@@ -8,24 +8,39 @@
 // separate scatter that runs first (atomserve/sampler.py:144-168).
 //
 // The reference sorts (torch.topk, or its 1024-thread Metal kernel, atomserve/kernels.py:336-435).
-// Here nothing is sorted: the k-th largest logit is found by a radix select on order-preserving
-// integer keys (four 8-bit digits, counting histograms in shared memory), and the top-p cut
+// Here a whole row is never sorted: the k-th largest logit is found by a radix select on order-preserving
+// integer keys (digits of 11, 11 and 10 bits, counting histograms in shared memory), and the top-p cut
 // by the same walk over histograms of probability mass, kept as 64-bit fixed point so that
 // the sums do not depend on the order of the atomic additions. Ties at a cut are broken towards
-// the lower token id, by a third select over the ids. When top-k leaves at most 1024
-// candidates they are compacted into shared memory and the later passes read only those.
+// the lower token id, by a further select over the ids. When top-k leaves at most 1024
+// candidates they are gathered into one block's shared memory and ranked there.
+//
+// What bounds it: a row of 151,936 logits is 600 KB, and with one block a row every one of
+// seven passes over it moved at the rate of one SM. Here each block of the cluster brings its eighth of the row
+// into shared memory once (76 KB, two blocks an SM) and all passes read it there; what is left is the
+// chain of passes with two cluster barriers each. Measured, 1 / 48 rows of 151,936: temperature 0.6, top-k 20, top-p
+// 0.95 122 / 124 -> 17 / 40 us; top-p 0.95 alone 371 / 480 -> 35 / 87 us; argmax 8.8 / 8.8 -> 3.8 / 6.5 us. An eighth and not a quarter, because rows in flight on the
+// device are the same (74 KB x 2 against 148 KB x 1 an SM) while a pass takes half as long.
 //
 // Random numbers are Philox-4x32-10 keyed by the row's seed; the counter is (token id, the
 // row's draw counter). A seeded request passes its own seed and counts its own draws, so what
 // it draws does not depend on its neighbours in the batch (atomserve/sampler.py:123-127).
+#include <cooperative_groups.h>
+
 #include "common.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace {
 
-constexpr int kThreads = 1024;
-constexpr int kBins = 256;
-constexpr int kHistCopies = 8;
+constexpr int kThreads = 512;
+constexpr int kWarps = kThreads / 32;
+constexpr int kCluster = 8;                      // blocks a row
+constexpr int kBins = 2048;                      // an 11-bit digit
+constexpr int kSegment = kBins / kCluster;       // bins whose totals one block forms
 constexpr int kCompact = 1024;
+constexpr int kMaxSlice = 48 * 1024;             // floats of a row that a block can hold in shared memory
+constexpr int kSplitSlice = 65535;               // most elements whose masses two 32-bit words can add up (see Scratch)
 
 __device__ __forceinline__ uint32_t order_key(float f) {
   const uint32_t u = __float_as_uint(f);
@@ -52,177 +67,241 @@ struct Philox {
   }
 };
 
-// A row as the passes see it: the full logits (id == position) or the compacted candidates.
-struct RowView {
+// A block's share of a row: `n` values from token `first` on, in shared memory where they fit, else in place.
+struct Slice {
   const float* val;
-  const int* id;  // null: identity
-  int n;
-  __device__ __forceinline__ float value(int i) const { return val[i]; }
-  __device__ __forceinline__ int token(int i) const { return id ? id[i] : i; }
+  int first, n;
+};
+
+struct Best {
+  float score;
+  int token;
+  __device__ __forceinline__ void take(float s, int t) {
+    if (s > score || (s == score && t < token)) { score = s; token = t; }
+  }
 };
 
 struct Scratch {
-  unsigned long long hist[kHistCopies][kBins];
-  float red[32];
-  int red_i[32];
-  unsigned long long bcast[4];
-  float cand_val[kCompact];
-  int cand_id[kCompact];
+  // A digit's histogram. Counts: word[0]. Masses, at most 2^32 each: the low 16 bits of each are added up in
+  // word[0] and the rest in word[1] (both native 32-bit atomics; 64-bit ones in shared memory are loops), which
+  // holds for up to kSplitSlice elements; otherwise, and where a mass may be out of that range (a row with an
+  // infinity on top or a NaN), 64-bit words.
+  union {
+    unsigned int word[2][kBins];
+    unsigned long long wide[kBins];
+  } hist;
+  unsigned long long total[kSegment];  // over the cluster, of this block's segment of the bins
+  unsigned long long segment_sum;
+  unsigned long long warp_part[kWarps];  // a sum being formed over the block
+  int odd;                               // this block's slice holds a NaN
+  Best best[2], warp_best[kWarps];  // [0]: the largest logit, [1]: the winner of the race
+  unsigned long long found[4];
   int cand_n;
+  __align__(16) uint32_t cand_key[kCompact];
+  __align__(16) int cand_id[kCompact];
+  uint32_t sorted_key[kCompact];
+  int sorted_id[kCompact];
 };
 
-// Calls f(i, value, valid) for every element of the row, the same number of times in every
-// thread of the block (valid false: no such element), so that f may use warp-wide ballots. The
-// full row is read with 16-byte loads, four in flight per thread; one scalar load per trip would
-// leave a row of 150,000 logits bound by the latency of its loads.
+__device__ __forceinline__ float key_value(uint32_t key) {
+  return __uint_as_float((key & 0x80000000u) ? (key & 0x7fffffffu) : ~key);
+}
+
+// Calls f(token, value) for every element of the slice; 16-byte reads, four elements a thread at a time.
 template <typename F>
-__device__ __forceinline__ void for_each_value(const RowView& row, F f) {
+__device__ __forceinline__ void for_each_value(const Slice& row, F f) {
   int done = 0;
-  if (row.id == nullptr && ((uintptr_t)row.val & 15) == 0) {
+  if (((uintptr_t)row.val & 15) == 0) {
     const float4* v4 = reinterpret_cast<const float4*>(row.val);
     const int n4 = row.n >> 2;
-    for (int base = 0; base < n4; base += blockDim.x * 4) {
-      float4 x[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int at = base + threadIdx.x + u * blockDim.x;
-        x[u] = at < n4 ? v4[at] : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int at = base + threadIdx.x + u * blockDim.x;
-        const float e[4] = {x[u].x, x[u].y, x[u].z, x[u].w};
-#pragma unroll
-        for (int k = 0; k < 4; ++k) f(at * 4 + k, e[k], at < n4);
-      }
+#pragma unroll 2
+    for (int i = threadIdx.x; i < n4; i += kThreads) {
+      const float4 x = v4[i];
+      const int t = row.first + 4 * i;
+      f(t, x.x);
+      f(t + 1, x.y);
+      f(t + 2, x.z);
+      f(t + 3, x.w);
     }
     done = n4 << 2;
   }
-  for (int base = done; base < row.n; base += blockDim.x) {
-    const int i = base + threadIdx.x;
-    const bool valid = i < row.n;
-    f(i, valid ? row.value(i) : 0.f, valid);
-  }
+  for (int i = done + threadIdx.x; i < row.n; i += kThreads) f(row.first + i, row.val[i]);
 }
 
-// Descending radix select over 32-bit keys. `item(i, value, key, weight)` says whether element i takes
-// part, its key and its non-negative integer weight. Finds the largest key c such that the
+// The best over the block, then over the cluster: every thread of every block gets it. `slot`: which of the
+// scratch's two (each is used once a kernel, so no barrier keeps a second use from a slow reader).
+__device__ Best cluster_best(const cg::cluster_group& cluster, Scratch& s, Best b, int slot) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float os = __shfl_xor_sync(0xffffffffu, b.score, o);
+    const int ot = __shfl_xor_sync(0xffffffffu, b.token, o);
+    b.take(os, ot);
+  }
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) s.warp_best[threadIdx.x >> 5] = b;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < kWarps; ++w) b.take(s.warp_best[w].score, s.warp_best[w].token);
+    s.best[slot] = b;
+  }
+  cluster.sync();
+  b = s.best[slot];
+#pragma unroll
+  for (int c = 0; c < kCluster; ++c) {
+    const Best o = *cluster.map_shared_rank(&s.best[slot], c);
+    b.take(o.score, o.token);
+  }
+  return b;
+}
+
+// Descending radix select over 32-bit keys of the cluster's row. `item(token, value, key)` says whether an
+// element takes part, and its key; `weight(value)` is its non-negative integer weight, worked out only for elements
+// that a digit's histogram counts. `target_of(total)` gives the target once the first histogram has told the total
+// weight (which so needs no pass of its own). Finds the largest key c such that the
 // weight of all taking-part elements with key > c is < target <= that weight plus the weight
-// of key == c. Returns c, and in `above` the weight strictly above c. (With weight 1 and
-// target k this is the k-th largest key.) If the total weight is below target, returns 0 with
+// of key == c. Returns c, and in `above` the weight strictly above c, in `equal` that of key == c. (With weight 1
+// and target k this is the k-th largest key.) If the total weight is below target, returns 0 with
 // `above` = total: everything is kept.
 //
-// `last_shift` 16 stops after the two high digits: the result then has its low 16 bits clear and
-// names a bin of 65,536 keys, `above` and `equal` counting what lies above and inside it.
+// `digits` 1 or 2 stops after that many: the result then has its low bits clear and names a range of keys,
+// `above` and `equal` counting what lies above and inside it.
 //
-// A whole row's first digit falls into a handful of bins (sign and exponent of logits that lie
-// close together), so lanes of a warp that hit the same bin hand their weight to one of them
-// before the atomic addition: up to three such groups a warp, the rest add for themselves.
-//
-// kUnit: every weight is 1 (a count). A group's weight is then its number of lanes, and the
-// histograms are 32-bit, whose shared-memory atomics are native (64-bit ones are not).
-template <bool kUnit, typename Item>
-__device__ uint32_t radix_select(const RowView& row, Scratch& s, unsigned long long target,
-                                 unsigned long long* above, unsigned long long* equal, Item item,
-                                 int last_shift = 0) {
+// kUnit: every weight is 1 (a count). `wide`: weights added up in 64-bit words (see Scratch).
+template <bool kUnit, typename Item, typename Weight, typename Target>
+__device__ uint32_t cluster_select(const cg::cluster_group& cluster, const Slice& row, Scratch& s, Target target_of,
+                                   unsigned long long* above, unsigned long long* equal, bool wide, int digits, Item item,
+                                   Weight weight) {
   uint32_t prefix = 0, mask = 0;
-  unsigned long long acc = 0;
-  const int lane = threadIdx.x & 31;
-  for (int shift = 24; shift >= last_shift; shift -= 8) {
-    for (int i = threadIdx.x; i < kHistCopies * kBins; i += blockDim.x) (&s.hist[0][0])[i] = 0ull;
+  unsigned long long acc = 0, target = 0;
+  const int rank = (int)cluster.block_rank(), lane = threadIdx.x & 31;
+  for (int digit = 0; digit < digits; ++digit) {
+    const int shift = digit == 0 ? 21 : (digit == 1 ? 10 : 0);
+    const uint32_t bins = digit == 2 ? 1024u : 2048u;
+    for (int i = threadIdx.x; i < kBins; i += kThreads) s.hist.wide[i] = 0ull;
     __syncthreads();
-    unsigned long long* h = s.hist[(threadIdx.x >> 5) % kHistCopies];
-    unsigned int* h32 = reinterpret_cast<unsigned int*>(h);  // kUnit: the copy's first 256 words
-    for_each_value(row, [&](int i, float v, bool valid) {
+    for_each_value(row, [&](int token, float v) {
       uint32_t key = 0;
-      unsigned long long w = 0;
-      bool take = valid && item(i, v, key, w) && (key & mask) == prefix && w;
-      const uint32_t bin = (key >> shift) & 255u;
-      unsigned remaining = __ballot_sync(0xffffffffu, take);
-      for (int round = 0; round < 3 && remaining; ++round) {
-        const int leader = __ffs(remaining) - 1;
-        const uint32_t leader_bin = __shfl_sync(0xffffffffu, bin, leader);
-        const bool mine = take && bin == leader_bin;
-        const unsigned group = __ballot_sync(0xffffffffu, mine);
-        if (kUnit) {
-          if (lane == leader) atomicAdd(&h32[leader_bin], (unsigned int)__popc(group));
-        } else {
-          unsigned long long sum = mine ? w : 0ull;
-          if (group & (group - 1))  // more than one lane in the group (the whole warp agrees)
-            for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-          if (lane == leader) atomicAdd(&h[leader_bin], sum);
-        }
-        if (mine) take = false;
-        remaining &= ~group;
+      if (!item(token, v, key) || (key & mask) != prefix) return;
+      const uint32_t bin = (key >> shift) & (bins - 1u);
+      if (kUnit) {
+        atomicAdd(&s.hist.word[0][bin], 1u);
+        return;
       }
-      if (take) {
-        if (kUnit) atomicAdd(&h32[bin], 1u);
-        else atomicAdd(&h[bin], w);
+      const unsigned long long w = weight(v);
+      if (wide) {
+        if (w) atomicAdd(&s.hist.wide[bin], w);
+      } else {
+        const unsigned int lo = (unsigned int)w & 0xffffu, hi = (unsigned int)(w >> 16);
+        if (lo) atomicAdd(&s.hist.word[0][bin], lo);
+        if (hi) atomicAdd(&s.hist.word[1][bin], hi);
       }
     });
+    cluster.sync();
+    // this block's segment of the bins, over the cluster
+    if (threadIdx.x < kSegment) {
+      const int bin = rank * kSegment + threadIdx.x;
+      unsigned long long t = 0;
+#pragma unroll
+      for (int c = 0; c < kCluster; ++c) {
+        const Scratch* o = cluster.map_shared_rank(&s, c);
+        if (kUnit) t += o->hist.word[0][bin];
+        else if (wide) t += o->hist.wide[bin];
+        else t += (unsigned long long)o->hist.word[0][bin] + ((unsigned long long)o->hist.word[1][bin] << 16);
+      }
+      s.total[threadIdx.x] = t;
+      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      if (lane == 0) s.warp_part[threadIdx.x >> 5] = t;
+    }
     __syncthreads();
-    unsigned long long bin_total = 0;
-    if (threadIdx.x < kBins)
-      for (int c = 0; c < kHistCopies; ++c)
-        bin_total += kUnit ? (unsigned long long)reinterpret_cast<const unsigned int*>(s.hist[c])[threadIdx.x] : s.hist[c][threadIdx.x];
-    __syncthreads();  // copy 0's 32-bit words lie where the 64-bit totals are written next
-    if (threadIdx.x < kBins) s.hist[0][threadIdx.x] = bin_total;
-    __syncthreads();
+    if (threadIdx.x == 0) {
+      unsigned long long t = 0;
+      for (int w = 0; w < kSegment / 32; ++w) t += s.warp_part[w];
+      s.segment_sum = t;
+    }
+    cluster.sync();
     if (threadIdx.x < 32) {
-      // The first bin, from the top, at which the weight so far reaches the target: lane l walks
-      // bins 255 - 8l downwards, after a scan over the lanes has told it the weight above them.
-      unsigned long long mine[8], lane_sum = 0;
+      // the segment, from the top, in which the weight so far reaches the target, then the bin within it: lane l
+      // walks eight of its bins downwards, after a scan over the lanes has told it the weight above them
+      unsigned long long sums[kCluster], a = acc;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        mine[j] = s.hist[0][kBins - 1 - (8 * lane + j)];
-        lane_sum += mine[j];
+      for (int c = 0; c < kCluster; ++c) sums[c] = *cluster.map_shared_rank(&s.segment_sum, c);
+      if (digit == 0) {
+        unsigned long long total = 0;
+#pragma unroll
+        for (int c = 0; c < kCluster; ++c) total += sums[c];
+        target = target_of(total);
+        if (lane == 0) s.found[3] = target;
       }
-      unsigned long long upto = lane_sum;  // inclusive scan over the lanes
+      int segment = -1;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const unsigned long long t = __shfl_up_sync(0xffffffffu, upto, o);
-        if (lane >= o) upto += t;
-      }
-      unsigned long long a = acc + upto - lane_sum;
-      int found = -1;
+      for (int c = kCluster - 1; c >= 0; --c)
+        if (segment < 0) {
+          if (a + sums[c] >= target) segment = c;
+          else a += sums[c];
+        }
+      if (segment < 0) {  // the whole set weighs less than the target
+        if (lane == 0) {
+          s.found[0] = a;
+          s.found[1] = ~0ull;
+          s.found[2] = 0ull;
+        }
+      } else {
+        const unsigned long long* totals = cluster.map_shared_rank(&s.total[0], segment);
+        constexpr int kEach = kSegment / 32;
+        unsigned long long mine[kEach], lane_sum = 0;
 #pragma unroll
-      for (int j = 0; j < 8; ++j)
-        if (found < 0) {
-          if (a + mine[j] >= target) found = j;
-          else a += mine[j];
+        for (int j = 0; j < kEach; ++j) {
+          mine[j] = totals[kSegment - 1 - (kEach * lane + j)];
+          lane_sum += mine[j];
         }
-      const unsigned hit = __ballot_sync(0xffffffffu, found >= 0);
-      if (hit == 0u) {
-        if (lane == 31) {  // the whole set weighs less than the target
-          s.bcast[0] = acc + upto;
-          s.bcast[1] = (unsigned long long)(long long)-1;
-          s.bcast[3] = 0ull;
+        unsigned long long upto = lane_sum;  // inclusive scan over the lanes
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const unsigned long long t = __shfl_up_sync(0xffffffffu, upto, o);
+          if (lane >= o) upto += t;
         }
-      } else if (lane == __ffs(hit) - 1) {
+        a += upto - lane_sum;
+        int at = -1;
         unsigned long long in_bin = 0;
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
-          if (j == found) in_bin = mine[j];
-        s.bcast[0] = a;
-        s.bcast[1] = (unsigned long long)(long long)(kBins - 1 - (8 * lane + found));
-        s.bcast[3] = in_bin;
+        for (int j = 0; j < kEach; ++j)
+          if (at < 0) {
+            if (a + mine[j] >= target) { at = j; in_bin = mine[j]; }
+            else a += mine[j];
+          }
+        const unsigned hit = __ballot_sync(0xffffffffu, at >= 0);
+        if (hit != 0u && lane == __ffs(hit) - 1) {
+          s.found[0] = a;
+          s.found[1] = (unsigned long long)(segment * kSegment + kSegment - 1 - (kEach * lane + at));
+          s.found[2] = in_bin;
+        }
       }
     }
     __syncthreads();
-    acc = s.bcast[0];
-    const long long digit = (long long)s.bcast[1];
-    *equal = s.bcast[3];  // after the last digit: the weight of key == result
+    acc = s.found[0];
+    *equal = s.found[2];
+    target = s.found[3];
+    const unsigned long long bin = s.found[1];
     __syncthreads();
-    if (digit < 0) {  // the whole set weighs less than target
+    if (bin == ~0ull) {  // the whole set weighs less than target
       *above = acc;
       return 0u;
     }
-    prefix |= (uint32_t)digit << shift;
-    mask |= 255u << shift;
+    prefix |= (uint32_t)bin << shift;
+    mask |= (bins - 1u) << shift;
   }
   *above = acc;
   return prefix;
 }
+
+// A count as the target, whatever the total.
+struct Count {
+  unsigned long long n;
+  __device__ __forceinline__ unsigned long long operator()(unsigned long long) const { return n; }
+};
+struct One {
+  __device__ __forceinline__ unsigned long long operator()(float) const { return 1ull; }
+};
 
 // The cut of one stage: keep key > cut_key, and of key == cut_key the tokens with id <= cut_id.
 struct Cut {
@@ -236,7 +315,7 @@ struct Cut {
 // After a select that found `key` with `need` more units wanted among the ties: the id below
 // which ties are kept. Unit weights (top-k) keep exactly `need` ties.
 template <typename Item>
-__device__ Cut cut_with_ties(const RowView& row, Scratch& s, uint32_t key, unsigned long long need,
+__device__ Cut cut_with_ties(const cg::cluster_group& cluster, const Slice& row, Scratch& s, uint32_t key, unsigned long long need,
                              unsigned long long equal, unsigned long long unit, Item item) {
   Cut cut{key, 0x7fffffff};
   if (key == 0u || unit == 0ull) return cut;
@@ -244,255 +323,308 @@ __device__ Cut cut_with_ties(const RowView& row, Scratch& s, uint32_t key, unsig
   const unsigned long long want = (need + unit - 1) / unit;
   if (want * unit >= equal) return cut;  // all of them: no pass over the ids
   unsigned long long dummy, dummy2;
-  auto by_id = [&](int i, float v, uint32_t& k2, unsigned long long& w2) {
+  const uint32_t idk = cluster_select<true>(cluster, row, s, Count{want}, &dummy, &dummy2, false, 3,
+                                            [&](int token, float v, uint32_t& k2) {
     uint32_t k;
-    unsigned long long w;
-    if (!item(i, v, k, w) || k != key) return false;
-    k2 = ~(uint32_t)row.token(i);  // descending on ~id is ascending on id
-    w2 = 1ull;
+    if (!item(token, v, k) || k != key) return false;
+    k2 = ~(uint32_t)token;  // descending on ~id is ascending on id
     return true;
-  };
-  const uint32_t idk = radix_select<true>(row, s, want, &dummy, &dummy2, by_id);
+  }, One{});
   if (idk != 0u) cut.id = (int)~idk;
   return cut;
 }
 
-__device__ int row_argmax(const RowView& row, Scratch& s, float* best_value) {
-  float best = -INFINITY;
-  int best_id = 0x7fffffff;
+// Probability mass of one token as 64-bit fixed point: exp((v - max) / T) * 2^32 (a scaling by a power of two is
+// exact in float32 too).
+__device__ __forceinline__ unsigned long long mass_of(float v, float vmax, float inv_t) {
+  return __float2ull_rz(expf((v - vmax) * inv_t) * 4294967296.f);  // the exponential is in [0, 1]
+}
+
+// What a kept token scores in the exponential race.
+__device__ __forceinline__ float race_score(float v, float vmax, float inv_t, uint64_t seed, uint64_t counter, int token) {
+  const float w = expf((v - vmax) * inv_t);
+  const uint32_t bits = Philox::draw(seed, counter, (uint32_t)token);
+  const float u = ((float)(bits >> 8) + 0.5f) * (1.f / 16777216.f);  // (0, 1)
+  const float e = fmaxf(-logf(u), 1e-10f);
+  return w / e;
+}
+
+// top-p's target: the mass at which the walk from the largest key down stops (the best token always stays).
+__device__ __forceinline__ unsigned long long mass_target(float p, unsigned long long total) {
+  unsigned long long target = (unsigned long long)ceil((double)p * (double)total);
+  if (target < 1ull) target = 1ull;
+  return target > total ? total : target;
+}
+
+// The end of a row whose top-k left candidates (at most kCompact, the k best among them) in this block's scratch:
+// each is ranked by counting those before it, the k best fall into their places, masses are added up along
+// them, and the kept ones race. A token is kept while the mass before it is below top-p's target: the cut that the
+// selects above find, ties (equal keys, equal masses) by ascending id included.
+__device__ int finish_candidates(Scratch& s, int k, float p, float vmax, float inv_t, uint64_t seed, uint64_t counter, int best) {
+  const int n = min(s.cand_n, kCompact), keep = min(k, n);
+  for (int i = threadIdx.x; i < n; i += kThreads) {
+    const uint32_t key = s.cand_key[i];
+    const int id = s.cand_id[i];
+    int before = 0, j = 0;
+    for (; j + 4 <= n; j += 4) {
+      const uint4 kk = *reinterpret_cast<const uint4*>(&s.cand_key[j]);
+      const int4 ii = *reinterpret_cast<const int4*>(&s.cand_id[j]);
+      before += (kk.x > key || (kk.x == key && ii.x < id)) + (kk.y > key || (kk.y == key && ii.y < id)) +
+                (kk.z > key || (kk.z == key && ii.z < id)) + (kk.w > key || (kk.w == key && ii.w < id));
+    }
+    for (; j < n; ++j) before += s.cand_key[j] > key || (s.cand_key[j] == key && s.cand_id[j] < id);
+    s.sorted_key[before] = key;
+    s.sorted_id[before] = id;
+  }
+  __syncthreads();
+  // two neighbouring places a thread: their masses, and the mass before them
+  static_assert(kCompact == 2 * kThreads, "two places a thread");
+  const int at = 2 * threadIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned long long m[2] = {0ull, 0ull};
+#pragma unroll
+  for (int u = 0; u < 2; ++u)
+    if (at + u < keep) {
+      const float v = key_value(s.sorted_key[at + u]);
+      m[u] = v == v ? mass_of(v, vmax, inv_t) : 0ull;  // a NaN takes a place among the k and has no mass
+    }
+  unsigned long long upto = m[0] + m[1];
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned long long t = __shfl_up_sync(0xffffffffu, upto, o);
+    if (lane >= o) upto += t;
+  }
+  if (lane == 31) s.warp_part[warp] = upto;
+  __syncthreads();
+  unsigned long long total = 0, before = upto - m[0] - m[1];
+  for (int w = 0; w < kWarps; ++w) {
+    if (w < warp) before += s.warp_part[w];
+    total += s.warp_part[w];
+  }
+  const bool cuts = p < 1.f;
+  const unsigned long long target = cuts ? mass_target(p, total) : 0ull;
+  Best mine{-1.f, 0x7fffffff};
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    if (at + u < keep && (!cuts || before < target)) {
+      const int token = s.sorted_id[at + u];
+      mine.take(race_score(key_value(s.sorted_key[at + u]), vmax, inv_t, seed, counter, token), token);
+    }
+    before += m[u];
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float os = __shfl_xor_sync(0xffffffffu, mine.score, o);
+    const int ot = __shfl_xor_sync(0xffffffffu, mine.token, o);
+    mine.take(os, ot);
+  }
+  __syncthreads();
+  if (lane == 0) s.warp_best[warp] = mine;
+  __syncthreads();
+  for (int w = 0; w < kWarps; ++w) mine.take(s.warp_best[w].score, s.warp_best[w].token);
+  return mine.token == 0x7fffffff ? best : mine.token;
+}
+
+// This block's share of the cluster's row, brought into shared memory where it fits, and the best of it.
+__device__ Slice take_slice(const cg::cluster_group& cluster, const float* logits, int V, float* room, int room_floats, Best* best,
+                            bool* nan) {
+  const int each = ((V + kCluster - 1) / kCluster + 3) & ~3;
+  const int first = min(V, (int)cluster.block_rank() * each), n = min(each, V - first);
+  const float* from = logits + first;
+  const bool keep = n <= room_floats;
+  *best = Best{-INFINITY, 0x7fffffff};
+  *nan = false;  // whether this thread met one
   int done = 0;
-  if (row.id == nullptr && ((uintptr_t)row.val & 15) == 0) {
-    // the full row: 16-byte loads, four in flight per thread
-    const float4* v4 = reinterpret_cast<const float4*>(row.val);
-    const int n4 = row.n >> 2;
-    for (int i = threadIdx.x; i < n4; i += blockDim.x * 4) {
+  if (((uintptr_t)from & 15) == 0) {
+    const float4* v4 = reinterpret_cast<const float4*>(from);
+    const int n4 = n >> 2;
+    for (int i = threadIdx.x; i < n4; i += 4 * kThreads) {  // four loads in flight
       float4 x[4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int at = i + u * blockDim.x;
-        x[u] = at < n4 ? v4[at] : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
-      }
+      for (int u = 0; u < 4; ++u)
+        if (i + u * kThreads < n4) x[u] = v4[i + u * kThreads];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        const int t0 = (i + u * blockDim.x) * 4;
-        const float e[4] = {x[u].x, x[u].y, x[u].z, x[u].w};
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-          if (e[k] > best || (e[k] == best && t0 + k < best_id)) { best = e[k]; best_id = t0 + k; }
+        const int j = i + u * kThreads;
+        if (j >= n4) break;
+        if (keep) reinterpret_cast<float4*>(room)[j] = x[u];
+        const int t = first + 4 * j;
+        *nan |= x[u].x != x[u].x || x[u].y != x[u].y || x[u].z != x[u].z || x[u].w != x[u].w;
+        best->take(x[u].x, t);
+        best->take(x[u].y, t + 1);
+        best->take(x[u].z, t + 2);
+        best->take(x[u].w, t + 3);
       }
     }
     done = n4 << 2;
   }
-  for (int i = done + threadIdx.x; i < row.n; i += blockDim.x) {
-    const float v = row.value(i);
-    const int t = row.token(i);
-    if (v > best || (v == best && t < best_id)) { best = v; best_id = t; }
-  }
+  for (int i = done + threadIdx.x; i < n; i += 8 * kThreads) {  // eight loads in flight
+    float x[8];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-    const int oi = __shfl_xor_sync(0xffffffffu, best_id, o);
-    if (ov > best || (ov == best && oi < best_id)) { best = ov; best_id = oi; }
-  }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  __syncthreads();
-  if (lane == 0) { s.red[warp] = best; s.red_i[warp] = best_id; }
-  __syncthreads();
-  if (warp == 0) {
-    const int nw = (blockDim.x + 31) >> 5;
-    best = lane < nw ? s.red[lane] : -INFINITY;
-    best_id = lane < nw ? s.red_i[lane] : 0x7fffffff;
+    for (int u = 0; u < 8; ++u)
+      if (i + u * kThreads < n) x[u] = from[i + u * kThreads];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, best_id, o);
-      if (ov > best || (ov == best && oi < best_id)) { best = ov; best_id = oi; }
+    for (int u = 0; u < 8; ++u) {
+      const int j = i + u * kThreads;
+      if (j >= n) break;
+      if (keep) room[j] = x[u];
+      *nan |= x[u] != x[u];
+      best->take(x[u], first + j);
     }
-    if (lane == 0) { s.red[0] = best; s.red_i[0] = best_id; }
   }
   __syncthreads();
-  const int id = s.red_i[0] == 0x7fffffff ? 0 : s.red_i[0];  // a row of NaN or -inf only
-  if (best_value) *best_value = s.red[0];
-  __syncthreads();
-  return id;
+  return Slice{keep ? room : from, first, n};
 }
 
-// Probability mass of one token as 64-bit fixed point: exp((v - max) / T) * 2^32.
-__device__ __forceinline__ unsigned long long mass_of(float v, float vmax, float inv_t) {
-  const float w = expf((v - vmax) * inv_t);  // in [0, 1]
-  return (unsigned long long)((double)w * 4294967296.0);
-}
-
-__global__ void __launch_bounds__(kThreads)
+__global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads, 2)
 sample_rows_kernel(int* __restrict__ out, const float* __restrict__ logits, int V,
                    const float* __restrict__ temperature, const int* __restrict__ top_k,
                    const float* __restrict__ top_p, const unsigned long long* __restrict__ seed,
-                   const unsigned long long* __restrict__ counter) {
+                   const unsigned long long* __restrict__ counter, int room_floats) {
   asb::pdl_wait();  // the stream's previous kernel has completed (programmatic dependent launch)
   asb::pdl_launch_dependents();
   __shared__ Scratch s;
-  const int b = blockIdx.x;
-  RowView row{logits + (size_t)b * V, nullptr, V};
+  extern __shared__ __align__(16) float room[];
+  const cg::cluster_group cluster = cg::this_cluster();
+  const int b = blockIdx.x / kCluster;
+  const bool leads = cluster.block_rank() == 0;
   const float temp = temperature[b];
 
-  float vmax;
-  const int best = row_argmax(row, s, &vmax);
+  if (threadIdx.x == 0) s.cand_n = 0;
+  Best top;
+  bool odd;
+  const Slice row = take_slice(cluster, logits + (size_t)b * V, V, room, room_floats, &top, &odd);
+  s.odd = 0;
+  __syncthreads();
+  if (odd) s.odd = 1;
+  top = cluster_best(cluster, s, top, 0);
+  const float vmax = top.score;
+  const int best = top.token == 0x7fffffff ? 0 : top.token;  // a row of NaN or -inf only
   if (!(temp > 0.f)) {  // greedy: the single best, lowest id among equals
-    if (threadIdx.x == 0) out[b] = best;
+    if (leads && threadIdx.x == 0) out[b] = best;
+    cluster.sync();  // nobody leaves while a neighbour may still read its best
     return;
   }
   const float inv_t = 1.f / temp;
+  const uint64_t sd = seed[b], ctr = counter[b];
+  const float p = top_p[b];
+  // masses are added up in 64-bit words where a slice has more elements than two 32-bit words can hold, or where a
+  // mass may lie outside [0, 2^32]
+  bool wide = V > kCluster * (kSplitSlice - 3) || isinf(vmax);
+#pragma unroll
+  for (int c = 0; c < kCluster; ++c) wide |= *cluster.map_shared_rank(&s.odd, c) != 0;
 
   // top-k
   const int k = top_k[b];
   Cut kcut{0u, 0x7fffffff};
   if (k > 0 && k < V) {
-    auto unit = [&](int i, float v, uint32_t& key, unsigned long long& w) {
+    auto any = [&](int token, float v, uint32_t& key) {
       key = order_key(v);
-      w = 1ull;
       return true;
     };
+    const Count kth{(unsigned long long)k};
     unsigned long long above, equal;
-    bool early = false;
+    uint32_t from = 0u;  // candidates: keys from here on
+    bool few = false;
     if (k <= kCompact) {
-      // The two high digits of the k-th largest key: if everything from that bin of 65,536 keys
-      // upwards fits the candidate buffer (it holds at least k), gather it now and finish the
-      // selection, like all later passes, on the candidates in shared memory.
-      // Only keys within four first-digit bins of the largest (a factor of 16 or so below the best
-      // logit when it is positive) are counted here, which spares the atomics of nearly the whole
-      // row; if fewer than k lie there, `high` comes back 0 and the full selection below runs.
+      // The high digits of the k-th largest key: if everything from that range of keys upwards fits the
+      // candidate buffer (it holds at least k), the ranking of the candidates finishes the selection.
+      // Only keys within four eighths of the exponent range's steps below the largest (a factor of 16 or so below
+      // the best logit when it is positive) are counted here, which spares the atomics of nearly the whole
+      // row; if fewer than k lie there, the result is 0 and the full selection below runs.
       const uint32_t top_bin = order_key(vmax) >> 24;
       const uint32_t floor_key = top_bin >= 3u ? (top_bin - 3u) << 24 : 0u;
-      auto unit_near_top = [&](int i, float v, uint32_t& key, unsigned long long& w) {
-        key = order_key(v);
-        w = 1ull;
-        return key >= floor_key;
-      };
-      const uint32_t high = radix_select<true>(row, s, (unsigned long long)k, &above, &equal, unit_near_top, 16);
-      if (high != 0u && above + equal <= (unsigned long long)kCompact) {
-        early = true;
-        if (threadIdx.x == 0) s.cand_n = 0;
-        __syncthreads();
-        for_each_value(row, [&](int i, float v, bool valid) {
-          if (valid && order_key(v) >= high) {
-            const int at = atomicAdd(&s.cand_n, 1);
-            if (at < kCompact) { s.cand_val[at] = v; s.cand_id[at] = i; }
-          }
-        });
-        __syncthreads();
-        row = RowView{s.cand_val, s.cand_id, min(s.cand_n, kCompact)};
-        const uint32_t key = radix_select<true>(row, s, (unsigned long long)k, &above, &equal, unit);
-        kcut = cut_with_ties(row, s, key, (unsigned long long)k - above, equal, 1ull, unit);
+      for (int digits = 1; digits <= 2 && !few; ++digits) {
+        from = cluster_select<true>(cluster, row, s, kth, &above, &equal, false, digits, [&](int token, float v, uint32_t& key) {
+          key = order_key(v);
+          return key >= floor_key;
+        }, One{});
+        if (from == 0u) break;
+        few = above + equal <= (unsigned long long)kCompact;
       }
     }
-    if (!early) {
-      const uint32_t key = radix_select<true>(row, s, (unsigned long long)k, &above, &equal, unit);
-      kcut = cut_with_ties(row, s, key, (unsigned long long)k - above, equal, 1ull, unit);
-      if (k <= kCompact) {  // later passes read the candidates from shared memory
-        if (threadIdx.x == 0) s.cand_n = 0;
-        __syncthreads();
-        for_each_value(row, [&](int i, float v, bool valid) {
-          if (valid && kcut.keeps(order_key(v), i)) {
-            const int at = atomicAdd(&s.cand_n, 1);
-            if (at < kCompact) { s.cand_val[at] = v; s.cand_id[at] = i; }
-          }
-        });
-        __syncthreads();
-        row = RowView{s.cand_val, s.cand_id, min(s.cand_n, kCompact)};
-        kcut = Cut{0u, 0x7fffffff};
-      }
+    if (!few) {
+      const uint32_t key = cluster_select<true>(cluster, row, s, kth, &above, &equal, false, 3, any, One{});
+      kcut = cut_with_ties(cluster, row, s, key, (unsigned long long)k - above, equal, 1ull, any);
+    }
+    if (k <= kCompact) {
+      // to the first block, which ends the row alone (the order they arrive in does not matter)
+      Scratch* lead = cluster.map_shared_rank(&s, 0);
+      for_each_value(row, [&](int token, float v) {
+        const uint32_t key = order_key(v);
+        if (few ? key >= from : kcut.keeps(key, token)) {
+          const int at = atomicAdd(&lead->cand_n, 1);
+          if (at < kCompact) { lead->cand_key[at] = key; lead->cand_id[at] = token; }
+        }
+      });
+      cluster.sync();
+      if (!leads) return;  // (and the first block reads nothing of its neighbours from here on)
+      const int token = finish_candidates(s, k, p, vmax, inv_t, sd, ctr, best);
+      if (threadIdx.x == 0) out[b] = token;
+      return;
     }
   }
 
-  // total mass of the kept, then the top-p cut
-  auto massed = [&](int i, float v, uint32_t& key, unsigned long long& w) {
-    key = order_key(v);
-    if (!kcut.keeps(key, row.token(i))) return false;
-    w = mass_of(v, vmax, inv_t);
-    return true;
-  };
-  unsigned long long total = 0;
-  for_each_value(row, [&](int i, float v, bool valid) {
-    uint32_t key;
-    unsigned long long w;
-    if (valid && massed(i, v, key, w)) total += w;
-  });
-  {
-    // integer sum over the block: exact, so independent of the order
-    for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) s.hist[0][threadIdx.x >> 5] = total;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      unsigned long long t = 0;
-      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += s.hist[0][w];
-      s.bcast[2] = t;
-    }
-    __syncthreads();
-    total = s.bcast[2];
-    __syncthreads();
-  }
-
+  // the top-p cut
   Cut pcut{0u, 0x7fffffff};
-  const float p = top_p[b];
   if (p < 1.f) {
+    auto kept = [&](int token, float v, uint32_t& key) {
+      key = order_key(v);
+      return kcut.keeps(key, token);
+    };
+    auto mass = [&](float v) { return mass_of(v, vmax, inv_t); };
     // keep a token while the mass ranked above it is < p * total: find the first key whose
     // cumulative mass (itself included) exceeds p * total, ties by ascending id
-    unsigned long long target = (unsigned long long)ceil((double)p * (double)total);
-    if (target < 1ull) target = 1ull;  // the best token always stays
-    if (target > total) target = total;
-    unsigned long long above, equal;
-    const uint32_t key = radix_select<false>(row, s, target, &above, &equal, massed);
+    unsigned long long above, equal, target = 0;
+    const uint32_t key = cluster_select<false>(cluster, row, s, [&](unsigned long long total) { return mass_target(p, total); },
+                                               &above, &equal, wide, 3, kept, mass);
+    target = s.found[3];
     // mass of one tied token (all ties share the key, hence the value)
-    unsigned long long unit = mass_of(__uint_as_float((key & 0x80000000u) ? (key & 0x7fffffffu) : ~key), vmax, inv_t);
-    pcut = cut_with_ties(row, s, key, target - above, equal, unit, massed);
+    pcut = cut_with_ties(cluster, row, s, key, target - above, equal, mass_of(key_value(key), vmax, inv_t), kept);
   }
 
   // exponential race among the kept
-  const unsigned long long sd = seed[b], ctr = counter[b];
-  float best_score = -1.f;
-  int best_token = 0x7fffffff;
-  for_each_value(row, [&](int i, float v, bool valid) {
-    if (!valid) return;
+  Best winner{-1.f, 0x7fffffff};
+  for_each_value(row, [&](int token, float v) {
     const uint32_t key = order_key(v);
-    const int token = row.token(i);
     if (!kcut.keeps(key, token) || !pcut.keeps(key, token)) return;
-    const float w = expf((v - vmax) * inv_t);
-    const uint32_t bits = Philox::draw(sd, ctr, (uint32_t)token);
-    const float u = ((float)(bits >> 8) + 0.5f) * (1.f / 16777216.f);  // (0, 1)
-    const float e = fmaxf(-logf(u), 1e-10f);
-    const float score = w / e;
-    if (score > best_score || (score == best_score && token < best_token)) {
-      best_score = score;
-      best_token = token;
-    }
+    winner.take(race_score(v, vmax, inv_t, sd, ctr, token), token);
   });
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float os = __shfl_xor_sync(0xffffffffu, best_score, o);
-    const int ot = __shfl_xor_sync(0xffffffffu, best_token, o);
-    if (os > best_score || (os == best_score && ot < best_token)) { best_score = os; best_token = ot; }
-  }
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) { s.red[threadIdx.x >> 5] = best_score; s.red_i[threadIdx.x >> 5] = best_token; }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int w = 1; w < (int)(blockDim.x >> 5); ++w)
-      if (s.red[w] > best_score || (s.red[w] == best_score && s.red_i[w] < best_token)) {
-        best_score = s.red[w];
-        best_token = s.red_i[w];
-      }
-    out[b] = best_token == 0x7fffffff ? best : best_token;
-  }
+  winner = cluster_best(cluster, s, winner, 1);
+  if (leads && threadIdx.x == 0) out[b] = winner.token == 0x7fffffff ? best : winner.token;
+  cluster.sync();  // nobody leaves while a neighbour may still read its best
 }
 
-__global__ void argmax_rows_kernel(int* __restrict__ out, const float* __restrict__ logits, int V) {
+__global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads, 2)
+argmax_rows_kernel(int* __restrict__ out, const float* __restrict__ logits, int V) {
   asb::pdl_wait();  // the stream's previous kernel has completed (programmatic dependent launch)
   asb::pdl_launch_dependents();
-  __shared__ Scratch s;
-  RowView row{logits + (size_t)blockIdx.x * V, nullptr, V};
-  const int best = row_argmax(row, s, nullptr);
-  if (threadIdx.x == 0) out[blockIdx.x] = best;
+  __shared__ Best slots[1 + kWarps];  // this block's best, and its warps'
+  const cg::cluster_group cluster = cg::this_cluster();
+  const int b = blockIdx.x / kCluster;
+  Best top;
+  bool nan;
+  take_slice(cluster, logits + (size_t)b * V, V, nullptr, -1, &top, &nan);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float os = __shfl_xor_sync(0xffffffffu, top.score, o);
+    const int ot = __shfl_xor_sync(0xffffffffu, top.token, o);
+    top.take(os, ot);
+  }
+  if ((threadIdx.x & 31) == 0) slots[1 + (threadIdx.x >> 5)] = top;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < kWarps; ++w) top.take(slots[1 + w].score, slots[1 + w].token);
+    slots[0] = top;
+  }
+  cluster.sync();
+  if (cluster.block_rank() == 0 && threadIdx.x == 0) {
+    for (int c = 1; c < kCluster; ++c) {
+      const Best o = *cluster.map_shared_rank(&slots[0], c);
+      top.take(o.score, o.token);
+    }
+    out[b] = top.token == 0x7fffffff ? 0 : top.token;  // a row of NaN or -inf only
+  }
+  cluster.sync();  // nobody leaves while the first block reads its best
 }
 
 __global__ void presence_penalty_kernel(float* __restrict__ logits, const int* __restrict__ rows,
@@ -508,7 +640,8 @@ __global__ void presence_penalty_kernel(float* __restrict__ logits, const int* _
 
 extern "C" int asb_argmax_rows(int* out, const float* logits, int B, int V, cudaStream_t stream) {
   if (B == 0) return 0;
-  asb::launch(argmax_rows_kernel, B, kThreads, 0, stream, out, logits, V);
+  if (B > 0x7fffffff / kCluster) return asb::fail("argmax_rows: %d rows", B);
+  asb::launch(argmax_rows_kernel, kCluster * B, kThreads, 0, stream, out, logits, V);
   return asb::check_launch("argmax_rows");
 }
 
@@ -526,6 +659,12 @@ extern "C" int asb_sample_rows(int* out, const float* logits, int B, int V,
                                cudaStream_t stream) {
   if (B == 0) return 0;
   if (V < 1) return asb::fail("sample_rows: vocabulary %d", V);
-  asb::launch(sample_rows_kernel, B, kThreads, 0, stream, out, logits, V, temperature, top_k, top_p, seed, counter);
+  if (B > 0x7fffffff / kCluster) return asb::fail("sample_rows: %d rows", B);
+  // a slice too long for shared memory is read in place in every pass
+  const int each = ((V + kCluster - 1) / kCluster + 3) & ~3, room = each <= kMaxSlice ? each : 0;
+  cudaError_t e = cudaFuncSetAttribute(sample_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(room * sizeof(float)));
+  if (e != cudaSuccess) return asb::fail("sample_rows: shared memory of %d floats: %s", room, cudaGetErrorString(e));
+  asb::launch(sample_rows_kernel, kCluster * B, kThreads, room * sizeof(float), stream, out, logits, V, temperature, top_k, top_p,
+              seed, counter, room);
   return asb::check_launch("sample_rows");
 }

@@ -2,6 +2,7 @@
 
 import math
 
+import numpy as np
 import pytest
 import torch
 
@@ -485,6 +486,50 @@ def test_seeded_rows_do_not_depend_on_neighbours(ops):
     alone = [run(row[None], [7], [i])[0] for i in range(20)]
     crowd = [run(torch.stack([others[0], row, others[1]]), [1, 7, 2], [i + 5, i, i + 9])[1] for i in range(20)]
     assert alone == crowd and len(set(alone)) > 3
+
+
+def philox_uniforms(seed: int, counter: int, n: int) -> np.ndarray:
+    """The race's uniforms of tokens 0..n-1: Philox-4x32-10 (Salmon et al. 2011), counter (token, draw counter, 0x5a17)."""
+    m32 = np.uint64(0xFFFFFFFF)
+    c = [np.arange(n, dtype=np.uint64), np.full(n, counter & 0xFFFFFFFF, np.uint64), np.full(n, counter >> 32, np.uint64),
+         np.full(n, 0x5A17, np.uint64)]  # fmt: skip
+    k0, k1 = seed & 0xFFFFFFFF, seed >> 32
+    for _ in range(10):
+        p0, p1 = np.uint64(0xD2511F53) * c[0], np.uint64(0xCD9E8D57) * c[2]
+        c = [(p1 >> np.uint64(32)) ^ c[1] ^ np.uint64(k0), p1 & m32, (p0 >> np.uint64(32)) ^ c[3] ^ np.uint64(k1), p0 & m32]
+        k0, k1 = (k0 + 0x9E3779B9) & 0xFFFFFFFF, (k1 + 0xBB67AE85) & 0xFFFFFFFF
+    return ((c[0] >> np.uint64(8)).astype(np.float64) + 0.5) / 2.0**24
+
+
+@pytest.mark.parametrize("V", [1, 3, 30, 33, 257, 4099, 32000, 400004])
+@pytest.mark.parametrize("k,p,temp", [(20, 0.95, 0.6), (0, 0.9, 1.0), (1024, 0.999, 1.0), (1025, 0.8, 1.3), (1, 1.0, 0.7), (0, 1.0, 1.0)])
+def test_sampled_token_wins_the_plain_race(ops, V, k, p, temp):
+    """The drawn token is the winner of the exponential race over the plain sampler's support, at row lengths around
+    the edges of a block's share of a row (eighths, multiples of four) and beyond what shared memory holds, with ties
+    and masked (-inf) tokens among the logits, and each way top-k can go."""
+    g = torch.Generator().manual_seed(V + k)
+    logits = torch.randn(3, V, generator=g) * 3
+    logits[1] = (logits[1] * 2).round() / 2  # ties at every cut
+    if V > 3:
+        logits[2, torch.randperm(V, generator=g)[: V // 2]] = -math.inf
+    seeds, counters = [5, (1 << 40) + 3, 77], [0, 9, 1 << 33]
+    out = ops.sample_rows(
+        logits.cuda(), torch.full((3,), temp, device="cuda"), torch.full((3,), k, dtype=torch.int32, device="cuda"),
+        torch.full((3,), p, device="cuda"), torch.tensor(seeds, device="cuda"), torch.tensor(counters, device="cuda"),
+    ).tolist()  # fmt: skip
+    assert ops.argmax_rows(logits.cuda()).tolist() == [int(torch.nonzero(r == r.max())[0]) for r in logits]
+    for r in range(3):
+        x = logits[r].double().numpy()
+        order = np.lexsort((np.arange(V), -x))  # largest first, lower ids first among equals
+        order = order[: k if 0 < k < V else V]
+        mass = np.exp((x[order] - x[order[0]]) / np.float64(np.float32(temp)))
+        before = np.cumsum(mass) - mass
+        kept = order[before < p * mass.sum() * (1 - 1e-9)] if p < 1 else order
+        edge = order[before < p * mass.sum() * (1 + 1e-6)] if p < 1 else order  # float32 masses may keep one more at the cut
+        score = np.exp((x - x.max()) / np.float64(np.float32(temp))) / np.maximum(-np.log(philox_uniforms(seeds[r], counters[r], V)), 1e-10)
+        assert out[r] in edge
+        # (the kernel's float32 exponential and logarithm differ from these by a few units in the last place)
+        assert score[out[r]] >= score[kept].max() * (1 - 1e-5)
 
 
 def test_presence_penalty(ops):
