@@ -84,6 +84,31 @@ def test_linear_rows_do_not_depend_on_the_batch(ops):
     assert torch.equal(ops.linear(x[60:].contiguous(), w), whole[60:])
 
 
+@pytest.mark.parametrize("K", [1, 12, 30, 256, 260, 771, 772, 1028, 8192, 8460, 12288])
+@pytest.mark.parametrize("N", [1, 63, 130, 384])
+def test_float32_linear_in_both_kernels(ops, N, K):
+    """The float32 product on either side of each of its dispatch's lines (4, 8, 16 and 32 rows; K by a multiple of 4,
+    by fewer runs of 256 than quarters, by more than eight runs a block; rows off 16 bytes): against float64, within the
+    bound of a sum cut into chains of 256, and each row the same bits whatever the number of rows beside it."""
+    g = torch.Generator().manual_seed(N + K)
+    x = torch.randn(131, K, generator=g).cuda()
+    w = torch.randn(N, K, generator=g).cuda()
+    res = torch.randn(131, N, generator=g).cuda()
+    exact = x.double() @ w.double().T
+    runs = -(-K // 256)
+    # a rounding per multiply-add of a chain, per run of a quarter, per quarter and for the residual
+    bound = (256 + -(-runs // 4) + 4 + 1) * 2.0**-24 * (x.double().abs() @ w.double().abs().T + res.double().abs())
+    whole, with_res = ops.linear(x, w), ops.linear(x, w, res)
+    assert ((whole.double() - exact).abs() <= bound).all()
+    assert ((with_res.double() - (exact + res.double())).abs() <= bound).all()
+    for M in (1, 4, 5, 8, 9, 16, 17, 32, 33, 64, 65):
+        assert torch.equal(ops.linear(x[:M], w), whole[:M]), M
+        assert torch.equal(ops.linear(x[130 - M : 130], w, res[130 - M : 130]), with_res[130 - M : 130]), M
+    off = torch.empty(131 * K + 1, device="cuda")[1:].view(131, K).copy_(x)  # rows that start off 16 bytes
+    for M in (3, 20, 131):
+        assert torch.equal(ops.linear(off[:M], w), whole[:M])
+
+
 def rope_reference(x, positions, hd, theta, rotary_dim=None):
     rd = rotary_dim or hd
     angles = plain.rope_angles(positions, rd, theta)
