@@ -13,7 +13,7 @@ from atomserve_b200.ops.library import KernelLibraryError, check, dtype_code, li
 KEY_TILE = 32
 TARGET_BLOCKS = 296  # two blocks for each of the 148 SMs before the key range is split
 SHORT_ROWS = 8  # requests with at most this many new tokens run row by row in the decode kernel
-MIXED_SCRATCH_BYTES = 128 << 20  # most that a mixed step's partial results may take (see _paged_attention_mma)
+MIXED_SCRATCH_BYTES = 128 << 20  # most that a step's partial results may take (see _paged_attention_parts)
 
 
 # Which kernel serves prompt portions in bfloat16 with head size 128: "tcgen05" (scores and output
@@ -94,6 +94,26 @@ def plan_decode_partitions(rows: int, num_kv_heads: int, group: int, max_context
     return (size, parts) if parts > 1 else (1 << 30, 1)
 
 
+def plan_decode_ranges(rows: int, num_kv_heads: int, group: int, max_context: int, window: int, head_dim: int = 128,
+                       partitions: tuple[int, int] | None = None) -> int:  # fmt: skip
+    """Equal ranges into which the decode kernel cuts the keys of all rows, each for a block per kv head (and 16 of its
+    heads); 0: each row is a range, and there is no merge. Where rows of the longest context would not be split, nothing
+    is. Otherwise as many ranges as the device holds at once, three blocks an SM, if that leaves a block eight key tiles
+    of the longest context; with less work three quarters of them, and no more than there are tiles: a merge of more
+    shares then costs more than the shorter walk saves (one request of 12,288 keys and 8 kv heads: 18.7 us in 16
+    ranges, 16.3 in 40, 19.3 in 55; of 2,048 keys: 10.8 us in 8, 9.4 in 32, 8.4 in 40; 64 requests of 300 to 3,000
+    keys: 90.3 us in 24, 78.4 in 55)."""
+    size, parts = partitions or plan_decode_partitions(rows, num_kv_heads, group, max_context, window, head_dim)
+    if parts <= 1:
+        return 0
+    if partitions:
+        return rows * parts
+    resident = lib().asb_decode_attention_resident_blocks(head_dim) or 3 * 148
+    full = max(1, resident // (num_kv_heads * -(-group // 16)))
+    tiles = rows * -(-(min(max_context, window) if window > 0 else max_context) // 64)
+    return full if tiles >= 8 * full else max(1, min(3 * full // 4, tiles))
+
+
 def paged_attention(
     q: torch.Tensor,
     k_cache: torch.Tensor,
@@ -113,6 +133,7 @@ def paged_attention(
     chunk: int | None = None,
     softcap: float | None = None,
     keep_first: int = 0,
+    earlier_keys_stored: bool = False,
 ) -> torch.Tensor:
     """softmax(q k^T * scale) v for every new token, keys read in place from the pages.
 
@@ -132,6 +153,9 @@ def paged_attention(
     the chunk. q may be [T, H, KV, hd], a vector per key head: a head's score is then the sum of the
     products with all kv heads' keys (its values are still those of its own kv head): how scores that
     are mixed across heads run, the mix being part of the queries.
+
+    `earlier_keys_stored`: the keys below every request's `req_pos_start` were written before the stream's previous
+    kernel was launched (by earlier steps, as in a model's step), so the decode kernel may read them while that kernel runs.
 
     bfloat16 with head size 64 or 128 runs the tensor-core kernels (decode kernel for requests
     that bring at most 8 tokens, prefill kernel for longer portions; `host_q_lens`, the tokens
@@ -165,7 +189,8 @@ def paged_attention(
     keep = int(keep_first) if span else 0
     if q.dtype == torch.bfloat16 and not generic and not summed and not keep and lib().asb_attention_mma_supported(hd, H // KV):
         return _paged_attention_mma(q, out, k_cache, v_cache, block_tables, req_q_start, req_pos_start,
-                                    num_requests, max_context, win, scale, partitions, host_q_lens, sink, chunk, softcap, span)  # fmt: skip
+                                    num_requests, max_context, win, scale, partitions, host_q_lens, sink, chunk, softcap, span,
+                                    earlier_keys_stored)  # fmt: skip
     if q.dtype == torch.bfloat16 and not generic and summed and not chunk and not softcap and sink is None and lib().asb_attention_parts_supported(hd, H, KV):
         return _paged_attention_parts(q, out, k_cache, v_cache, block_tables, req_q_start, req_pos_start, num_requests, max_context,
                                       win, keep, scale, partitions, host_q_lens)  # fmt: skip
@@ -183,7 +208,7 @@ def paged_attention(
 
 
 def _paged_attention_mma(q, out, k_cache, v_cache, block_tables, req_q_start, req_pos_start, num_requests,
-                         max_context, win, scale, partitions, host_q_lens, sink=None, chunk=0, softcap=0.0, span=None):  # fmt: skip
+                         max_context, win, scale, partitions, host_q_lens, sink=None, chunk=0, softcap=0.0, span=None, earlier_keys_stored=False):  # fmt: skip
     span = win if span is None else span  # what bounds the keys of a row, for the planner
     T, H, hd = q.shape
     KV, bs = k_cache.shape[1], k_cache.shape[2]
@@ -196,6 +221,23 @@ def _paged_attention_mma(q, out, k_cache, v_cache, block_tables, req_q_start, re
         has_long = any(n > SHORT_ROWS for n in host_q_lens)
         all_single = all(n == 1 for n in host_q_lens)
         short_rows = sum(n for n in host_q_lens if n <= SHORT_ROWS)
+
+    def decode(compact):
+        """The launch for the rows of short requests: all T rows of the step, or the `compact` short ones of a step
+        that holds longer portions too. Its scratch belongs to the stream that is current now."""
+        group = H // KV
+        ranges = plan_decode_ranges(short_rows, KV, group, max_context, span, hd, partitions)
+        floats = 4 * (compact or T) + 2 * ranges * KV * -(-group // 16) * min(group, 16) * (hd + 2)
+        scratch = torch.empty(floats, device=q.device, dtype=torch.float32) if ranges else None
+
+        def launch():
+            check(lib().asb_decode_attention(
+                ptr(out), ptr(q), ptr(k_cache), ptr(v_cache), ptr(block_tables), ptr(req_q_start), ptr(req_pos_start),
+                ptr(scratch), ptr(sink), T, num_requests, H, KV, hd, bs, block_tables.shape[1], win, chunk, ranges,
+                float(scale), softcap, int(all_single), compact, int(earlier_keys_stored), stream()))  # fmt: skip
+
+        return launch
+
     if has_long and PREFILL_KERNEL == "tcgen05" and lib().asb_attention_tcgen05_supported(hd, H // KV, bs):
         from atomserve_b200.ops.linear import gemm_status
 
@@ -208,36 +250,10 @@ def _paged_attention_mma(q, out, k_cache, v_cache, block_tables, req_q_start, re
         if not has_short:
             portions()
             return out
-        # What is left for the decode kernel: the short rows, with the key partitions their number
-        # and context call for (a decoding request beside a prompt portion has as long a context
-        # as in a step of its own). When the caller says how many tokens each request brings, the
-        # kernel starts blocks for the short rows only and the partial results hold only those
-        # rows; otherwise blocks start for every row of the step and the portions' leave at once.
-        ps, np_ = partitions or plan_decode_partitions(short_rows, KV, H // KV, max_context, span, hd)
-        compact = short_rows if host_q_lens is not None else 0
-        scratch_rows = compact or T
-        if partitions is None and scratch_rows * H * np_ * (hd + 2) * 4 > MIXED_SCRATCH_BYTES:
-            ps, np_ = 1 << 30, 1
-        part_m = part_l = part_acc = None
-        if np_ > 1:
-            part_m = torch.empty(scratch_rows * H * np_, device=q.device, dtype=torch.float32)
-            # (without the short rows' count the merge runs over every row of the step and leaves
-            # alone those whose sums are zero: the portions' rows, stored by their own kernel)
-            part_l = (torch.empty if compact else torch.zeros)(scratch_rows * H * np_, device=q.device, dtype=torch.float32)
-            part_acc = torch.empty(scratch_rows * H * np_ * hd, device=q.device, dtype=torch.float32)
-
-        def single_tokens():
-            check(lib().asb_paged_attention_mma_masked(
-                ptr(out), ptr(q), ptr(k_cache), ptr(v_cache), ptr(block_tables), ptr(req_q_start),
-                ptr(req_pos_start), ptr(part_m), ptr(part_l), ptr(part_acc), ptr(sink), T, num_requests, H, KV, hd, bs,
-                block_tables.shape[1], win, chunk, ps, np_, float(scale), softcap, 1, 0, 0, compact, stream()))  # fmt: skip
-            if np_ > 1 and compact:
-                check(lib().asb_attention_reduce_short(ptr(out), ptr(part_m), ptr(part_l), ptr(part_acc), ptr(req_q_start),
-                                                       num_requests, SHORT_ROWS, compact, H, np_, hd, dtype_code(q), stream()))  # fmt: skip
-            elif np_ > 1:
-                check(lib().asb_attention_reduce(ptr(out), ptr(part_m), ptr(part_l), ptr(part_acc), T * H, np_, hd,
-                                                 dtype_code(q), stream()))  # fmt: skip
-
+        # What is left for the decode kernel: the short rows. When the caller says how many tokens
+        # each request brings, the kernel's rows are the short ones only; otherwise it goes over
+        # every row of the step and leaves the portions' alone.
+        single_tokens = decode(short_rows if host_q_lens is not None else 0)
         if not MIXED_OVERLAP or torch.cuda.is_current_stream_capturing():
             portions()
             single_tokens()
@@ -256,22 +272,12 @@ def _paged_attention_mma(q, out, k_cache, v_cache, block_tables, req_q_start, re
             join.record(side)
         main.wait_event(join)
         return out
-    ps, np_ = 1 << 30, 1
-    if has_short and not has_long:
-        ps, np_ = partitions or plan_decode_partitions(short_rows, KV, H // KV, max_context, span, hd)
-    part_m = part_l = part_acc = None
-    if np_ > 1:
-        part_m = torch.empty(T * H * np_, device=q.device, dtype=torch.float32)
-        part_l = torch.empty_like(part_m)
-        part_acc = torch.empty(T * H * np_ * hd, device=q.device, dtype=torch.float32)
-    check(lib().asb_paged_attention_mma_masked(
-        ptr(out), ptr(q), ptr(k_cache), ptr(v_cache), ptr(block_tables), ptr(req_q_start),
-        ptr(req_pos_start), ptr(part_m), ptr(part_l), ptr(part_acc), ptr(sink), T, num_requests, H, KV, hd, bs,
-        block_tables.shape[1], win, chunk, ps, np_, float(scale), softcap, int(has_short), int(has_long), int(all_single), 0,
-        stream()))  # fmt: skip
-    if np_ > 1:
-        check(lib().asb_attention_reduce(ptr(out), ptr(part_m), ptr(part_l), ptr(part_acc), T * H, np_, hd,
-                                         dtype_code(q), stream()))  # fmt: skip
+    if has_long:
+        check(lib().asb_prefill_attention_mma(
+            ptr(out), ptr(q), ptr(k_cache), ptr(v_cache), ptr(block_tables), ptr(req_q_start), ptr(req_pos_start), ptr(sink),
+            T, num_requests, H, KV, hd, bs, block_tables.shape[1], win, chunk, float(scale), softcap, stream()))  # fmt: skip
+    if has_short:
+        decode(short_rows if has_long and host_q_lens is not None else 0)()
     return out
 
 

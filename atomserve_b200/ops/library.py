@@ -32,7 +32,7 @@ _SIGNATURES = {
     "asb_silu_mul": [_P, _P, _I, _I, _I, _P],
     "asb_qk_norm_rope_store": [_P] * 9 + [_I] * 6 + [_F, _I, _P],
     "asb_paged_attention": [_P] * 10 + [_I] * 10 + [_F, _I, _P],
-    "asb_paged_attention_mma": [_P] * 10 + [_I] * 10 + [_F, _I, _I, _I, _I, _P],
+    "asb_decode_attention": [_P] * 9 + [_I] * 10 + [_F, _F, _I, _I, _I, _P],
     "asb_prefill_attention_tcgen05": [_P] * 7 + [_I] * 9 + [_F, _P, _P],
     "asb_attention_tcgen05_supported": [_I, _I, _I],
     "asb_attention_reduce": [_P, _P, _P, _P, _I, _I, _I, _I, _P],
@@ -75,7 +75,6 @@ _SIGNATURES = {
     "asb_softcap": [_P, ctypes.c_longlong, _F, _P],
     # attention with a sink in the softmax's denominator
     "asb_paged_attention_sink": [_P] * 11 + [_I] * 10 + [_F, _I, _P],
-    "asb_paged_attention_mma_sink": [_P] * 11 + [_I] * 10 + [_F, _I, _I, _I, _I, _P],
     "asb_prefill_attention_tcgen05_sink": [_P] * 8 + [_I] * 9 + [_F, _P, _P],
     # blocks with the norm on the sublayer's output, and their mixers
     "asb_residual_out_norm": [_P] * 10 + [_I, _I, _F, _F, _I, _I, _P],
@@ -103,7 +102,7 @@ _SIGNATURES = {
     "asb_moe_combine_identity": [_P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _P, _P, _I, _I, _P],
     # attention within chunks of the sequence and with capped scores
     "asb_paged_attention_masked": [_P] * 11 + [_I] * 11 + [_F, _F, _I, _P],
-    "asb_paged_attention_mma_masked": [_P] * 11 + [_I] * 11 + [_F, _F, _I, _I, _I, _I, _P],
+    "asb_prefill_attention_mma": [_P] * 8 + [_I] * 9 + [_F, _F, _P],
     "asb_prefill_attention_tcgen05_masked": [_P] * 8 + [_I] * 10 + [_F, _F, _P, _P],
     # layers whose two sublayers read one stream; a hashed table of token pairs; a product over two streams
     "asb_residual_terms_norm": [_P] * 8 + [_F] * 4 + [_I] + [_P] * 3 + [_I, _I, _F, _I, _P],

@@ -852,3 +852,43 @@ def test_gemm_tcgen05_on_pairs_of_sms(ops, M, N, K, rows):
     if fused is not None:
         gate, up = ref[:, 0::2], ref[:, 1::2]
         assert torch.allclose(fused.double().cpu(), gate / (1 + torch.exp(-gate)) * up, atol=3e-2, rtol=3e-2)
+
+
+@pytest.mark.parametrize("lens,H,KV,hd,bs,window,ranges", [
+    ([1], 8, 2, 128, 16, None, 7),                                    # more ranges than tiles
+    ([1, 64, 65, 129, 4000], 8, 2, 128, 16, None, 13),                # ranges over several rows and within one
+    ([1 + (53 * i) % 700 for i in range(300)], 4, 2, 64, 8, None, 50),  # more rows than a round of the scan, rows of 1 to 11 tiles
+    ([500, 3, 2000, 777], 40, 2, 128, 16, 300, 31),                   # twenty heads a kv head: two chunks; a window
+    ([900] * 6, 16, 1, 64, 4, None, 64),                              # sixteen heads; every range ends inside a row
+])  # fmt: skip
+@pytest.mark.parametrize("stored", [False, True])
+def test_decode_attention_ranges(ops, monkeypatch, lens, H, KV, hd, bs, window, ranges, stored):
+    """The decode kernel's equal ranges of all rows' key tiles, for numbers of ranges that the planner would not take,
+    against the plain attention. bfloat16 values and probabilities: 2^-8 of values of size one, a few times over."""
+    import atomserve_b200.ops.attention as attention
+
+    rows = len(lens)
+    dev, dense, qs = paged_setup(lens, [1] * rows, H, KV, hd, bs, torch.bfloat16)
+    ref = attention_reference(qs, dense, lens, [1] * rows, window)
+    monkeypatch.setattr(attention, "plan_decode_ranges", lambda *a: ranges)
+    out = ops.paged_attention(**dev, num_requests=rows, max_context=max(lens), window=window, scale=hd**-0.5,
+                              host_q_lens=[1] * rows, earlier_keys_stored=stored)  # fmt: skip
+    assert torch.allclose(out.float().cpu(), ref, atol=2e-2, rtol=2e-2), float((out.float().cpu() - ref).abs().max())
+
+
+@pytest.mark.parametrize("lens,q_lens,ranges", [
+    ([900, 1200, 64, 700, 2100, 33], [2, 300, 1, 8, 1, 1], 11),       # short rows of one to eight tokens around a portion
+    ([70 + i for i in range(140)] + [400], [1] * 140 + [64], 29),     # more rows than a round of the scan, beside a portion
+])  # fmt: skip
+@pytest.mark.parametrize("known", [True, False])
+def test_decode_attention_ranges_in_mixed_steps(ops, monkeypatch, lens, q_lens, ranges, known):
+    """The same beside prompt portions, whose rows the decode kernel leaves alone, with and without host knowledge of
+    what each request brings."""
+    import atomserve_b200.ops.attention as attention
+
+    dev, dense, qs = paged_setup(lens, q_lens, 10, 2, 128, 16, torch.bfloat16)
+    ref = attention_reference(qs, dense, lens, q_lens, None)
+    monkeypatch.setattr(attention, "plan_decode_ranges", lambda *a: ranges)
+    out = ops.paged_attention(**dev, num_requests=len(lens), max_context=max(lens), window=None, scale=128**-0.5,
+                              host_q_lens=q_lens if known else None, earlier_keys_stored=True)  # fmt: skip
+    assert torch.allclose(out.float().cpu(), ref, atol=2e-2, rtol=2e-2), float((out.float().cpu() - ref).abs().max())
