@@ -114,6 +114,23 @@ def plan_decode_ranges(rows: int, num_kv_heads: int, group: int, max_context: in
     return full if tiles >= 8 * full else max(1, min(3 * full // 4, tiles))
 
 
+def plan_portion_parts(q_lens: list[int] | None, num_kv_heads: int, group: int, max_context: int, window: int) -> int:
+    """Blocks (1, 2 or 4) that share the keys of each of the tcgen05 kernel's blocks (128 rows of one kv head's heads).
+    Two blocks an SM run at once; the choice minimises waves x (64-key tiles per block + 4 tiles' worth of start-up, and 2
+    more to merge), as if all tiles saw the longest context. Whole prompts that fill the device stay in one part."""
+    if q_lens is None:
+        return 1
+    tokens = 128 // group
+    blocks = sum(-(-n // tokens) for n in q_lens if n > SHORT_ROWS) * num_kv_heads
+    span = max_context if window <= 0 else min(max_context, window + tokens)
+    best = None
+    for parts in (1, 2, 4):
+        cost = -(-blocks * parts // TARGET_BLOCKS) * (-(-span // (64 * parts)) + 4 + (2 if parts > 1 else 0))
+        if best is None or cost < best[0]:
+            best = (cost, parts)
+    return best[1]
+
+
 def paged_attention(
     q: torch.Tensor,
     k_cache: torch.Tensor,
@@ -245,7 +262,7 @@ def _paged_attention_mma(q, out, k_cache, v_cache, block_tables, req_q_start, re
             check(lib().asb_prefill_attention_tcgen05_masked(
                 ptr(out), ptr(q), ptr(k_cache), ptr(v_cache), ptr(block_tables), ptr(req_q_start), ptr(req_pos_start), ptr(sink),
                 T, num_requests, H, KV, hd, bs, k_cache.shape[0], block_tables.shape[1], win, chunk, float(scale), softcap,
-                ptr(gemm_status(q.device)), stream()))  # fmt: skip
+                plan_portion_parts(host_q_lens, KV, H // KV, max_context, span), ptr(gemm_status(q.device)), stream()))  # fmt: skip
 
         if not has_short:
             portions()

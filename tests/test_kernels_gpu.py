@@ -892,3 +892,27 @@ def test_decode_attention_ranges_in_mixed_steps(ops, monkeypatch, lens, q_lens, 
     out = ops.paged_attention(**dev, num_requests=len(lens), max_context=max(lens), window=None, scale=128**-0.5,
                               host_q_lens=q_lens if known else None, earlier_keys_stored=True)  # fmt: skip
     assert torch.allclose(out.float().cpu(), ref, atol=2e-2, rtol=2e-2), float((out.float().cpu() - ref).abs().max())
+
+
+@pytest.mark.parametrize("lens,q_lens,H,KV,window", [
+    ([700, 40, 65], [300, 40, 9], 32, 8, None),     # tiles that see fewer key tiles than there are parts, beside long ones
+    ([1500, 90], [130, 64], 10, 2, None),           # padding rows in every tile, an odd number of key tiles
+    ([1200, 300], [200, 100], 16, 1, 150),          # a window: parts in which a row sees nothing
+])  # fmt: skip
+@pytest.mark.parametrize("parts", [1, 2, 4])
+@pytest.mark.parametrize("with_sink", [False, True])
+def test_prefill_attention_tcgen05_in_parts(ops, monkeypatch, lens, q_lens, H, KV, window, parts, with_sink):
+    """Prompt portions whose key tiles are divided among the blocks of a cluster, against the general kernel in float32."""
+    import atomserve_b200.ops.attention as attention
+    from atomserve_b200.ops.linear import check_gemm_status
+
+    dev, dense, qs = paged_setup(lens, q_lens, H, KV, 128, 16, torch.bfloat16)
+    sink = torch.linspace(-2, 3, H, device="cuda") if with_sink else None
+    common = dict(num_requests=len(lens), max_context=max(lens), window=window, scale=128**-0.5, host_q_lens=q_lens, sink=sink)
+    wide = {k: (v.float() if v.dtype == torch.bfloat16 else v) for k, v in dev.items()}
+    ref = ops.paged_attention(**wide, **common, generic=True)
+    monkeypatch.setattr(attention, "plan_portion_parts", lambda *a: parts)
+    out = ops.paged_attention(**dev, **common)
+    check_gemm_status()
+    # bfloat16 values and probabilities: 2^-8 of values of size one, a few times over
+    assert torch.allclose(out.float(), ref, atol=2e-2, rtol=2e-2), float((out.float() - ref).abs().max())
