@@ -44,6 +44,7 @@
 
 // How the pair kernel cuts its last round of tiles along K (gemm_tcgen05_pair.cu).
 extern "C" long long asb_gemm_tcgen05_pair_cut(int M, int N, int K, int bn, int* out3);
+extern "C" long long asb_gemm_tcgen05_pair_swapped_cut(int M, int N, int K, int bn, int* out3);
 extern "C" double asb_gemm_tcgen05_pair_us_per_kb(int bn);
 
 namespace {
@@ -569,6 +570,7 @@ unsigned long long* g_stamps = nullptr;  // asb_gemm_tcgen05_timeline
 struct Plan {
   int swap, bn, bn_kernel, tiles_p, tiles_q, kb_per_tile, stream, blocks, max_slots;
   int stages, stage_size;
+  int wide;             // 0, or the tokens (a multiple of 32) of the tiles of 256 weight rows that pairs of SMs compute
   int pair;             // 0, or the weight rows (128 to 256 in steps of 32) of the tiles that pairs of SMs compute (gemm_tcgen05_pair.cu)
   long long workspace;  // float32 elements
 };
@@ -608,8 +610,15 @@ int stage_room(int bn_kernel) {
 //     tiles to fill the device the 256-row tile wins (gate/up at 2,048 tokens: 339 -> 268 us, the
 //     vendor library 284), and the 128-row tile where there are few weight rows and a few
 //     hundred tokens (o at 512 tokens on the 14B shape: 34.5 -> 27.6 us);
+//   tiles of 256 weight rows by 32 to 256 tokens on pairs of SMs (gemm_tcgen05_pair.cu, swapped), where one round holds
+//     all tiles: tokens are rounded up to 32 a tile only, and few tiles are cut along K. Qwen3-8B: down at 302 tokens
+//     44.5 -> 33.4 us, at 384 45.1 -> 36.6; o at 160 17.5 -> 14.1; qkv at 448 23.8 -> 21.2. (More rounds would pay for an
+//     epilogue that writes 64 bytes a token and warp: gate/up at 302 tokens 66.2 us in three rounds, 67.9 without.)
 //   swapped operands with the flattened K-block sequence cut into equal ranges, up to 512 tokens:
 //     the partial sums cost about 14 us, which only long K over few tokens repays (down at 200).
+// With 17 to 64 tokens and more than one round of those pair tiles whose rest can be cut (gate/up), the pair tiles also
+// take the place of the other two forms: gate/up of Qwen3-8B at 32 tokens 44.6 -> 40.8 us, at 64 44.0 -> 42.4 (at 8 tokens
+// 39.3 against 40.8, at 96 44.4 against 46.2).
 // With swapped operands, whole tiles are dealt round-robin unless cutting the flattened K-block
 // sequence into equal ranges shortens the busiest SM's share of the operand stream by more than
 // the partial sums cost to write and read back; unswapped single-SM tiles are never cut.
@@ -618,7 +627,7 @@ Plan make_plan(int M, int N, int K) {
   const int sms_now = sm_count();
   const int unswapped_tiles = ((M + BM - 1) / BM) * ((N + 255) / 256);
   const int kb_per_tile = (K + BK - 1) / BK;
-  pl.pair = 0;
+  pl.pair = pl.wide = 0;
   pl.swap = M <= 32 || (M <= BM && 2 * unswapped_tiles < sms_now) ? 1 : 0;
   pl.bn = pl.swap ? (M <= 16 ? 16 : (M <= 32 ? 32 : (M <= 64 ? 64 : 128))) : (N <= 128 ? 128 : 256);
   pl.bn_kernel = pl.bn;
@@ -631,6 +640,11 @@ Plan make_plan(int M, int N, int K) {
       const double cost = (double)((tiles + sms_now - 1) / sms_now) * (128 + bn);
       if (cost < best) { best = cost; pl.bn = bn; pl.bn_kernel = bn <= 128 ? 128 : 256; }
     }
+  }
+  if (M > 16 && M <= 64 && g_force_swap < 0 && (N + 255) / 256 > sms_now / 2) {
+    int cut[3];
+    const int bn = M <= 32 ? 32 : 64;
+    if (asb_gemm_tcgen05_pair_swapped_cut(M, N, K, bn, cut) > 0) pl.wide = bn;
   }
   if (M > BM && g_force_swap < 0) {
     const double kb = kb_per_tile;
@@ -658,10 +672,22 @@ Plan make_plan(int M, int N, int K) {
       cost += 5.98;
       if (cost < best) { best = cost; pl.swap = 0; pl.pair = bn; }
     }
+    // pairs of SMs on tiles of 256 weight rows by equal tiles of tokens, where one round holds them all
+    const int weight_tiles = (N + 255) / 256;
+    for (int n = (M + 255) / 256; n * weight_tiles <= pairs && n <= 4; ++n) {
+      const int bn = ((M + n - 1) / n + 31) / 32 * 32;
+      const double per_kb = asb_gemm_tcgen05_pair_us_per_kb(bn);
+      int cut[3];
+      const long long floats = asb_gemm_tcgen05_pair_swapped_cut(M, N, K, bn, cut);
+      double cost = 5.98 + (floats > 0 ? 2.0 * cut[2] * per_kb + 2.0 + 8.0 * floats / 6.0e6 : kb * per_kb);
+      const double memory = 11.0 + (double)N * K * 2 / 6.5e6;  // the weights' bytes
+      if (cost < memory) cost = memory;
+      if (cost < 0.97 * best) { best = cost; pl.swap = 0; pl.pair = 0; pl.wide = bn; }
+    }
     if (M <= 512) {
       const double share = (double)((N + BM - 1) / BM) * ((M + 255) / 256) * kb / sms_now;  // K blocks per SM
       const double cost = 14.0 + (share < 4 ? 4 : share) * 0.457;
-      if (cost < best) { best = cost; pl.swap = 1; pl.pair = 0; pl.bn = pl.bn_kernel = 256; }
+      if (cost < best) { best = cost; pl.swap = 1; pl.pair = pl.wide = 0; pl.bn = pl.bn_kernel = 256; }
     }
   }
   if (g_force_swap >= 0) {  // the tuning aid's choice
@@ -710,6 +736,7 @@ Plan make_plan(int M, int N, int K) {
     pl.max_slots = (int)((pl.kb_per_tile + shortest - 1) / shortest) + 1;
     pl.workspace = (long long)tiles * pl.max_slots * BM * pl.bn;
   }
+  if (g_force_swap == 3) pl.wide = g_force_bn;
   return pl;
 }
 
@@ -733,6 +760,9 @@ int launch(const CUtensorMap& mp, const CUtensorMap& mq, const GemmParams& p, co
 extern "C" int asb_gemm_tcgen05_pair(void* out, const void* x, const void* w, const void* residual, int M, int N,
                                      int K, int mode, int bn, float* workspace, int* status, const float* glu_bias,
                                      int glu_act, cudaStream_t stream);
+extern "C" int asb_gemm_tcgen05_pair_swapped(void* out, const void* x, const void* w, const void* residual, int M, int N,
+                                             int K, int mode, int bn, float* workspace, int* status,
+                                             const float* glu_bias, int glu_act, cudaStream_t stream);
 
 // Float32 workspace elements a call needs (0 when every tile is computed whole).
 extern "C" long long asb_gemm_tcgen05_workspace(int M, int N, int K, int* stream_out) {
@@ -740,6 +770,18 @@ extern "C" long long asb_gemm_tcgen05_workspace(int M, int N, int K, int* stream
   const Plan pl = make_plan(M, N, K);
   if (stream_out) *stream_out = pl.stream;
   return pl.workspace;
+}
+
+// The form of a call that takes the place of what asb_gemm_tcgen05_plan tells: pairs of SMs on tiles of 256 weight rows by
+// out4[0] tokens (0: not used), of which out4[1] run whole, and each of the others in out4[2] pieces of out4[3] stages (two K blocks).
+// Returns its workspace's float32 elements.
+extern "C" long long asb_gemm_tcgen05_wide_plan(int M, int N, int K, int* out4) {
+  out4[0] = out4[1] = out4[2] = out4[3] = 0;
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  const Plan pl = make_plan(M, N, K);
+  if (!pl.wide) return 0;
+  out4[0] = pl.wide;
+  return asb_gemm_tcgen05_pair_swapped_cut(M, N, K, pl.wide, out4 + 1);
 }
 
 // Profiling aid: later calls write their timeline (see GemmParams::stamps) into `buffer`, device
@@ -799,6 +841,8 @@ static int gemm_tcgen05_run(void* out, const void* x, const void* w, const void*
   const Plan pl = make_plan(M, N, K);
   if (mode == 3 && !(pl.stream && pl.swap && pl.tiles_q == 1))
     return asb::fail("gemm_tcgen05: [%d, %d] x [%d, %d] does not run with partial sums", M, K, N, K);
+  if (pl.wide && mode != 3)
+    return asb_gemm_tcgen05_pair_swapped(out, x, w, residual, M, N, K, mode, pl.wide, workspace, status, glu_bias, glu_act, stream);
   if (pl.pair && mode != 3)
     return asb_gemm_tcgen05_pair(out, x, w, residual, M, N, K, mode, pl.pair, workspace, status, glu_bias, glu_act, stream);
   if (pl.workspace > 0 && !workspace) return asb::fail("gemm_tcgen05: this shape needs a workspace of %lld floats", pl.workspace);

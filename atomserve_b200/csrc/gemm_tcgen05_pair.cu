@@ -10,6 +10,11 @@
 // wakes, TMA request, L2 latency, barrier, MMA thread wakes) is longer than the MMAs of the other
 // three (csrc/gemm_tcgen05.cu has that kernel and the swapped, few-token forms).
 //
+// The operands can also swap (Swap): the pair's 256 rows are weight rows and its columns a tile of 32 to 256 tokens. A few
+// hundred tokens then pay for their own number rounded up to 32 instead of to 128 or 256, each weight is read from
+// memory once, and long K over few weight rows is cut among the pairs. Everything below holds with "token rows" and
+// "weight rows" exchanged; the epilogue's lanes are output columns.
+//
 // Roles per CTA: warps 0 and 6-8 load (TMA, no multicast), warp 1 of the even CTA issues the pair's MMAs,
 // warps 2-5 run the epilogue for the CTA's 128 token rows. Barriers: full[s] lives in the even
 // CTA and counts both CTAs' arrivals and bytes (the odd CTA's TMA completes there through the
@@ -30,7 +35,7 @@ namespace {
 
 using namespace asb::t5;
 
-constexpr int BM = 128;  // token rows per CTA
+constexpr int BM = 128;  // rows of the first operand (tokens, or weights with Swap) per CTA
 constexpr int BK = 64;   // K elements per stage: 128 bytes, one swizzle atom
 constexpr int UMMA_K = 16;
 constexpr int kMaxLoaders = 4;   // threads that request operands, a warp each: warps 0, 6, 7, 8
@@ -46,14 +51,15 @@ struct PairParams {
   int glu_act;            // kStoreSwiGLU: the gate's activation (asb::GluAct)
   int M, N, ldo;
   int epilogue;
-  int bn;                  // weight rows per tile: a multiple of 32, at most the kernel's BN
-  int tiles_m, num_tiles;  // tile t -> tokens (t % tiles_m) * 256, weight rows (t / tiles_m) * bn
+  int bn;                  // weight rows (tokens with Swap) per tile: a multiple of 32, at most the kernel's BN
+  int tiles_in, num_tiles;  // tile t -> tokens (t % tiles_in) * 256, weight rows (t / tiles_in) * bn; with Swap tokens
+                           // (t % tiles_in) * bn, weight rows (t / tiles_in) * 256: tiles of the same weights are neighbours
   int kb_per_tile;
   // The last, partial round of tiles can be cut along K so that every pair has a share of it:
   // tiles [0, whole_tiles) are dealt whole, round-robin; each later tile is computed by `split`
   // pairs, piece j taking the stages [j * piece_stages, (j + 1) * piece_stages) of the tile's K
   // and leaving its float32 sums in workspace slot (tile - whole_tiles) * split + j, a slot being
-  // [256 tokens][BN]; tail_reduce_kernel adds the slots up and stores the result. With
+  // [256 tokens][BN] ([BN tokens][256] with Swap); tail_reduce_kernel adds the slots up and stores the result. With
   // whole_tiles = num_tiles nothing is cut.
   float* workspace;
   int whole_tiles, split, piece_stages;
@@ -72,7 +78,7 @@ struct PairConfig {
   static constexpr int kRoom = 227 * 1024 - 1024 - 384;
   static constexpr int kStages = kRoom / kStage > 10 ? 10 : kRoom / kStage;
   static constexpr int kSmem = kStages * kStage + 1024 + 384;
-  static constexpr int kTmemCols = 2 * BN;          // two accumulators of BN columns
+  static constexpr int kTmemCols = 2 * BN <= 128 ? 128 : (2 * BN <= 256 ? 256 : 512);  // two accumulators of BN columns, a power of two
   // Loader j takes the stages j, j + kLoaders, ...: never more loaders than slots, or two of them
   // would wait for the same slot's same phase (and a step of more than kStages slots would leave
   // the ring: an earlier build did, and faulted).
@@ -102,6 +108,11 @@ __device__ __forceinline__ void mbar_expect_tx_cluster(uint32_t cluster_bar, uin
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
 }
+template <bool Swap>
+__device__ __forceinline__ int first_tile(const PairParams& p, int t) { return Swap ? t / p.tiles_in : t % p.tiles_in; }  // of 256 rows
+template <bool Swap>
+__device__ __forceinline__ int second_tile(const PairParams& p, int t) { return Swap ? t % p.tiles_in : t / p.tiles_in; }  // of bn rows
+
 // A TMA tile load (no multicast) whose bytes are counted on a barrier of the CTA pair.
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, uint32_t cluster_bar, int x, int y) {
   asm volatile(
@@ -124,9 +135,10 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
                ::"r"(bar), "h"(both) : "memory");
 }
 
-template <int BN>
+// map_a: the operand of 256 rows a tile (x, or w with Swap); map_b: that of bn rows.
+template <int BN, bool Swap>
 __global__ void __launch_bounds__(kThreads, 1)
-gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
+gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                          const PairParams p) {
   using C = PairConfig<BN>;
   extern __shared__ unsigned char smem_raw[];
@@ -191,11 +203,11 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
       int item = 0, ks = 0, s = 0;   // work item, stage within it, slot
       int len = item_len(0);
       uint32_t phase = 0;
-      int x0 = 0, w0 = 0, k0 = 0;    // the item's token rows, weight rows and first stage of K
+      int a0 = 0, b0 = 0, k0 = 0;    // this CTA's rows of the item's operands, and its first stage of K
       auto place = [&]() {
         const int t = item_tile(item);
-        x0 = (t % p.tiles_m) * 256 + (int)rank * BM;
-        w0 = (t / p.tiles_m) * p.bn + (int)rank * (p.bn / 2);
+        a0 = first_tile<Swap>(p, t) * 256 + (int)rank * BM;
+        b0 = second_tile<Swap>(p, t) * p.bn + (int)rank * (p.bn / 2);
         k0 = item < n_whole ? 0 : piece_begin;
       };
       auto advance = [&](int by) {
@@ -206,6 +218,12 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
         s += by;  // by <= kLoaders <= kStages: at most one turn of the ring
         if (s >= C::kStages) { s -= C::kStages; phase ^= 1u; }
       };
+      auto load_a = [&](uint32_t dst, uint32_t bar, int j) { tma_load_2d_pair(dst + j * C::kA, &map_a, bar, ((k0 + ks) * C::kSub + j) * BK, a0); };
+      auto load_b = [&](uint32_t dst, uint32_t bar, int j) {
+        tma_load_2d_pair(dst + C::kSub * C::kA + j * C::kB, &map_b, bar, ((k0 + ks) * C::kSub + j) * BK, b0);
+      };
+      auto load_weights = [&](uint32_t dst, uint32_t bar, int j) { if (Swap) load_a(dst, bar, j); else load_b(dst, bar, j); };
+      auto load_tokens = [&](uint32_t dst, uint32_t bar, int j) { if (Swap) load_b(dst, bar, j); else load_a(dst, bar, j); };
       place();
       advance(me);
       // the weights, which no kernel writes, fill the pipeline before the wait for the previous kernel
@@ -217,8 +235,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
           const uint32_t bar = cluster_address(full_bar(s), 0);
           mbar_expect_tx_cluster(bar, stage_bytes);
 #pragma unroll
-          for (int j = 0; j < C::kSub; ++j)
-            tma_load_2d_pair(base + s * C::kStage + C::kSub * C::kA + j * C::kB, &map_w, bar, ((k0 + ks) * C::kSub + j) * BK, w0);
+          for (int j = 0; j < C::kSub; ++j) load_weights(base + s * C::kStage, bar, j);
           advance(C::kLoaders);
         }
         item = item1; ks = ks1; s = s1; len = len1; phase = phase1;
@@ -233,11 +250,10 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
           if (!mbar_wait(empty_bar(s), phase ^ 1u, p.status, 31)) break;
           mbar_expect_tx_cluster(bar, stage_bytes);
 #pragma unroll
-          for (int j = 0; j < C::kSub; ++j)
-            tma_load_2d_pair(dst + C::kSub * C::kA + j * C::kB, &map_w, bar, ((k0 + ks) * C::kSub + j) * BK, w0);
+          for (int j = 0; j < C::kSub; ++j) load_weights(dst, bar, j);
         }
 #pragma unroll
-        for (int j = 0; j < C::kSub; ++j) tma_load_2d_pair(dst + j * C::kA, &map_x, bar, ((k0 + ks) * C::kSub + j) * BK, x0);
+        for (int j = 0; j < C::kSub; ++j) load_tokens(dst, bar, j);
         advance(C::kLoaders);
       }
       if (me == 0) {
@@ -298,8 +314,69 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
       ok = __shfl_sync(0xffffffffu, ok_i, 0) != 0;
       if (!ok) break;
       fence_after_sync();
-      const int row = (t % p.tiles_m) * 256 + (int)rank * BM + quad * 32 + lane;  // this thread's token
-      const int n0 = (t / p.tiles_m) * p.bn;
+      const int row = first_tile<Swap>(p, t) * 256 + (int)rank * BM + quad * 32 + lane;  // this thread's token (weight row with Swap)
+      const int n0 = second_tile<Swap>(p, t) * p.bn;
+      if constexpr (Swap) {
+        // lanes are output columns, tensor-memory columns are tokens
+        const bool piece = (int)seg >= n_whole;
+        float* slot = p.workspace + (size_t)pair * 256 * BN + (int)rank * BM + quad * 32 + lane;
+#pragma unroll 1
+        for (int c = 0; c < p.bn; c += 32) {
+          const int tokens = min(32, p.M - (n0 + c));
+          if (tokens <= 0) break;  // uniform
+          uint32_t raw[32];
+          tmem_ld32(tmem_base + ((uint32_t)(quad * 32) << 16) + buf * BN + (uint32_t)c, raw);
+          if (piece) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              if (j < tokens) slot[(size_t)(c + j) * 256] = __uint_as_float(raw[j]);
+            continue;
+          }
+          if (p.epilogue == kStoreSwiGLU) {
+            // Weight rows alternate gate, up, which so sit in neighbouring lanes: of two tokens the even lane takes the
+            // first and the odd one the second, and each hands the other what it lacks. (With the even lanes alone at
+            // work the epilogue of a tile of 160 tokens took longer than its products.)
+            const int odd = lane & 1;
+            __nv_bfloat16* o = (__nv_bfloat16*)p.out + (size_t)(n0 + c + odd) * (p.ldo / 2) + row / 2;
+#pragma unroll
+            for (int j = 0; j < 32; j += 2) {
+              const float other = __shfl_xor_sync(0xffffffffu, __uint_as_float(odd ? raw[j] : raw[j + 1]), 1);
+              const float gate = odd ? other : __uint_as_float(raw[j]), up = odd ? __uint_as_float(raw[j + 1]) : other;
+              if (row < p.N && j + odd < tokens)
+                o[(size_t)j * (p.ldo / 2)] = __float2bfloat16_rn(asb::glu_pair(gate, up, p.glu_bias, row & ~1, p.glu_act));
+            }
+            continue;
+          }
+          if (row >= p.N) continue;
+          const size_t at = (size_t)(n0 + c) * p.ldo + row;
+          if (p.epilogue == kStoreF32) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              if (j < tokens) ((float*)p.out)[at + (size_t)j * p.ldo] = __uint_as_float(raw[j]);
+            continue;
+          }
+          if (p.epilogue == kStoreBf16Residual) {
+            const __nv_bfloat16* res = (const __nv_bfloat16*)p.residual + at;
+            __nv_bfloat16 rv[32];
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              if (j < tokens) rv[j] = res[(size_t)j * p.ldo];
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              if (j < tokens) raw[j] = __float_as_uint(__uint_as_float(raw[j]) + __bfloat162float(rv[j]));
+          }
+#pragma unroll
+          for (int j = 0; j < 32; ++j) {
+            float v = __uint_as_float(raw[j]);
+            if (p.epilogue == kStoreBf16Relu2) v = relu2(v);
+            if (j < tokens) ((__nv_bfloat16*)p.out)[at + (size_t)j * p.ldo] = __float2bfloat16_rn(v);
+          }
+        }
+        fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(cluster_address(acc_empty(buf), 0));
+        continue;
+      }
       if ((int)seg >= n_whole) {
         // a piece of a cut tile: the sums go to this pair's workspace slot as they are
         float* slot_row = p.workspace + ((size_t)pair * 256 + (size_t)((int)rank * BM + quad * 32 + lane)) * BN;
@@ -404,16 +481,18 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
 // Adds up the pieces of the tiles that the GEMM cut along K and stores them as the GEMM stores
 // whole tiles. grid = (cut tiles, pieces of a tile's 256 x BN elements); a thread owns four
 // consecutive weight rows of one token.
-template <int BN>
+template <int BN, bool Swap>
 __global__ void tail_reduce_kernel(const PairParams p) {
+  constexpr int kWide = Swap ? 256 : BN;  // weight rows of a slot
   const int cut = blockIdx.x, tile = p.whole_tiles + cut;
   const int i = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
-  const int r = i / BN, c = i % BN;
-  const int row = (tile % p.tiles_m) * 256 + r, n = (tile / p.tiles_m) * p.bn + c;
+  const int r = i / kWide, c = i % kWide;
+  const int row = Swap ? second_tile<Swap>(p, tile) * p.bn + r : first_tile<Swap>(p, tile) * 256 + r;
+  const int n = Swap ? first_tile<Swap>(p, tile) * 256 + c : second_tile<Swap>(p, tile) * p.bn + c;
   asb::pdl_wait();  // the GEMM has completed
   asb::pdl_launch_dependents();
-  if (i >= 256 * BN || c >= p.bn || row >= p.M || n >= p.N) return;
-  const float* ws = p.workspace + ((size_t)cut * p.split * 256 + r) * BN + c;
+  if (i >= 256 * BN || (Swap ? r : c) >= p.bn || row >= p.M || n >= p.N) return;
+  const float* ws = p.workspace + (size_t)cut * p.split * 256 * BN + (size_t)r * kWide + c;
   float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
   for (int j0 = 0; j0 < p.split; j0 += 4) {  // four loads in flight; the sum still runs in piece order
     float4 a[4];
@@ -458,10 +537,10 @@ int sm_count() {
   return count;
 }
 
-template <int BN>
-int launch_pairs(const CUtensorMap& mx, const CUtensorMap& mw, const PairParams& p, cudaStream_t stream) {
+template <int BN, bool Swap>
+int launch_pairs(const CUtensorMap& ma, const CUtensorMap& mb, const PairParams& p, cudaStream_t stream) {
   using C = PairConfig<BN>;
-  auto kern = gemm_tcgen05_pair_kernel<BN>;
+  auto kern = gemm_tcgen05_pair_kernel<BN, Swap>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem);
   if (e != cudaSuccess) return asb::fail("gemm_tcgen05_pair: shared memory %d: %s", C::kSmem, cudaGetErrorString(e));
   int pairs = sm_count() / 2;
@@ -482,10 +561,10 @@ int launch_pairs(const CUtensorMap& mx, const CUtensorMap& mw, const PairParams&
   config.numAttrs = asb::pdl_enabled() ? 2 : 1;
   asb::prefer_shared_carveout((const void*)kern);
   asb::count_launch();
-  cudaLaunchKernelEx(&config, kern, mx, mw, p);
+  cudaLaunchKernelEx(&config, kern, ma, mb, p);
   if (int rc = asb::check_launch("gemm_tcgen05_pair")) return rc;
   if (p.whole_tiles < p.num_tiles) {
-    asb::launch(tail_reduce_kernel<BN>, dim3(p.num_tiles - p.whole_tiles, 256 * BN / 4 / 256), 256, 0, stream, p);
+    asb::launch(tail_reduce_kernel<BN, Swap>, dim3(p.num_tiles - p.whole_tiles, 256 * BN / 4 / 256), 256, 0, stream, p);
     return asb::check_launch("gemm_tcgen05_pair tail_reduce");
   }
   return 0;
@@ -509,8 +588,10 @@ static int kernel_rows(int bn) { return bn <= 128 ? 128 : 256; }  // the instant
 // Tuning aid: 0 keeps every tile whole in the calls that follow, 1 (the default) lets the last round be cut.
 extern "C" void asb_gemm_tcgen05_pair_tune(int cut) { g_cut_enabled = cut; }
 
-extern "C" long long asb_gemm_tcgen05_pair_cut(int M, int N, int K, int bn, int* out3) {
-  const int tiles = ((M + 255) / 256) * ((N + bn - 1) / bn), pairs = sm_count() / 2;
+// `a_rows`, `b_rows`: rows of the operand of 256 and of bn rows a tile. A cut costs a launch of `launch_us` and the sums'
+// bytes at `tbs` TB/s.
+static long long cut_plan(int a_rows, int b_rows, int K, int bn, int slot_rows, double launch_us, double tbs, int* out3) {
+  const int tiles = ((a_rows + 255) / 256) * ((b_rows + bn - 1) / bn), pairs = sm_count() / 2;
   const int stages = ((K + BK - 1) / BK + 1) / 2;
   out3[0] = tiles; out3[1] = 1; out3[2] = stages;
   const int left = tiles % pairs;
@@ -522,9 +603,20 @@ extern "C" long long asb_gemm_tcgen05_pair_cut(int M, int N, int K, int bn, int*
   split = (stages + piece - 1) / piece;  // no empty piece
   const double us_per_stage = 2 * asb_gemm_tcgen05_pair_us_per_kb(bn);
   const double bytes = (double)left * split * 256 * bn * 4 * 2;
-  if ((stages - piece) * us_per_stage <= 3.0 + bytes / 3.0e6) return 0;
+  if ((stages - piece) * us_per_stage <= launch_us + bytes / (tbs * 1e6)) return 0;
   out3[0] = tiles - left; out3[1] = split; out3[2] = piece;
-  return (long long)left * split * 256 * kernel_rows(bn);  // a slot is as wide as the kernel's widest tile
+  return (long long)left * split * 256 * slot_rows;  // a slot is as wide as the kernel's widest tile
+}
+
+extern "C" long long asb_gemm_tcgen05_pair_cut(int M, int N, int K, int bn, int* out3) {
+  return cut_plan(M, N, K, bn, kernel_rows(bn), 3.0, 3.0, out3);
+}
+
+// The same with the operands swapped: tiles of 256 weight rows by bn tokens (whose sums come to less and stay in L2: fitted
+// to 130 to 512 tokens on the o and down projections of Qwen3-8B).
+static int swapped_kernel_tokens(int bn) { return bn <= 64 ? 64 : (bn <= 128 ? 128 : (bn <= 192 ? 192 : 256)); }
+extern "C" long long asb_gemm_tcgen05_pair_swapped_cut(int M, int N, int K, int bn, int* out3) {
+  return cut_plan(N, M, K, bn, swapped_kernel_tokens(bn), 2.0, 6.0, out3);
 }
 
 // out = x . w^T (+ residual) on pairs of SMs, for more than 128 tokens. x [M, K] and w [N, K]
@@ -533,9 +625,9 @@ extern "C" long long asb_gemm_tcgen05_pair_cut(int M, int N, int K, int bn, int*
 // bn: weight rows per pair tile: 128, or a multiple of 32 from 160 to 256 (one kernel, built for 256
 // rows, runs those: narrower tiles let one round of them occupy more pairs of SMs).
 // workspace: float32, asb_gemm_tcgen05_pair_cut(M, N, K, bn) elements (null if that is 0).
-extern "C" int asb_gemm_tcgen05_pair(void* out, const void* x, const void* w, const void* residual, int M, int N,
-                                     int K, int mode, int bn, float* workspace, int* status, const float* glu_bias,
-                                     int glu_act, cudaStream_t stream) {
+static int run_pairs(bool swap, void* out, const void* x, const void* w, const void* residual, int M, int N,
+                     int K, int mode, int bn, float* workspace, int* status, const float* glu_bias,
+                     int glu_act, cudaStream_t stream) {
   if (mode < 0 || mode == 3 || mode > 4) return asb::fail("gemm_tcgen05_pair: unknown mode %d", mode);
   if (mode == 4 && residual) return asb::fail("gemm_tcgen05_pair: the squared-ReLU form takes no residual");
   if (mode == 2 && (residual || N % 2)) return asb::fail("gemm_tcgen05_pair: the SwiGLU form takes no residual and an even N");
@@ -544,7 +636,8 @@ extern "C" int asb_gemm_tcgen05_pair(void* out, const void* x, const void* w, co
   if (K < 8 || K % 8) return asb::fail("gemm_tcgen05_pair: K = %d must be a positive multiple of 8 (16-byte TMA rows)", K);
   if (((uintptr_t)x & 15) || ((uintptr_t)w & 15)) return asb::fail("gemm_tcgen05_pair: operands must be 16-byte aligned");
   if (!status) return asb::fail("gemm_tcgen05_pair: a status word is required");
-  if (bn != 128 && !(bn >= 160 && bn <= 256 && bn % 32 == 0))
+  if (swap && !(bn >= 32 && bn <= 256 && bn % 32 == 0)) return asb::fail("gemm_tcgen05_pair: %d tokens per tile (a multiple of 32 to 256)", bn);
+  if (!swap && bn != 128 && !(bn >= 160 && bn <= 256 && bn % 32 == 0))
     return asb::fail("gemm_tcgen05_pair: %d weight rows per tile (128, or a multiple of 32 from 160 to 256)", bn);
   PairParams p;
   p.out = out;
@@ -557,21 +650,43 @@ extern "C" int asb_gemm_tcgen05_pair(void* out, const void* x, const void* w, co
   p.ldo = N;
   p.epilogue = mode == 4 ? kStoreBf16Relu2 : mode == 2 ? kStoreSwiGLU : (mode == 1 ? kStoreF32 : (residual ? kStoreBf16Residual : kStoreBf16));
   p.bn = bn;
-  p.tiles_m = (M + 255) / 256;
-  p.num_tiles = p.tiles_m * ((N + bn - 1) / bn);
+  const int a_rows = swap ? N : M, b_rows = swap ? M : N;
+  const int a_tiles = (a_rows + 255) / 256, b_tiles = (b_rows + bn - 1) / bn;
+  p.tiles_in = swap ? b_tiles : a_tiles;
+  p.num_tiles = a_tiles * b_tiles;
   p.kb_per_tile = (K + BK - 1) / BK;
   int cut[3];
-  const long long need = asb_gemm_tcgen05_pair_cut(M, N, K, bn, cut);
+  const long long need = swap ? asb_gemm_tcgen05_pair_swapped_cut(M, N, K, bn, cut) : asb_gemm_tcgen05_pair_cut(M, N, K, bn, cut);
   if (need > 0 && !workspace) return asb::fail("gemm_tcgen05_pair: this shape needs a workspace of %lld floats", need);
   p.workspace = workspace;
   p.whole_tiles = cut[0];
   p.split = cut[1];
   p.piece_stages = cut[2];
-  alignas(64) CUtensorMap mx, mw;
+  alignas(64) CUtensorMap ma, mb;
   const cuuint64_t strides[1] = {(cuuint64_t)K * 2};
-  const cuuint64_t dims_x[2] = {(cuuint64_t)K, (cuuint64_t)M}, dims_w[2] = {(cuuint64_t)K, (cuuint64_t)N};
-  const cuuint32_t box_x[2] = {(cuuint32_t)BK, (cuuint32_t)BM}, box_w[2] = {(cuuint32_t)BK, (cuuint32_t)(bn / 2)};
-  if (int rc = make_bf16_map(&mx, x, 2, dims_x, strides, box_x)) return rc;
-  if (int rc = make_bf16_map(&mw, w, 2, dims_w, strides, box_w)) return rc;
-  return bn == 128 ? launch_pairs<128>(mx, mw, p, stream) : launch_pairs<256>(mx, mw, p, stream);
+  const cuuint64_t dims_a[2] = {(cuuint64_t)K, (cuuint64_t)a_rows}, dims_b[2] = {(cuuint64_t)K, (cuuint64_t)b_rows};
+  const cuuint32_t box_a[2] = {(cuuint32_t)BK, (cuuint32_t)BM}, box_b[2] = {(cuuint32_t)BK, (cuuint32_t)(bn / 2)};
+  if (int rc = make_bf16_map(&ma, swap ? w : x, 2, dims_a, strides, box_a)) return rc;
+  if (int rc = make_bf16_map(&mb, swap ? x : w, 2, dims_b, strides, box_b)) return rc;
+  if (!swap) return bn == 128 ? launch_pairs<128, false>(ma, mb, p, stream) : launch_pairs<256, false>(ma, mb, p, stream);
+  switch (swapped_kernel_tokens(bn)) {
+    case 64: return launch_pairs<64, true>(ma, mb, p, stream);
+    case 128: return launch_pairs<128, true>(ma, mb, p, stream);
+    case 192: return launch_pairs<192, true>(ma, mb, p, stream);
+    default: return launch_pairs<256, true>(ma, mb, p, stream);
+  }
+}
+
+extern "C" int asb_gemm_tcgen05_pair(void* out, const void* x, const void* w, const void* residual, int M, int N,
+                                     int K, int mode, int bn, float* workspace, int* status, const float* glu_bias,
+                                     int glu_act, cudaStream_t stream) {
+  return run_pairs(false, out, x, w, residual, M, N, K, mode, bn, workspace, status, glu_bias, glu_act, stream);
+}
+
+// The same with the operands swapped: a pair's tile is 256 weight rows by bn tokens (a multiple of 32 up to 256; any number
+// of tokens). workspace: asb_gemm_tcgen05_pair_swapped_cut(M, N, K, bn) elements.
+extern "C" int asb_gemm_tcgen05_pair_swapped(void* out, const void* x, const void* w, const void* residual, int M, int N,
+                                             int K, int mode, int bn, float* workspace, int* status,
+                                             const float* glu_bias, int glu_act, cudaStream_t stream) {
+  return run_pairs(true, out, x, w, residual, M, N, K, mode, bn, workspace, status, glu_bias, glu_act, stream);
 }

@@ -77,6 +77,19 @@ def gemm_workspace(device: torch.device, floats: int) -> torch.Tensor:
 _WORKSPACE_FLOATS: dict[tuple[int, int, int], int] = {}
 
 
+def _workspace_floats(M: int, N: int, K: int) -> int:
+    need = _WORKSPACE_FLOATS.get((M, N, K))
+    if need is None:
+        query, wide = lib().asb_gemm_tcgen05_workspace, lib().asb_gemm_tcgen05_wide_plan
+        query.restype = wide.restype = ctypes.c_longlong
+        out = (ctypes.c_int * 4)()
+        need = wide(M, N, K, out)
+        if not out[0]:
+            need = query(M, N, K, None)
+        _WORKSPACE_FLOATS[(M, N, K)] = need
+    return need
+
+
 def gemm_tcgen05(x: torch.Tensor, w: torch.Tensor, residual: torch.Tensor | None, out_dtype: torch.dtype,
                  swiglu: bool = False, out: torch.Tensor | None = None, relu2: bool = False) -> torch.Tensor:  # fmt: skip
     """bfloat16 x [M, K] . w [N, K]^T on tcgen05 tensor cores (TMA operands, TMEM accumulator).
@@ -86,11 +99,7 @@ def gemm_tcgen05(x: torch.Tensor, w: torch.Tensor, residual: torch.Tensor | None
     N = w.shape[0]
     if out is None:
         out = torch.empty(M, N // 2 if swiglu else N, device=x.device, dtype=out_dtype)
-    need = _WORKSPACE_FLOATS.get((M, N, K))
-    if need is None:
-        query = lib().asb_gemm_tcgen05_workspace
-        query.restype = ctypes.c_longlong
-        need = _WORKSPACE_FLOATS[(M, N, K)] = query(M, N, K, None)
+    need = _workspace_floats(M, N, K)
     workspace = gemm_workspace(x.device, need) if need else None
     check(lib().asb_gemm_tcgen05(ptr(out), ptr(x), ptr(w), ptr(residual), M, N, K, 4 if relu2 else 2 if swiglu else int(out_dtype == torch.float32),
                                  ptr(workspace), ptr(gemm_status(x.device)), stream()))  # fmt: skip
@@ -129,6 +138,11 @@ def _plan(M: int, N: int, K: int) -> tuple[int, ...]:
     if plan is None:
         out = (ctypes.c_int * 8)()
         check(lib().asb_gemm_tcgen05_plan(M, N, K, out))
+        wide = (ctypes.c_int * 4)()
+        lib().asb_gemm_tcgen05_wide_plan.restype = ctypes.c_longlong
+        lib().asb_gemm_tcgen05_wide_plan(M, N, K, wide)
+        if wide[0]:
+            out[0] = 0  # that form takes the place of one that cuts K into partial sums
         plan = _PLANS[(M, N, K)] = tuple(out)
     return plan
 
@@ -164,8 +178,8 @@ def gemm_timeline(buffer: torch.Tensor | None) -> None:
 
 def gemm_tune(swap: int = -1, rows: int = 0, cut_last_round: bool = True) -> None:
     """Tuning aid: force how the tensor-core GEMM runs the calls that follow. swap 0: unswapped
-    tiles on single SMs, 1: swapped operands, 2: tiles on pairs of SMs, -1: the planner's choice;
-    rows: weight rows per unswapped tile (a multiple of 32, single SMs from 64 to 256, pairs from
+    tiles on single SMs, 1: swapped operands, 2: tiles on pairs of SMs, 3: the same with swapped operands (rows: tokens per
+    tile, a multiple of 32 up to 256), -1: the planner's choice; rows: weight rows per unswapped tile (a multiple of 32, single SMs from 64 to 256, pairs from
     128 to 256; 0: the planner's); cut_last_round: whether the pair form may cut its last round of
     tiles along K. The plans and workspace sizes remembered per shape are forgotten, because they
     differ between the forms."""
@@ -225,11 +239,7 @@ def linear_glu(x: torch.Tensor, w_interleaved: torch.Tensor, bias_interleaved: t
     if b is not None and (b.dtype != torch.float32 or b.shape != (N,) or not b.is_contiguous()):
         raise KernelLibraryError(f"linear_glu: bias must be contiguous float32 [{N}]")
     out = torch.empty(M, N // 2, device=x.device, dtype=torch.bfloat16)
-    need = _WORKSPACE_FLOATS.get((M, N, K))
-    if need is None:
-        query = lib().asb_gemm_tcgen05_workspace
-        query.restype = ctypes.c_longlong
-        need = _WORKSPACE_FLOATS[(M, N, K)] = query(M, N, K, None)
+    need = _workspace_floats(M, N, K)
     workspace = gemm_workspace(x.device, need) if need else None
     check(lib().asb_gemm_tcgen05_glu(ptr(out), ptr(x), ptr(w_interleaved), ptr(b), GLU_ACTIVATIONS[activation], M, N, K,
                                      ptr(workspace), ptr(gemm_status(x.device)), stream()))  # fmt: skip

@@ -916,3 +916,39 @@ def test_prefill_attention_tcgen05_in_parts(ops, monkeypatch, lens, q_lens, H, K
     check_gemm_status()
     # bfloat16 values and probabilities: 2^-8 of values of size one, a few times over
     assert torch.allclose(out.float(), ref, atol=2e-2, rtol=2e-2), float((out.float() - ref).abs().max())
+
+
+@pytest.mark.parametrize("tokens", [32, 64, 96, 160, 224, 256])
+@pytest.mark.parametrize("M,N,K", [(300, 512, 256), (33, 130, 72), (257, 4104, 520), (160, 6144, 4160), (5, 24576, 1024), (70, 256, 64),
+                                   (131, 2000, 12288), (513, 1000, 4160)])  # fmt: skip
+def test_gemm_tcgen05_on_pairs_of_sms_swapped(ops, M, N, K, tokens):
+    """The pair form with its operands swapped (tiles of 256 weight rows by 32 to 256 tokens), forced: every epilogue against
+    float64; tokens, weight rows and K that end inside a tile, one tile, more tiles than pairs, tiles cut along K."""
+    from atomserve_b200.ops.linear import check_gemm_status, gemm_tcgen05, gemm_tune
+
+    g = torch.Generator().manual_seed(M + N + K)
+    x = torch.randn(M, K, generator=g).bfloat16().cuda()
+    w = (torch.randn(N, K, generator=g) / math.sqrt(K)).bfloat16().cuda()
+    res = torch.randn(M, N, generator=g).bfloat16().cuda()
+    ref = x.double().cpu() @ w.double().cpu().T
+    gemm_tune(3, tokens)
+    try:
+        full = gemm_tcgen05(x, w, None, torch.float32)
+        plain_out = gemm_tcgen05(x, w, None, torch.bfloat16)
+        with_res = gemm_tcgen05(x, w, res, torch.bfloat16)
+        squared = gemm_tcgen05(x, w, None, torch.bfloat16, relu2=True)
+        fused = gemm_tcgen05(x, w, None, torch.bfloat16, swiglu=True)
+        again = gemm_tcgen05(x, w, None, torch.float32)
+        gemm_tune(3, tokens, cut_last_round=False)
+        uncut = gemm_tcgen05(x, w, None, torch.float32)
+    finally:
+        gemm_tune()
+    check_gemm_status()
+    assert torch.allclose(uncut, full, atol=1e-4, rtol=1e-4)  # cut or whole, the same products are added, in another order
+    assert torch.allclose(full.double().cpu(), ref, atol=2e-3, rtol=1e-3), float((full.double().cpu() - ref).abs().max())
+    assert torch.equal(again, full)
+    assert torch.allclose(plain_out.double().cpu(), ref, atol=3e-2, rtol=2e-2)
+    assert torch.allclose(with_res.double().cpu(), ref + res.double().cpu(), atol=3e-2, rtol=2e-2)
+    assert torch.allclose(squared.double().cpu(), ref.clamp_min(0) ** 2, atol=3e-2, rtol=2e-2)
+    gate, up = ref[:, 0::2], ref[:, 1::2]
+    assert torch.allclose(fused.double().cpu(), gate / (1 + torch.exp(-gate)) * up, atol=3e-2, rtol=3e-2)
