@@ -258,18 +258,37 @@ __device__ __forceinline__ DecodeRow row_after(const DecodeParams& p, Starts sta
   return no_row();
 }
 
-// Sum of the tiles of the rows below `upto` (every thread gets it; `scratch`: one word per warp).
-__device__ __forceinline__ int tiles_below(const DecodeParams& p, Starts starts, int upto, int* scratch) {
+// Sum over the block (every thread gets it; `scratch`: one word per warp).
+__device__ __forceinline__ int block_total(int v, int* scratch) {
+  v = __reduce_add_sync(0xffffffffu, v);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = v;
+  __syncthreads();
   int s = 0;
-  for (int i = threadIdx.x; i < upto; i += kThreads) s += decode_row(p, starts, i).tiles;
-  s = __reduce_add_sync(0xffffffffu, s);
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = s;
-  __syncthreads();
-  s = 0;
 #pragma unroll
   for (int w = 0; w < kThreads / 32; ++w) s += scratch[w];
   return s;
+}
+
+// Sum of the tiles of the rows below `upto`.
+__device__ __forceinline__ int tiles_below(const DecodeParams& p, Starts starts, int upto, int* scratch) {
+  int s = 0;
+  for (int i = threadIdx.x; i < upto; i += kThreads) s += decode_row(p, starts, i).tiles;
+  return block_total(s, scratch);
+}
+
+// Ranges that end with their rows: the fewest tiles a range such that every row cut into equal ranges of at most that many
+// leaves no more than p.ranges of them, if that is within what the equal ranges of the whole sequence have and kCrossing more;
+// else 0 (also with more rows than threads; `mine`: the tiles of row threadIdx.x). A block that walks from one row into
+// the next pays for a second merge and a second start, about three tiles' time: three requests of 500 to 1,500 keys, 32 heads
+// over 8, 12.5 -> 9.3 us.
+constexpr int kCrossing = 3;
+__device__ __forceinline__ int tiles_a_range(const DecodeParams& p, int mine, int total, int* scratch) {
+  if (p.rows > kThreads) return 0;
+  const int least = (total + p.ranges - 1) / p.ranges;
+  for (int c = least; c < least + kCrossing; ++c)
+    if (c > 0 && block_total((mine + c - 1) / c, scratch) <= p.ranges) return c;
+  return 0;
 }
 
 // A place in the sequence of tiles.
@@ -299,7 +318,7 @@ decode_attention_kernel(const __grid_constant__ DecodeParams p) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   constexpr int kTileBytes = kKeyTile * HD * 2;
   constexpr int kChunks = HD / 8;
-  __shared__ int scan[kThreads / 32], found[2], starts_at[kStarts];
+  __shared__ int scan[kThreads / 32], found[3], starts_at[kStarts];
   __shared__ float mm[4 * 16], ml[4 * 16];
   // [K stage 0][V stage 0][K stage 1][V stage 1][Q of two rows, 8 or 16 heads]; a merge uses the K and V of a tile
   // that has been read
@@ -318,15 +337,9 @@ decode_attention_kernel(const __grid_constant__ DecodeParams p) {
   DecodeCursor at;           // the tile being computed
   int n;                     // tiles of this block
   if (p.ranges > 0) {
-    const int total = tiles_below(p, starts, p.rows, scan), ranges = min(p.ranges, total);
-    if (range >= ranges) return;  // (uniform; none is empty below)
-    const int begin = (int)asb::range_begin(total, ranges, range);
-    n = (int)asb::range_begin(total, ranges, range + 1) - begin;
-    // the row that tile `begin` belongs to: a scan over the rows' tiles, as many rows at a time as there are threads
-    int above = 0;           // tiles of the rows before this round's
-    for (int i0 = 0;; i0 += kThreads) {
-      const int i = i0 + threadIdx.x;
-      const int mine = i < p.rows ? decode_row(p, starts, i).tiles : 0;
+    // A scan over a value per row, as many rows at a time as there are threads: this thread's row holds [from, to).
+    int from, to, above = 0;
+    auto scan_rows = [&](int mine) {
       int upto = mine;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -343,11 +356,38 @@ decode_attention_kernel(const __grid_constant__ DecodeParams p) {
         if (w < warp) upto += scan[w];
         round += scan[w];
       }
-      const int to = above + upto, from = to - mine;
-      if (begin >= from && begin < to) { found[0] = i; found[1] = begin - from; }
-      __syncthreads();
-      if (found[0] >= 0) break;
+      to = above + upto;
+      from = to - mine;
       above += round;
+    };
+    int mine = (int)threadIdx.x < p.rows ? decode_row(p, starts, threadIdx.x).tiles : 0;
+    const int total = p.rows <= kThreads ? block_total(mine, scan) : tiles_below(p, starts, p.rows, scan);
+    const int per = tiles_a_range(p, mine, total, scan);
+    if (per > 0) {           // ranges that end with their rows
+      const int cuts = (mine + per - 1) / per;
+      scan_rows(cuts);
+      if (range >= above) return;  // (uniform; some block has work, and waits)
+      if (range >= from && range < to) {
+        const int k = range - from;
+        found[0] = threadIdx.x;
+        found[1] = mine * k / cuts;
+        found[2] = mine * (k + 1) / cuts - found[1];
+      }
+      __syncthreads();
+      n = found[2];
+    } else {
+      const int ranges = min(p.ranges, total);
+      if (range >= ranges) return;
+      const int begin = (int)asb::range_begin(total, ranges, range);
+      n = (int)asb::range_begin(total, ranges, range + 1) - begin;
+      for (int i0 = 0;;) {   // the row that tile `begin` belongs to
+        scan_rows(mine);
+        if (begin >= from && begin < to) { found[0] = i0 + threadIdx.x; found[1] = begin - from; }
+        __syncthreads();
+        if (found[0] >= 0) break;
+        i0 += kThreads;
+        mine = i0 + (int)threadIdx.x < p.rows ? decode_row(p, starts, i0 + threadIdx.x).tiles : 0;
+      }
     }
     at.i = found[0];
     at.t = found[1];
@@ -678,10 +718,17 @@ decode_merge_kernel(const __grid_constant__ DecodeParams p) {
   int first = 0, last = 0, row = i;
   bool served = true;
   if (p.all_single) {
-    const int total = tiles_below(p, nullptr, p.rows, scan), ranges = min(p.ranges, total);
-    const int begin = tiles_below(p, nullptr, i, scan), tiles = decode_row(p, nullptr, i).tiles;
-    first = asb::block_of(total, ranges, begin);
-    last = asb::block_of(total, ranges, begin + tiles - 1);
+    const int mine = (int)threadIdx.x < p.rows ? decode_row(p, nullptr, threadIdx.x).tiles : 0;
+    const int total = p.rows <= kThreads ? block_total(mine, scan) : tiles_below(p, nullptr, p.rows, scan);
+    const int per = tiles_a_range(p, mine, total, scan), tiles = decode_row(p, nullptr, i).tiles;
+    if (per > 0) {
+      first = block_total((int)threadIdx.x < i ? (mine + per - 1) / per : 0, scan);
+      last = first + (tiles + per - 1) / per - 1;
+    } else {
+      const int ranges = min(p.ranges, total), begin = tiles_below(p, nullptr, i, scan);
+      first = asb::block_of(total, ranges, begin);
+      last = asb::block_of(total, ranges, begin + tiles - 1);
+    }
   } else if (p.short_rows == 0) {  // a launch over all rows of a step meets longer requests', which the decode kernel left alone
     served = decode_row(p, p.req_q_start, i).tiles > 0;
   }

@@ -578,6 +578,10 @@ struct Plan {
 // Tuning aid (asb_gemm_tcgen05_tune): orientation and tile width forced for the calls that follow.
 int g_force_swap = -1, g_force_bn = 0;
 
+// Most tokens for which the swapped pair tiles are considered: at 450 and 600 tokens they won call by call (qkv 23.8 -> 21.2 us)
+// and lost in a step of the whole model (6 layers of Qwen3-8B: 1,431 -> 1,503 us at 450).
+constexpr int kWideTokens = 400;
+
 int stage_room(int bn_kernel) {
   switch (bn_kernel) {
     case 16: return Config<16>::kStageRoom;
@@ -612,7 +616,7 @@ int stage_room(int bn_kernel) {
 //     hundred tokens (o at 512 tokens on the 14B shape: 34.5 -> 27.6 us);
 //   tiles of 256 weight rows by 32 to 256 tokens on pairs of SMs (gemm_tcgen05_pair.cu, swapped), where one round holds
 //     all tiles: tokens are rounded up to 32 a tile only, and few tiles are cut along K. Qwen3-8B: down at 302 tokens
-//     44.5 -> 33.4 us, at 384 45.1 -> 36.6; o at 160 17.5 -> 14.1; qkv at 448 23.8 -> 21.2. (More rounds would pay for an
+//     44.5 -> 33.4 us, at 384 45.1 -> 36.6; o at 160 17.5 -> 14.1. (More rounds would pay for an
 //     epilogue that writes 64 bytes a token and warp: gate/up at 302 tokens 66.2 us in three rounds, 67.9 without.)
 //   swapped operands with the flattened K-block sequence cut into equal ranges, up to 512 tokens:
 //     the partial sums cost about 14 us, which only long K over few tokens repays (down at 200).
@@ -674,7 +678,7 @@ Plan make_plan(int M, int N, int K) {
     }
     // pairs of SMs on tiles of 256 weight rows by equal tiles of tokens, where one round holds them all
     const int weight_tiles = (N + 255) / 256;
-    for (int n = (M + 255) / 256; n * weight_tiles <= pairs && n <= 4; ++n) {
+    for (int n = (M + 255) / 256; M <= kWideTokens && n * weight_tiles <= pairs && n <= 4; ++n) {
       const int bn = ((M + n - 1) / n + 31) / 32 * 32;
       const double per_kb = asb_gemm_tcgen05_pair_us_per_kb(bn);
       int cut[3];

@@ -98,37 +98,48 @@ def plan_decode_ranges(rows: int, num_kv_heads: int, group: int, max_context: in
                        partitions: tuple[int, int] | None = None) -> int:  # fmt: skip
     """Equal ranges into which the decode kernel cuts the keys of all rows, each for a block per kv head (and 16 of its
     heads); 0: each row is a range, and there is no merge. Where rows of the longest context would not be split, nothing
-    is. Otherwise as many ranges as the device holds at once, three blocks an SM, if that leaves a block eight key tiles
-    of the longest context; with less work three quarters of them, and no more than there are tiles: a merge of more
-    shares then costs more than the shorter walk saves (one request of 12,288 keys and 8 kv heads: 18.7 us in 16
-    ranges, 16.3 in 40, 19.3 in 55; of 2,048 keys: 10.8 us in 8, 9.4 in 32, 8.4 in 40; 64 requests of 300 to 3,000
-    keys: 90.3 us in 24, 78.4 in 55)."""
+    is, nor where rows of up to 24 key tiles make blocks for half of what the device holds at once (64 rows of 100 to 300
+    keys, 8 kv heads: 25.6 -> 16.5 us). Otherwise as many ranges as the device holds at once, three blocks an SM, if that
+    leaves a block eight key tiles of the longest context; with less work three quarters of them, and no more than there
+    are tiles: a merge of more shares then costs more than the shorter walk saves (one request of 12,288 keys and 8 kv
+    heads: 18.7 us in 16 ranges, 16.3 in 40, 19.3 in 55; of 2,048 keys: 10.8 us in 8, 9.4 in 32, 8.4 in 40; 64 requests
+    of 300 to 3,000 keys: 90.3 us in 24, 78.4 in 55)."""
     size, parts = partitions or plan_decode_partitions(rows, num_kv_heads, group, max_context, window, head_dim)
     if parts <= 1:
         return 0
     if partitions:
         return rows * parts
     resident = lib().asb_decode_attention_resident_blocks(head_dim) or 3 * 148
-    full = max(1, resident // (num_kv_heads * -(-group // 16)))
-    tiles = rows * -(-(min(max_context, window) if window > 0 else max_context) // 64)
+    lanes = num_kv_heads * -(-group // 16)
+    longest = -(-(min(max_context, window) if window > 0 else max_context) // 64)
+    if longest <= 24 and 2 * rows * lanes >= resident:
+        return 0
+    full, tiles = max(1, resident // lanes), rows * longest
     return full if tiles >= 8 * full else max(1, min(3 * full // 4, tiles))
 
 
 def plan_portion_parts(q_lens: list[int] | None, num_kv_heads: int, group: int, max_context: int, window: int) -> int:
-    """Blocks (1, 2 or 4) that share the keys of each of the tcgen05 kernel's blocks (128 rows of one kv head's heads).
-    Two blocks an SM run at once; the choice minimises waves x (64-key tiles per block + 4 tiles' worth of start-up, and 2
-    more to merge), as if all tiles saw the longest context. Whole prompts that fill the device stay in one part."""
-    if q_lens is None:
-        return 1
+    """Blocks (1, 2 or 4) that share the keys of each of the tcgen05 kernel's blocks (128 rows of one kv head's heads). By
+    the estimate: waves of two blocks an SM, each of its share of the longest context's 64-key tiles (a tile's time 1, and
+    1.3 where every SM has two blocks) and 4 tiles' time to start, 4 more to merge. (512 tokens, 32 heads over 8, one and
+    two parts: at position 0 13.2 and 14.7 us, at 1,000 28.5 and 24.7, at 7,000 115 and 77; 100 tokens at 5,000: 99.7, and
+    31.7 in four.) Divided only where that saves 15 % by the estimate: single tokens may run beside the portions."""
     tokens = 128 // group
-    blocks = sum(-(-n // tokens) for n in q_lens if n > SHORT_ROWS) * num_kv_heads
-    span = max_context if window <= 0 else min(max_context, window + tokens)
-    best = None
-    for parts in (1, 2, 4):
-        cost = -(-blocks * parts // TARGET_BLOCKS) * (-(-span // (64 * parts)) + 4 + (2 if parts > 1 else 0))
-        if best is None or cost < best[0]:
-            best = (cost, parts)
-    return best[1]
+    tiles = -(-(max_context if window <= 0 else min(max_context, window + tokens)) // 64)
+    if q_lens is None or tiles < 8:
+        return 1
+    return _portion_parts(sum(-(-n // tokens) for n in q_lens if n > SHORT_ROWS) * num_kv_heads, tiles)
+
+
+@functools.lru_cache(maxsize=4096)
+def _portion_parts(blocks: int, tiles: int) -> int:
+    def cost(parts):
+        now = blocks * parts
+        per_tile = 1 + 0.3 * min(1.0, max(0.0, 2 * now / TARGET_BLOCKS - 1))
+        return -(-now // TARGET_BLOCKS) * (-(-tiles // parts) * per_tile + (8 if parts > 1 else 4))
+
+    best = min((2, 4), key=cost)
+    return best if cost(best) < 0.85 * cost(1) else 1
 
 
 def paged_attention(
