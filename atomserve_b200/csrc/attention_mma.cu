@@ -336,6 +336,8 @@ decode_attention_kernel(const __grid_constant__ DecodeParams p) {
   const Starts starts = copy_starts(p, starts_at);
   DecodeCursor at;           // the tile being computed
   int n;                     // tiles of this block
+  // A block without work waits for the previous kernel before it leaves: a launch whose blocks all left without
+  // waiting would be over before that kernel, and whatever waits for this launch would not have waited for that one.
   if (p.ranges > 0) {
     // A scan over a value per row, as many rows at a time as there are threads: this thread's row holds [from, to).
     int from, to, above = 0;
@@ -366,7 +368,10 @@ decode_attention_kernel(const __grid_constant__ DecodeParams p) {
     if (per > 0) {           // ranges that end with their rows
       const int cuts = (mine + per - 1) / per;
       scan_rows(cuts);
-      if (range >= above) return;  // (uniform; some block has work, and waits)
+      if (range >= above) {    // (uniform; with no rows of this kernel's in the step, every block comes here)
+        asb::pdl_wait();
+        return;
+      }
       if (range >= from && range < to) {
         const int k = range - from;
         found[0] = threadIdx.x;
@@ -377,7 +382,10 @@ decode_attention_kernel(const __grid_constant__ DecodeParams p) {
       n = found[2];
     } else {
       const int ranges = min(p.ranges, total);
-      if (range >= ranges) return;
+      if (range >= ranges) {
+        asb::pdl_wait();
+        return;
+      }
       const int begin = (int)asb::range_begin(total, ranges, range);
       n = (int)asb::range_begin(total, ranges, range + 1) - begin;
       for (int i0 = 0;;) {   // the row that tile `begin` belongs to
@@ -398,7 +406,7 @@ decode_attention_kernel(const __grid_constant__ DecodeParams p) {
     at.d = decode_row(p, starts, at.i);
     n = at.d.tiles;
     if (n == 0) {
-      asb::pdl_wait();       // (every block of the launch may come here)
+      asb::pdl_wait();
       return;
     }
   }

@@ -894,6 +894,32 @@ def test_decode_attention_ranges_in_mixed_steps(ops, monkeypatch, lens, q_lens, 
     assert torch.allclose(out.float().cpu(), ref, atol=2e-2, rtol=2e-2), float((out.float().cpu() - ref).abs().max())
 
 
+@pytest.mark.parametrize("hd,group", [(64, 4), (128, 4), (128, 20)])
+def test_decode_launch_without_rows_keeps_the_order_of_kernels(ops, monkeypatch, hd, group):
+    """A step of long portions whose lengths the host does not tell: the decode kernel is launched and finds no row of
+    its own. What follows on the stream still comes after the portions' kernel: here a product of its output."""
+    import atomserve_b200.ops.attention as attention
+
+    monkeypatch.setattr(attention, "MIXED_OVERLAP", False)  # both kernels on one stream
+    KV, lens, q_lens = 2, [700, 1200, 64, 2000], [300, 500, 9, 1200]
+    H = KV * group
+    dev, dense, qs = paged_setup(lens, q_lens, H, KV, hd, 16, torch.bfloat16)
+    w = (torch.randn(256, H * hd, generator=torch.Generator().manual_seed(1)) * 0.05).bfloat16().cuda()
+    common = dict(num_requests=len(lens), max_context=max(lens), window=None, scale=hd**-0.5)
+    known = ops.paged_attention(**dev, **common, host_q_lens=q_lens)
+    ref = ops.paged_attention(**dev, **common)
+    torch.cuda.synchronize()
+    assert torch.allclose(ref.float(), known.float(), atol=2e-2, rtol=2e-2)  # (a portion's keys may be divided among blocks)
+    expect = ops.linear(ref.view(-1, H * hd), w)
+    assert attention.plan_decode_ranges(sum(q_lens), KV, group, max(lens), 0, hd, (64, 4)) > 0
+    for partitions in (None, (64, 4)):
+        torch.cuda.synchronize()
+        for _ in range(20):
+            out = ops.paged_attention(**dev, **common, partitions=partitions)
+            got = ops.linear(out.view(-1, H * hd), w)
+            assert torch.equal(out, ref) and torch.equal(got, expect)
+
+
 @pytest.mark.parametrize("lens,q_lens,H,KV,window", [
     ([700, 40, 65], [300, 40, 9], 32, 8, None),     # tiles that see fewer key tiles than there are parts, beside long ones
     ([1500, 90], [130, 64], 10, 2, None),           # padding rows in every tile, an odd number of key tiles
