@@ -114,7 +114,10 @@ parts_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __
     }
     tile -= n;
   }
-  if (r >= p.R) return;  // the whole block leaves before any barrier or allocation
+  if (r >= p.R) {  // the whole block leaves before any barrier or allocation
+    asb::pdl_wait();  // (a launch all of whose blocks left without it would be over before the stream's previous kernel)
+    return;
+  }
   const int q0 = tile * p.QT, nq = min(p.QT, q_len - q0);
   const int row0 = p.req_q_start[r] + q0, pos0 = p.req_pos_start[r] + q0;
   const int kvh = blockIdx.x % p.KV, head0 = kvh * p.G;

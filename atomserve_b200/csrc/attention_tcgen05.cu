@@ -138,7 +138,10 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
     }
     tile -= tiles;
   }
-  if (r >= p.R) return;  // the whole block (and cluster) leaves before any barrier or allocation
+  if (r >= p.R) {  // the whole block (and cluster) leaves before any barrier or allocation
+    asb::pdl_wait();  // (a launch all of whose blocks left without it would be over before the stream's previous kernel)
+    return;
+  }
   const int q0 = tile * p.QT;
   const int nq = min(p.QT, q_len - q0);
   const int row0 = p.req_q_start[r] + q0;

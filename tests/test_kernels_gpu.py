@@ -920,6 +920,36 @@ def test_decode_launch_without_rows_keeps_the_order_of_kernels(ops, monkeypatch,
             assert torch.equal(out, ref) and torch.equal(got, expect)
 
 
+@pytest.mark.parametrize("summed", [False, True])
+def test_portions_launch_without_tiles_keeps_the_order_of_kernels(ops, monkeypatch, summed):
+    """A step of short requests whose lengths the host does not tell: the portions' kernel is launched first and finds no
+    tile of its own. The decode kernel behind it still comes after what makes the queries, a product here."""
+    import atomserve_b200.ops.attention as attention
+
+    monkeypatch.setattr(attention, "MIXED_OVERLAP", False)  # both kernels on one stream
+    lens, q_lens, H, KV, hd = [700, 1200, 64, 2000] * 8, [1, 8, 2, 1] * 8, 8, 2, 128
+    dev, dense, qs = paged_setup(lens, q_lens, H, KV, hd, 16, torch.bfloat16)
+    T, parts = sum(q_lens), KV if summed else 1
+    g = torch.Generator().manual_seed(2)
+    x = torch.randn(T, 4096, generator=g).bfloat16().cuda()
+    w = (torch.randn(H * parts * hd, 4096, generator=g) / 64).bfloat16().cuda()
+
+    def queries():
+        q = ops.linear(x, w)
+        return q.view(T, H, KV, hd) if summed else q.view(T, H, hd)
+
+    common = dict(dev, num_requests=len(lens), max_context=max(lens), window=None, scale=hd**-0.5)
+    common["q"] = queries()
+    torch.cuda.synchronize()
+    ref = ops.paged_attention(**common)
+    known = ops.paged_attention(**common, host_q_lens=q_lens)
+    torch.cuda.synchronize()
+    assert torch.allclose(ref.float(), known.float(), atol=2e-2, rtol=2e-2)  # (shares of a row's keys may be others)
+    for _ in range(20):
+        common["q"] = queries()
+        assert torch.equal(ops.paged_attention(**common), ref)
+
+
 @pytest.mark.parametrize("lens,q_lens,H,KV,window", [
     ([700, 40, 65], [300, 40, 9], 32, 8, None),     # tiles that see fewer key tiles than there are parts, beside long ones
     ([1500, 90], [130, 64], 10, 2, None),           # padding rows in every tile, an odd number of key tiles
