@@ -674,18 +674,18 @@ decode_attention_kernel(const __grid_constant__ DecodeParams p) {
         float mx = -INFINITY;
 #pragma unroll
         for (int w = 0; w < 4; ++w)
-          if (ml[w * 16 + qr] > 0.f) mx = fmaxf(mx, mm[w * 16 + qr]);
+          if (ml[w * 16 + qr] != 0.f) mx = fmaxf(mx, mm[w * 16 + qr]);  // (zero: the warp saw no key; a sum that is NaN counts)
         float a = 0.f, den = 0.f;
 #pragma unroll
         for (int w = 0; w < 4; ++w)
-          if (ml[w * 16 + qr] > 0.f) {
+          if (ml[w * 16 + qr] != 0.f) {
             const float f = fast_exp2(mm[w * 16 + qr] - mx);
             den += ml[w * 16 + qr] * f;
             a += ma[(size_t)(w * gc + qr) * HD + col] * f;
           }
         if (p.sink && first_t == 0) {  // the sink counts once per row: with its first tile
           const float sk = p.sink[head0 + qr] * kLog2e;
-          if (den > 0.f) {
+          if (den != 0.f) {
             den += exp2f(sk - mx);  // (the sums stay relative to mx: nothing is rescaled)
           } else {
             mx = sk;
@@ -769,7 +769,7 @@ decode_merge_kernel(const __grid_constant__ DecodeParams p) {
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      if (!(s[u].y > 0.f)) continue;
+      if (s[u].y == 0.f) continue;
       const float m_new = fmaxf(mx, s[u].x), f_old = exp2f(mx - m_new), f = exp2f(s[u].x - m_new);
       den = den * f_old + s[u].y * f;
 #pragma unroll

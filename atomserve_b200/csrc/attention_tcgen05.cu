@@ -465,14 +465,14 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
       for (int s = 0; s < kMaxParts; ++s) {
         ml[s] = make_float2(-INFINITY, 0.f);
         if (s < p.parts) ml[s] = reinterpret_cast<const float2*>(cluster.map_shared_rank(smem_raw + kPartBytes, s))[row];
-        if (ml[s].y > 0.f) m = fmaxf(m, ml[s].x);
+        if (ml[s].y != 0.f) m = fmaxf(m, ml[s].x);  // (a sum of zero: no key seen there; one that is NaN counts)
       }
       if (qi < nq) {
         const int head = head0 + (row - qi * p.G);
         float l = 0.f, f[kMaxParts];
 #pragma unroll
         for (int s = 0; s < kMaxParts; ++s) {
-          f[s] = ml[s].y > 0.f ? fast_exp2(ml[s].x - m) : 0.f;
+          f[s] = ml[s].y != 0.f ? fast_exp2(ml[s].x - m) : 0.f;
           l += ml[s].y * f[s];
         }
         if (p.sink) l += exp2f(p.sink[head] * 1.4426950408889634f - m);
@@ -486,7 +486,7 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
           for (int i = 0; i < 8; ++i) v[i] = 0.f;
 #pragma unroll
           for (int s = 0; s < kMaxParts; ++s) {
-            if (!(f[s] > 0.f)) continue;  // (nothing there, or nothing that counts)
+            if (ml[s].y == 0.f) continue;
             const float* o = reinterpret_cast<const float*>(cluster.map_shared_rank(smem_raw, s));
 #pragma unroll
             for (int i = 0; i < 8; ++i) v[i] += o[(c + i) * kRows + row] * f[s];

@@ -974,6 +974,29 @@ def test_prefill_attention_tcgen05_in_parts(ops, monkeypatch, lens, q_lens, H, K
     assert torch.allclose(out.float(), ref, atol=2e-2, rtol=2e-2), float((out.float() - ref).abs().max())
 
 
+@pytest.mark.parametrize("bad", [math.nan, math.inf])
+@pytest.mark.parametrize("where", [5, 700, 1500])
+@pytest.mark.parametrize("q_lens,shares", [([1, 1, 1], 0), ([1, 1, 1], 2), ([1, 1, 1], 17), ([200, 90, 64], 1), ([200, 90, 64], 2), ([200, 90, 64], 4)])
+@pytest.mark.parametrize("with_sink", [False, True])
+def test_a_key_that_is_not_finite_shows_however_keys_are_shared(ops, monkeypatch, bad, where, q_lens, shares, with_sink):
+    """One key of request 0 (kv head 1) with a NaN or an infinity: exactly the outputs that see it are NaN, whether a row's
+    keys are one walk or shares that are merged (the decode kernel's ranges, the parts of a portion)."""
+    import atomserve_b200.ops.attention as attention
+
+    lens, H, KV, hd, bs = [1600, 300, 700], 8, 2, 128, 16
+    dev, dense, qs = paged_setup(lens, q_lens, H, KV, hd, bs, torch.bfloat16)
+    dev["k_cache"][dev["block_tables"][0, where // bs].long(), 1, where % bs] = bad
+    sink = torch.linspace(-2, 3, H, device="cuda") if with_sink else None
+    monkeypatch.setattr(attention, "plan_decode_ranges", lambda *a: shares)
+    monkeypatch.setattr(attention, "plan_portion_parts", lambda *a: shares)
+    out = ops.paged_attention(**dev, num_requests=3, max_context=max(lens), window=None, scale=hd**-0.5, host_q_lens=q_lens, sink=sink)
+    sees = torch.arange(lens[0] - q_lens[0], lens[0]) >= where  # by position, of request 0's rows
+    expect = torch.zeros(sum(q_lens), H, dtype=torch.bool)
+    expect[: q_lens[0], H // KV :] = sees[:, None]
+    got = torch.isnan(out).cpu()
+    assert torch.equal(got.all(-1), expect) and torch.equal(got.any(-1), expect)
+
+
 @pytest.mark.parametrize("tokens", [32, 64, 96, 160, 224, 256])
 @pytest.mark.parametrize("M,N,K", [(300, 512, 256), (33, 130, 72), (257, 4104, 520), (160, 6144, 4160), (5, 24576, 1024), (70, 256, 64),
                                    (131, 2000, 12288), (513, 1000, 4160)])  # fmt: skip
