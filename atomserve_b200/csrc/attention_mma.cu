@@ -177,13 +177,14 @@ struct DecodeParams {
   float softcap;             // 0: none; else score <- softcap tanh(score / softcap)
   int all_single;            // every request brings exactly one token: request = row
   int short_rows;            // > 0: rows count only those of requests with at most kShortRows tokens
-  int early;                 // 1: keys below a request's first new position were written before the stream's previous kernel began
+  int early;                 // 1: the index arrays, and the keys below a request's first new position, were written before the
+                             // stream's previous kernel was launched; else nothing is read before the wait for it
   int ranges;                // 0: a range is a row, whatever its length
   float scale;
 };
 
-// One row of the launch. The index arrays were uploaded before the step's first kernel and are read before the wait
-// for the previous one, from L2: an SM's L1 could still hold their lines from an earlier step.
+// One row of the launch. The index arrays may be read before the wait for the previous kernel (`early`), and so from
+// L2: an SM's L1 could still hold their lines from an earlier step.
 struct DecodeRow {
   int row, r, pos, fresh;    // flat row, request, position, first position that this step writes
   int lo, tile0, tiles;      // first visible key, its tile, tiles to walk (0: not a row of this kernel)
@@ -333,6 +334,7 @@ decode_attention_kernel(const __grid_constant__ DecodeParams p) {
   const int range = blockIdx.x / p.lanes, head_lane = blockIdx.x - range * p.lanes;
   const int kvh = head_lane / p.HC, head0 = kvh * p.G + (head_lane - kvh * p.HC) * p.GC;
   const int gc = min(p.GC, kvh * p.G + p.G - head0);
+  if (!p.early) asb::pdl_wait();
   const Starts starts = copy_starts(p, starts_at);
   DecodeCursor at;           // the tile being computed
   int n;                     // tiles of this block
@@ -712,7 +714,7 @@ decode_attention_kernel(const __grid_constant__ DecodeParams p) {
 
 // Merges the rows that the ranges of the decode kernel cut: a block per (row, head). Which ranges hold a share of a row
 // follows from the rows' tiles: where a row's tiles are at hand (every request brings one token) that is worked out before
-// the wait (one request of 12,000 keys: 19.5 -> 17.5 us with the decode kernel), elsewhere the decode kernel says it.
+// the wait, from index arrays that are there: the decode kernel lets this one start after its own wait (or `early` says so) (one request of 12,000 keys: 19.5 -> 17.5 us with the decode kernel), elsewhere the decode kernel says it.
 template <int HD>
 __global__ void __launch_bounds__(kThreads)
 decode_merge_kernel(const __grid_constant__ DecodeParams p) {

@@ -52,6 +52,7 @@ struct PartsParams {
   int G, QT;                 // query heads per kv head, tokens per tile (128 / G)
   int window, keep;          // 0: none
   int k_stages;
+  int early;                 // 1: the index arrays were written before the stream's previous kernel was launched
   float scale_log2;          // softmax scale times log2(e)
 };
 
@@ -102,6 +103,7 @@ parts_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __
     return;
   }
 
+  if (!p.early) asb::pdl_wait();
   // Which request and tile of its tokens? (kv head fastest, late tiles first: the longest blocks start first)
   int tile = blockIdx.x / p.KV, r = 0, q_len = 0;
   for (; r < p.R; ++r) {
@@ -394,11 +396,11 @@ extern "C" int asb_attention_parts_tcgen05_supported(int hd, int group, int bloc
 }
 
 // Attention for every request that brings more than 8 tokens (others are left untouched). q
-// [T, H, KV, 128], out [T, H, 128] bfloat16; caches [num_blocks, KV, bs, 128].
+// [T, H, KV, 128], out [T, H, 128] bfloat16; caches [num_blocks, KV, bs, 128]. early: see PartsParams.
 extern "C" int asb_attention_parts_tcgen05(void* out, const void* q, const void* k_cache, const void* v_cache,
                                            const int* block_tables, const int* req_q_start, const int* req_pos_start,
                                            int num_tokens, int R, int H, int KV, int hd, int bs, int num_blocks,
-                                           int table_width, int window, int keep, float scale, int* status,
+                                           int table_width, int window, int keep, float scale, int early, int* status,
                                            cudaStream_t stream) {
   if (num_tokens == 0 || R == 0) return 0;
   if (KV < 1 || H % KV) return asb::fail("attention_parts_tcgen05: %d heads over %d kv heads", H, KV);
@@ -412,7 +414,7 @@ extern "C" int asb_attention_parts_tcgen05(void* out, const void* q, const void*
   p.R = R; p.H = H; p.KV = KV; p.bs = bs; p.table_width = table_width;
   p.G = H / KV;
   p.QT = kRows / p.G;
-  p.window = window; p.keep = window > 0 ? keep : 0;
+  p.window = window; p.keep = window > 0 ? keep : 0; p.early = early;
   p.scale_log2 = scale * 1.4426950408889634f;
   const int stages = resident_stages(KV);
   p.k_stages = stages ? stages : 3;

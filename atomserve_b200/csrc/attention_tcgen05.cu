@@ -85,6 +85,7 @@ struct AttnParams {
   float cap_log2;            // 0: none; else softcap times log2(e): score <- softcap tanh(score / softcap)
   float scale_over_cap;      // 2 log2(e) scale / softcap: the exponent of the tanh's one exponential
   int parts;                 // blocks (a cluster) among which a tile's keys are divided: 1, 2 or 4
+  int early;                 // 1: the index arrays were written before the stream's previous kernel was launched
 };
 
 __device__ __forceinline__ float fast_exp2(float x) {
@@ -121,6 +122,7 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
     return;
   }
 
+  if (!p.early) asb::pdl_wait();
   // Which request and tile of its tokens? Only requests with more than kShortRows tokens count.
   // Blocks are numbered kv head fastest: the hardware hands blocks out in the order of their
   // numbers, so every kv head's block of a request's last tile (the one that sees the most keys)
@@ -516,13 +518,13 @@ extern "C" int asb_attention_tcgen05_supported(int hd, int group, int block_size
 
 // Attention for every request that brings more than 8 tokens in this step (others are left
 // untouched for the decode kernel). q, out: [T, H, 128] bfloat16; caches [num_blocks, KV, bs, 128].
-// chunk, softcap (0: none), parts: see AttnParams.
+// chunk, softcap (0: none), parts, early: see AttnParams.
 extern "C" int asb_prefill_attention_tcgen05_masked(void* out, const void* q, const void* k_cache, const void* v_cache,
                                                     const int* block_tables, const int* req_q_start,
                                                     const int* req_pos_start, const float* sink, int num_tokens, int R,
                                                     int H, int KV, int hd, int bs, int num_blocks, int table_width,
                                                     int window, int chunk, float scale, float softcap, int parts,
-                                                    int* status, cudaStream_t stream) {
+                                                    int early, int* status, cudaStream_t stream) {
   if (chunk < 0 || softcap < 0.f) return asb::fail("prefill_attention_tcgen05: chunk %d and softcap %f must not be negative", chunk, (double)softcap);
   if (num_tokens == 0 || R == 0) return 0;
   if (KV < 1 || H % KV) return asb::fail("prefill_attention_tcgen05: %d heads over %d kv heads", H, KV);
@@ -541,6 +543,7 @@ extern "C" int asb_prefill_attention_tcgen05_masked(void* out, const void* q, co
   p.window = window;
   p.chunk = chunk;
   p.parts = parts;
+  p.early = early;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.cap_log2 = softcap * 1.4426950408889634f;
   p.scale_over_cap = softcap > 0.f ? 2.f * p.scale_log2 / softcap : 0.f;
@@ -595,7 +598,7 @@ extern "C" int asb_prefill_attention_tcgen05_sink(void* out, const void* q, cons
                                                   int window, float scale, int* status, cudaStream_t stream) {
   return asb_prefill_attention_tcgen05_masked(out, q, k_cache, v_cache, block_tables, req_q_start, req_pos_start, sink,
                                               num_tokens, R, H, KV, hd, bs, num_blocks, table_width, window, 0, scale,
-                                              0.f, 1, status, stream);
+                                              0.f, 1, 0, status, stream);
 }
 
 extern "C" int asb_prefill_attention_tcgen05(void* out, const void* q, const void* k_cache, const void* v_cache,

@@ -182,8 +182,9 @@ def paged_attention(
     products with all kv heads' keys (its values are still those of its own kv head): how scores that
     are mixed across heads run, the mix being part of the queries.
 
-    `earlier_keys_stored`: the keys below every request's `req_pos_start` were written before the stream's previous
-    kernel was launched (by earlier steps, as in a model's step), so the decode kernel may read them while that kernel runs.
+    `earlier_keys_stored`: the keys below every request's `req_pos_start` and the index tensors were written before the
+    stream's previous kernel was launched (by earlier steps and by the step's upload, as in a model's step), so the kernels
+    may read them while that kernel runs. Without it they read nothing before that kernel has completed.
 
     bfloat16 with head size 64 or 128 runs the tensor-core kernels (decode kernel for requests
     that bring at most 8 tokens, prefill kernel for longer portions; `host_q_lens`, the tokens
@@ -221,7 +222,7 @@ def paged_attention(
                                     earlier_keys_stored)  # fmt: skip
     if q.dtype == torch.bfloat16 and not generic and summed and not chunk and not softcap and sink is None and lib().asb_attention_parts_supported(hd, H, KV):
         return _paged_attention_parts(q, out, k_cache, v_cache, block_tables, req_q_start, req_pos_start, num_requests, max_context,
-                                      win, keep, scale, partitions, host_q_lens)  # fmt: skip
+                                      win, keep, scale, partitions, host_q_lens, earlier_keys_stored)  # fmt: skip
     ps, np_ = partitions or plan_partitions(T, num_requests, KV, H // KV, max_context, span)
     part_m = part_l = part_acc = None
     if np_ > 1:
@@ -273,7 +274,7 @@ def _paged_attention_mma(q, out, k_cache, v_cache, block_tables, req_q_start, re
             check(lib().asb_prefill_attention_tcgen05_masked(
                 ptr(out), ptr(q), ptr(k_cache), ptr(v_cache), ptr(block_tables), ptr(req_q_start), ptr(req_pos_start), ptr(sink),
                 T, num_requests, H, KV, hd, bs, k_cache.shape[0], block_tables.shape[1], win, chunk, float(scale), softcap,
-                plan_portion_parts(host_q_lens, KV, H // KV, max_context, span), ptr(gemm_status(q.device)), stream()))  # fmt: skip
+                plan_portion_parts(host_q_lens, KV, H // KV, max_context, span), int(earlier_keys_stored), ptr(gemm_status(q.device)), stream()))  # fmt: skip
 
         if not has_short:
             portions()
@@ -332,7 +333,7 @@ def plan_parts_partitions(rows: int, heads: int, kv_heads: int, max_context: int
 
 
 def _paged_attention_parts(q, out, k_cache, v_cache, block_tables, req_q_start, req_pos_start, num_requests, max_context, win, keep,
-                           scale, partitions, host_q_lens):  # fmt: skip
+                           scale, partitions, host_q_lens, earlier_keys_stored):  # fmt: skip
     T, H, KV, hd = q.shape
     bs = k_cache.shape[2]
     lens = host_q_lens
@@ -352,7 +353,7 @@ def _paged_attention_parts(q, out, k_cache, v_cache, block_tables, req_q_start, 
 
         check(lib().asb_attention_parts_tcgen05(
             ptr(out), ptr(q), ptr(k_cache), ptr(v_cache), ptr(block_tables), ptr(req_q_start), ptr(req_pos_start), T, num_requests, H, KV, hd,
-            bs, k_cache.shape[0], block_tables.shape[1], win, keep, float(scale), ptr(gemm_status(q.device)), stream()))  # fmt: skip
+            bs, k_cache.shape[0], block_tables.shape[1], win, keep, float(scale), int(earlier_keys_stored), ptr(gemm_status(q.device)), stream()))  # fmt: skip
     elif has_long:
         launch(False, True, 1, 1, None, None, None, 0)
     if has_short:

@@ -103,7 +103,7 @@ _SIGNATURES = {
     # attention within chunks of the sequence and with capped scores
     "asb_paged_attention_masked": [_P] * 11 + [_I] * 11 + [_F, _F, _I, _P],
     "asb_prefill_attention_mma": [_P] * 8 + [_I] * 9 + [_F, _F, _P],
-    "asb_prefill_attention_tcgen05_masked": [_P] * 8 + [_I] * 10 + [_F, _F, _I, _P, _P],
+    "asb_prefill_attention_tcgen05_masked": [_P] * 8 + [_I] * 10 + [_F, _F, _I, _I, _P, _P],
     # layers whose two sublayers read one stream; a hashed table of token pairs; a product over two streams
     "asb_residual_terms_norm": [_P] * 8 + [_F] * 4 + [_I] + [_P] * 3 + [_I, _I, _F, _I, _P],
     "asb_partial_residual_terms_norm": [_P] * 4 + [_I] * 5 + [_F] + [_P] * 5 + [_F] * 4 + [_I] + [_P] * 2 + [_I, _I, _F, _P],
@@ -114,7 +114,7 @@ _SIGNATURES = {
     "asb_mixed_heads_prepare": [_P, _P] + [_I] * 5 + [_P] * 12 + [_I] * 10 + [_F, _F, _I, _P],
     "asb_paged_attention_parts": [_P] * 11 + [_I] * 13 + [_F, _F, _I, _P],
     "asb_attention_parts": [_P] * 10 + [_I] * 11 + [_F] + [_I] * 4 + [_P],
-    "asb_attention_parts_tcgen05": [_P] * 7 + [_I] * 10 + [_F, _P, _P],
+    "asb_attention_parts_tcgen05": [_P] * 7 + [_I] * 10 + [_F, _I, _P, _P],
     "asb_attention_parts_tcgen05_supported": [_I, _I, _I],
     "asb_attention_parts_supported": [_I, _I, _I],
     "asb_attention_parts_heads": [_I, _I],

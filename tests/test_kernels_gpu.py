@@ -920,6 +920,32 @@ def test_decode_launch_without_rows_keeps_the_order_of_kernels(ops, monkeypatch,
             assert torch.equal(out, ref) and torch.equal(got, expect)
 
 
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("q_lens", [[1] * 48, [1, 3, 8, 1] * 12, [200, 64, 9] * 4, [1, 90] * 12])
+def test_attention_reads_indexes_that_the_previous_kernel_writes(ops, monkeypatch, q_lens, hd):
+    """Positions that come from the library kernel right before (an argmax over wide rows, which lets its successor start
+    early): without `earlier_keys_stored` every attention kernel reads them only when that kernel has completed."""
+    import atomserve_b200.ops.attention as attention
+
+    monkeypatch.setattr(attention, "MIXED_OVERLAP", False)  # all kernels on one stream
+    R, V, H, KV, bs = len(q_lens), 200000, 8, 2, 16
+    width = V // bs // 8
+    g = torch.Generator().manual_seed(hd + R)
+    kc, vc = (torch.randn(64, KV, bs, hd, generator=g).bfloat16().cuda() for _ in range(2))
+    tables = torch.randint(0, 64, (R, width), generator=g).int().cuda()
+    q = torch.randn(sum(q_lens), H, hd, generator=g).bfloat16().cuda()
+    starts = torch.tensor([0] + list(torch.tensor(q_lens).cumsum(0)), dtype=torch.int32).cuda()
+    common = dict(num_requests=R, max_context=3300, window=None, scale=hd**-0.5, host_q_lens=q_lens)
+    for i in range(6):
+        at = torch.randint(0, 3000, (R,), generator=g)
+        marked = torch.zeros(R, V, device="cuda")
+        marked[torch.arange(R, device="cuda"), at.cuda()] = 1.0
+        ref = ops.paged_attention(q, kc, vc, tables, starts, at.int().cuda(), **common)
+        torch.cuda.synchronize()
+        out = ops.paged_attention(q, kc, vc, tables, starts, ops.argmax_rows(marked), **common)
+        assert torch.equal(out, ref), i
+
+
 @pytest.mark.parametrize("summed", [False, True])
 def test_portions_launch_without_tiles_keeps_the_order_of_kernels(ops, monkeypatch, summed):
     """A step of short requests whose lengths the host does not tell: the portions' kernel is launched first and finds no
