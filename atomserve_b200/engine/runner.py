@@ -341,6 +341,8 @@ class ModelRunner:
             state_slots=dv["state_slots"], logits_rows=dv["logits_rows"], max_context=max_context,
             host_q_lens=[len(r.tokens) for r in rows] + [1] * pad, host_pos_start=[r.start for r in rows] + [0] * pad,
             host_state_slots=[r.cache.state_slot for r in rows] + [pad_slot] * pad,
+            # (a request with two rows meets keys that this step stores)
+            earlier_keys_stored=len({r.cache.uid for r in rows}) == real,
         )  # fmt: skip
         groups = [(dv[f"slots{g}"], dv[f"tables{g}"].view(R, w)) for g, w in enumerate(widths)]
         return ctx, groups, (T, R, tuple(widths), B)
@@ -373,7 +375,7 @@ class ModelRunner:
 
     def _step_graph(self, rows: list[Row], device_tokens: torch.Tensor | None = None) -> torch.Tensor:
         """Decode-only step through a captured graph. The graph is keyed by everything that
-        fixes kernel shapes and buffer offsets: requests (rounded up to a bucket and padded with
+        fixes kernel arguments, shapes and buffer offsets: requests (rounded up to a bucket and padded with
         dummy requests when every row wants its logits, as in generation), table width (rounded
         up to a power of two), wanted rows, and the bucket of the longest context (which sets
         the key partitions). At most GraphCache.limit graphs are kept, and they share one pool of
@@ -388,7 +390,7 @@ class ModelRunner:
         if device_tokens is not None:  # behind the upload, before anything reads the ids
             ctx.token_ids[: len(rows)].copy_(device_tokens)
         ctx.max_context = context_bucket(ctx.max_context)
-        key = (*key, ctx.max_context)
+        key = (*key, ctx.max_context, ctx.earlier_keys_stored)
         self._bind(groups)
         out_rows = key[3]
         if self._graph_logits is None or self._graph_logits.shape[0] < out_rows:

@@ -141,6 +141,9 @@ class StepContext:
     host_q_lens: list[int] = field(default_factory=list)
     host_pos_start: list[int] = field(default_factory=list)
     host_state_slots: list[int] = field(default_factory=list)
+    # the index arrays, and all that the cache holds below each request's first new position, were written before the step's
+    # first kernel (so no request has two rows in the step): kernels may read them early
+    earlier_keys_stored: bool = False
     # what a part works out once per step for all layers of its kind (a cut of the step's requests
     # into segments, say), under a name of the part's choosing
     plans: dict[str, Any] = field(default_factory=dict)

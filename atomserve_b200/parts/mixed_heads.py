@@ -104,7 +104,7 @@ class MixedHeadsAttention(Mixer):
         out = ops.paged_attention(
             q, cache.k, cache.v, cache.block_tables, ctx.req_q_start, ctx.req_pos_start,
             num_requests=ctx.num_requests, max_context=ctx.max_context, window=self.window, scale=self.scale,
-            host_q_lens=ctx.host_q_lens or None, keep_first=self.keep_first,
+            host_q_lens=ctx.host_q_lens or None, keep_first=self.keep_first, earlier_keys_stored=ctx.earlier_keys_stored,
         )  # fmt: skip
         return out.view(-1, H * self.head_dim)
 

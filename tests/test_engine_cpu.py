@@ -41,6 +41,21 @@ def engine_for(model, bs, **kw):
     return Engine(ModelRunner(model, cache), Scheduler(config, cache), toy_parts.ArgmaxSampler())
 
 
+def test_a_request_with_two_rows_has_keys_that_the_step_stores(setup):
+    """Kernels may read the keys below a request's first new position early only where no request has two rows in the
+    step: the second row's earlier keys are the first's."""
+    cfg, bs, w, model = setup
+    cache = CacheManager(model.cache_requirements(), bs, 32, 4, torch.float32, "cpu")
+    runner = ModelRunner(model, cache)
+    ra, rb = cache.new_request(), cache.new_request()
+    for rc in (ra, rb):
+        cache.admit(rc), cache.reserve(rc, 0, 8)
+    assert runner.prepare([Row([1], 4, ra, [0]), Row([2], 6, rb, [0])])[0].earlier_keys_stored
+    assert runner.prepare([Row([1, 2, 3], 4, ra, [0]), Row([2], 6, rb, [0])], pad_requests=4)[0].earlier_keys_stored
+    assert not runner.prepare([Row([1], 4, ra, [0]), Row([2], 6, rb, [0]), Row([3], 5, ra, [0])])[0].earlier_keys_stored
+    assert not runner.prepare([Row([1, 2], 4, ra, [0]), Row([3], 6, ra, [0])])[0].earlier_keys_stored
+
+
 def test_step_function_matches_the_oracle_in_a_mixed_batch(setup):
     cfg, bs, w, model = setup
     cache = CacheManager(model.cache_requirements(), bs, 32, 4, torch.float32, "cpu")

@@ -49,6 +49,24 @@ def test_each_request_alone_and_whole(models, name, dtype):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("graphs", [True, False])
+def test_a_request_that_comes_twice_in_a_step(models, dtype, graphs):
+    """A trace may name a request in several entries of one step: each sees the keys that the entries before it bring."""
+    cfg, bs, folder, ps, oracle = models["d"]
+    for i in (1, 3):  # prompts of 200 and 330 tokens
+        rp = replayer(folder, dtype, bs, 4 * 384, graphs=graphs)
+        got, at = [], 0
+        for sizes in ([64, 64, 1, 8, 1], [1, 1], [1, 1, 1], [1, 3, 1, 1, 2]):
+            entries = []
+            for n in sizes:
+                entries.append(dict(id="x", tokens=ps[i][at : at + n], want=list(range(n))))
+                at += n
+            got.append(rp.step(entries, end=[]).clone())
+        got.append(rp.step([dict(id="x", tokens=ps[i][at:], want=list(range(len(ps[i]) - at)))], end=["x"]))
+        check(torch.cat(got), oracle[i], dtype, f"prompt of {len(ps[i])} in entries of one step")
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("name", ["a", "b", "c", "d", "e"])
 def test_prefill_then_last_32_one_by_one(models, name, dtype):
     cfg, bs, folder, ps, oracle = models[name]
