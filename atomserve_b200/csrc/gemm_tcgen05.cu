@@ -741,6 +741,17 @@ Plan make_plan(int M, int N, int K) {
     pl.workspace = (long long)tiles * pl.max_slots * BM * pl.bn;
   }
   if (g_force_swap == 3) pl.wide = g_force_bn;
+  if (pl.wide) {  // nothing of the form it displaced is told or run
+    const int weight_tiles = (N + 255) / 256, token_tiles = (M + pl.wide - 1) / pl.wide, pairs = sms / 2;
+    int cut[3];
+    pl.swap = 1;
+    pl.pair = pl.stream = pl.max_slots = 0;
+    pl.bn = pl.wide;
+    pl.tiles_p = weight_tiles;
+    pl.tiles_q = token_tiles;
+    pl.workspace = asb_gemm_tcgen05_pair_swapped_cut(M, N, K, pl.wide, cut);
+    pl.blocks = 2 * (weight_tiles * token_tiles < pairs ? weight_tiles * token_tiles * cut[1] : pairs);
+  }
   return pl;
 }
 
@@ -776,9 +787,9 @@ extern "C" long long asb_gemm_tcgen05_workspace(int M, int N, int K, int* stream
   return pl.workspace;
 }
 
-// The form of a call that takes the place of what asb_gemm_tcgen05_plan tells: pairs of SMs on tiles of 256 weight rows by
-// out4[0] tokens (0: not used), of which out4[1] run whole, and each of the others in out4[2] pieces of out4[3] stages (two K blocks).
-// Returns its workspace's float32 elements.
+// Whether a call runs on pairs of SMs with swapped operands: tiles of 256 weight rows by out4[0] tokens (0: not that form),
+// of which out4[1] run whole, and each of the others in out4[2] pieces of out4[3] stages (two K blocks).
+// Returns its workspace's float32 elements, which asb_gemm_tcgen05_workspace tells too.
 extern "C" long long asb_gemm_tcgen05_wide_plan(int M, int N, int K, int* out4) {
   out4[0] = out4[1] = out4[2] = out4[3] = 0;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
@@ -801,7 +812,8 @@ extern "C" void asb_gemm_tcgen05_tune(int swap, int bn) { g_force_swap = swap; g
 // tile, token columns (swapped) or weight rows (unswapped) per tile, K blocks per tile, tiles,
 // thread blocks, weight rows of the tiles of pairs of SMs (0: single SMs)}. With pairs, a tile is
 // 256 tokens by that many weight rows and two thread blocks share it; how the last round of
-// tiles is cut along K, asb_gemm_tcgen05_pair_cut tells. A shape that cuts K with
+// tiles is cut along K, asb_gemm_tcgen05_pair_cut tells. Swapped operands on pairs of SMs (whole tiles of
+// 256 weight rows) are told apart by asb_gemm_tcgen05_wide_plan. A shape that cuts K with
 // swapped operands can leave its product as partial sums (mode 3 of asb_gemm_tcgen05), which
 // csrc/gemm_partials.cuh describes.
 extern "C" int asb_gemm_tcgen05_plan(int M, int N, int K, int* out8) {
@@ -845,9 +857,9 @@ static int gemm_tcgen05_run(void* out, const void* x, const void* w, const void*
   const Plan pl = make_plan(M, N, K);
   if (mode == 3 && !(pl.stream && pl.swap && pl.tiles_q == 1))
     return asb::fail("gemm_tcgen05: [%d, %d] x [%d, %d] does not run with partial sums", M, K, N, K);
-  if (pl.wide && mode != 3)
+  if (pl.wide)
     return asb_gemm_tcgen05_pair_swapped(out, x, w, residual, M, N, K, mode, pl.wide, workspace, status, glu_bias, glu_act, stream);
-  if (pl.pair && mode != 3)
+  if (pl.pair)
     return asb_gemm_tcgen05_pair(out, x, w, residual, M, N, K, mode, pl.pair, workspace, status, glu_bias, glu_act, stream);
   if (pl.workspace > 0 && !workspace) return asb::fail("gemm_tcgen05: this shape needs a workspace of %lld floats", pl.workspace);
 

@@ -80,13 +80,9 @@ _WORKSPACE_FLOATS: dict[tuple[int, int, int], int] = {}
 def _workspace_floats(M: int, N: int, K: int) -> int:
     need = _WORKSPACE_FLOATS.get((M, N, K))
     if need is None:
-        query, wide = lib().asb_gemm_tcgen05_workspace, lib().asb_gemm_tcgen05_wide_plan
-        query.restype = wide.restype = ctypes.c_longlong
-        out = (ctypes.c_int * 4)()
-        need = wide(M, N, K, out)
-        if not out[0]:
-            need = query(M, N, K, None)
-        _WORKSPACE_FLOATS[(M, N, K)] = need
+        query = lib().asb_gemm_tcgen05_workspace
+        query.restype = ctypes.c_longlong
+        need = _WORKSPACE_FLOATS[(M, N, K)] = query(M, N, K, None)
     return need
 
 
@@ -138,11 +134,6 @@ def _plan(M: int, N: int, K: int) -> tuple[int, ...]:
     if plan is None:
         out = (ctypes.c_int * 8)()
         check(lib().asb_gemm_tcgen05_plan(M, N, K, out))
-        wide = (ctypes.c_int * 4)()
-        lib().asb_gemm_tcgen05_wide_plan.restype = ctypes.c_longlong
-        lib().asb_gemm_tcgen05_wide_plan(M, N, K, wide)
-        if wide[0]:
-            out[0] = 0  # that form takes the place of one that cuts K into partial sums
         plan = _PLANS[(M, N, K)] = tuple(out)
     return plan
 

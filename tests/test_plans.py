@@ -42,7 +42,8 @@ def test_decode_attention_partition_plans_cover_every_context(monkeypatch):
 def test_gemm_plans_keep_every_tile_within_its_partial_sum_slots():
     """The tensor-core GEMM's schedule is host arithmetic inside the library (it needs no GPU):
     whatever the shape, the tiles cover the product, only swapped operands cut K, every block has
-    at least one K block, and no tile is shared by more blocks than it has workspace slots."""
+    at least one K block, and no tile is shared by more blocks than it has workspace slots. What the plan and the
+    workspace's size are told for is the form that runs."""
     import ctypes
     import random
 
@@ -57,8 +58,11 @@ def test_gemm_plans_keep_every_tile_within_its_partial_sum_slots():
     pair_cut, workspace = lib().asb_gemm_tcgen05_pair_cut, lib().asb_gemm_tcgen05_workspace
     pair_cut.argtypes, pair_cut.restype = [ctypes.c_int] * 4 + [ctypes.POINTER(ctypes.c_int)], ctypes.c_longlong
     workspace.argtypes, workspace.restype = [ctypes.c_int] * 3 + [ctypes.POINTER(ctypes.c_int)], ctypes.c_longlong
-    out, cut = (ctypes.c_int * 8)(), (ctypes.c_int * 3)()
-    cut_plans = 0
+    wide_plan, wide_cut = lib().asb_gemm_tcgen05_wide_plan, lib().asb_gemm_tcgen05_pair_swapped_cut
+    wide_plan.argtypes, wide_plan.restype = [ctypes.c_int] * 3 + [ctypes.POINTER(ctypes.c_int)], ctypes.c_longlong
+    wide_cut.argtypes, wide_cut.restype = [ctypes.c_int] * 4 + [ctypes.POINTER(ctypes.c_int)], ctypes.c_longlong
+    out, cut, wide = (ctypes.c_int * 8)(), (ctypes.c_int * 3)(), (ctypes.c_int * 4)()
+    cut_plans = wide_plans = wide_cut_plans = 0
     rng = random.Random(1)
     shapes = [(8, 4096, 4096), (1, 151936, 4096), (512, 4096, 12288), (2048, 24576, 4096), (300, 5120, 17408)]
     for _ in range(3000):
@@ -69,6 +73,25 @@ def test_gemm_plans_keep_every_tile_within_its_partial_sum_slots():
         plan(M, N, K, out)
         cuts_k, swap, max_slots, bn, kb, tiles, blocks, pair = list(out)
         assert kb == -(-K // 64) and 1 <= blocks <= 148, (M, N, K)
+        floats = wide_plan(M, N, K, wide)
+        if wide[0]:  # tiles of 256 weight rows by wide[0] tokens, a pair of SMs on each; the plan and the workspace are this form's
+            wide_plans += 1
+            tokens, whole, split, piece = list(wide)
+            stages = -(-kb // 2)
+            assert tokens % 32 == 0 and 32 <= tokens <= 256 and bn == tokens and swap and not cuts_k and not pair and not max_slots, (M, N, K)
+            assert tiles == -(-N // 256) * -(-M // tokens), (M, N, K)
+            assert workspace(M, N, K, None) == floats == wide_cut(M, N, K, tokens, cut) and list(cut) == [whole, split, piece], (M, N, K)
+            if split == 1:
+                assert whole == tiles and floats == 0 and blocks == 2 * min(tiles, 74), (M, N, K)
+            else:  # the last round cut along K, a slot a piece, as wide as the kernel's widest tile
+                wide_cut_plans += 1
+                slot = 256 * next(s for s in (64, 128, 192, 256) if s >= tokens)
+                assert floats == (tiles - whole) * split * slot, (M, N, K)
+                assert whole % 74 == 0 and 0 < tiles - whole and (tiles - whole) * split <= 74, (M, N, K)
+                assert (split - 1) * piece < stages <= split * piece, (M, N, K)
+                assert blocks == 2 * (74 if whole else tiles * split), (M, N, K)
+            continue
+        assert floats == 0
         if pair:  # tiles of 256 tokens by `pair` weight rows, two blocks (a pair of SMs) on each
             assert pair in (128, 160, 192, 224, 256) and bn == pair and not swap and not cuts_k and M > 128, (M, N, K)
             assert tiles == -(-M // 256) * -(-N // pair), (M, N, K)
@@ -105,7 +128,7 @@ def test_gemm_plans_keep_every_tile_within_its_partial_sum_slots():
             first = bisect.bisect_right(begins, tile * kb) - 1
             last = bisect.bisect_right(begins, tile * kb + kb - 1) - 1
             assert last - first + 1 <= max_slots, (M, N, K, tile)
-    assert cut_plans > 20
+    assert cut_plans > 20 and wide_plans > 50 and wide_cut_plans > 20
 
 
 def test_decode_graph_keys_are_few_and_the_cache_of_graphs_is_bounded():
