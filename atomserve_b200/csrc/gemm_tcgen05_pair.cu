@@ -325,6 +325,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
           const int tokens = min(32, p.M - (n0 + c));
           if (tokens <= 0) break;  // uniform
           uint32_t raw[32];
+          __syncwarp();  // the read takes the whole warp, and lanes beyond N come from the store's branch early
           tmem_ld32(tmem_base + ((uint32_t)(quad * 32) << 16) + buf * BN + (uint32_t)c, raw);
           if (piece) {
 #pragma unroll
@@ -398,6 +399,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       for (int c = 0; c < p.bn; c += 32) {
         if (n0 + c >= p.N) break;  // uniform
         uint32_t raw[32];
+        __syncwarp();  // the read takes the whole warp, and lanes beyond M come from the store's branch early
         tmem_ld32(tmem_base + ((uint32_t)(quad * 32) << 16) + buf * BN + (uint32_t)c, raw);
         if (row >= p.M) continue;
         const int valid = min(32, p.N - (n0 + c));
