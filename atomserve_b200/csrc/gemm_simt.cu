@@ -245,7 +245,7 @@ __device__ __forceinline__ void copy16(float* to, const float* from, bool valid)
 template <int MR, int CLUSTER>
 __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(kThreads)
 rows_kernel(float* __restrict__ out, const float* __restrict__ x, const float* __restrict__ w,
-            const float* __restrict__ residual, int M, int N, int K) {
+            const float* __restrict__ residual, int M, int N, int K, int w_stored) {
   extern __shared__ __align__(16) float smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int rank = (int)(blockIdx.x % CLUSTER);
@@ -272,7 +272,8 @@ rows_kernel(float* __restrict__ out, const float* __restrict__ x, const float* _
   };
   auto fetch_w = [&](int step) { if (step < steps) fetch_rows(step, 0, kRowsN, w, n0, N); };
   auto fetch_x = [&](int step) { if (step < steps) fetch_rows(step, kRowsN, kRowsN + MR, x, 0, M); };
-  // weights, which no kernel writes, come before the wait for the stream's previous kernel
+  // a model's weights, which no kernel of a step writes, come before the wait for the stream's previous kernel
+  if (!w_stored) asb::pdl_wait();
 #pragma unroll
   for (int s = 0; s < kRowStages - 1; ++s) fetch_w(s);
   asb::pdl_wait();
@@ -388,28 +389,29 @@ size_t rows_smem(int mr, int blocks, int runs) {
 }
 
 template <int MR, int CLUSTER>
-int launch_rows(float* out, const float* x, const float* w, const float* residual, int M, int N, int K, cudaStream_t stream) {
+int launch_rows(float* out, const float* x, const float* w, const float* residual, int M, int N, int K, int w_stored, cudaStream_t stream) {
   const size_t smem = rows_smem(MR, CLUSTER, (K + kRun - 1) / kRun);
   auto kernel = rows_kernel<MR, CLUSTER>;
   if (int rc = allow_smem(kernel, smem)) return rc;
-  asb::launch(kernel, dim3(CLUSTER * (unsigned)((N + kRowsN - 1) / kRowsN)), kThreads, smem, stream, out, x, w, residual, M, N, K);
+  asb::launch(kernel, dim3(CLUSTER * (unsigned)((N + kRowsN - 1) / kRowsN)), kThreads, smem, stream, out, x, w, residual, M, N, K, w_stored);
   return 0;
 }
 
 template <int MR>
-int rows(float* out, const float* x, const float* w, const float* residual, int M, int N, int K, cudaStream_t stream) {
+int rows(float* out, const float* x, const float* w, const float* residual, int M, int N, int K, int w_stored, cudaStream_t stream) {
   // eight blocks a cluster where four would have more than eight runs each to keep the sums of
-  if (K > 32 * kRun) return launch_rows<MR, 8>(out, x, w, residual, M, N, K, stream);
-  if (K > (kQuarters - 1) * kRun) return launch_rows<MR, kQuarters>(out, x, w, residual, M, N, K, stream);
-  return launch_rows<MR, 1>(out, x, w, residual, M, N, K, stream);
+  if (K > 32 * kRun) return launch_rows<MR, 8>(out, x, w, residual, M, N, K, w_stored, stream);
+  if (K > (kQuarters - 1) * kRun) return launch_rows<MR, kQuarters>(out, x, w, residual, M, N, K, w_stored, stream);
+  return launch_rows<MR, 1>(out, x, w, residual, M, N, K, w_stored, stream);
 }
 
 }  // namespace
 
 // in_dtype: element type of x and w. out_dtype: element type of out and residual (float32 out
-// from bfloat16 inputs gives logits straight from the accumulator).
+// from bfloat16 inputs gives logits straight from the accumulator). w_stored: w was written before the stream's
+// previous kernel was launched, and may be read while that kernel runs.
 extern "C" int asb_gemm_simt(void* out, const void* x, const void* w, const void* residual,
-                             int M, int N, int K, int in_dtype, int out_dtype,
+                             int M, int N, int K, int in_dtype, int out_dtype, int w_stored,
                              cudaStream_t stream) {
   if (M == 0 || N == 0) return 0;
   if (K < 1) return asb::fail("gemm_simt: K = %d", K);
@@ -423,9 +425,9 @@ extern "C" int asb_gemm_simt(void* out, const void* x, const void* w, const void
     const float* rf = (const float*)residual;
     if (M > 16 || !aligned || rows_smem(mr, 8, (K + kRun - 1) / kRun) > kMostSmem)
       rc = tiles<float, float>(out, x, w, residual, M, N, K, stream);
-    else if (mr == 4) rc = rows<4>((float*)out, xf, wf, rf, M, N, K, stream);
-    else if (mr == 8) rc = rows<8>((float*)out, xf, wf, rf, M, N, K, stream);
-    else rc = rows<16>((float*)out, xf, wf, rf, M, N, K, stream);
+    else if (mr == 4) rc = rows<4>((float*)out, xf, wf, rf, M, N, K, w_stored, stream);
+    else if (mr == 8) rc = rows<8>((float*)out, xf, wf, rf, M, N, K, w_stored, stream);
+    else rc = rows<16>((float*)out, xf, wf, rf, M, N, K, w_stored, stream);
   } else if (in_dtype == asb::kBFloat16 && out_dtype == asb::kBFloat16) {
     rc = tiles<__nv_bfloat16, __nv_bfloat16>(out, x, w, residual, M, N, K, stream);
   } else if (in_dtype == asb::kBFloat16 && out_dtype == asb::kFloat32) {

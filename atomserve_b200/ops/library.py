@@ -44,7 +44,7 @@ _SIGNATURES = {
     "asb_gemm_tcgen05_plan": [_I, _I, _I, _P],
     "asb_partial_add_rmsnorm": [_P, _P, _P, _I, _I, _I, _I, _I, _P, _P, _I, _I, _F, _P],
     "asb_qk_norm_rope_store_partial": [_P] * 4 + [_I] * 5 + [_P] * 5 + [_I] * 6 + [_F, _P],
-    "asb_gemm_simt": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
+    "asb_gemm_simt": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P],
     "asb_argmax_rows": [_P, _P, _I, _I, _P],
     "asb_presence_penalty": [_P, _P, _P, _P, _I, _I, _P],
     "asb_sample_rows": [_P, _P, _I, _I, _P, _P, _P, _P, _P, _P],

@@ -22,13 +22,13 @@ from atomserve_b200.ops.status import status_for
 
 
 def gemm_simt(x: torch.Tensor, w: torch.Tensor, residual: torch.Tensor | None, out_dtype: torch.dtype,
-              out: torch.Tensor | None = None) -> torch.Tensor:  # fmt: skip
+              out: torch.Tensor | None = None, weights_stored: bool = False) -> torch.Tensor:  # fmt: skip
     M, K = x.shape
     N = w.shape[0]
     if out is None:
         out = torch.empty(M, N, device=x.device, dtype=out_dtype)
     check(lib().asb_gemm_simt(ptr(out), ptr(x), ptr(w), ptr(residual), M, N, K, dtype_code(x),
-                              dtype_code(out), stream()))  # fmt: skip
+                              dtype_code(out), int(weights_stored), stream()))  # fmt: skip
     return out
 
 
@@ -257,8 +257,13 @@ def linear(
     residual: torch.Tensor | None = None,
     out_dtype: torch.dtype | None = None,
     out: torch.Tensor | None = None,
+    weights_stored: bool = False,
 ) -> torch.Tensor:
-    """`out`, if given, is the contiguous [M, N] tensor of the output dtype that takes the result."""
+    """`out`, if given, is the contiguous [M, N] tensor of the output dtype that takes the result.
+
+    `weights_stored`: w was written before the stream's previous kernel was launched, as a model's weights are. A float32
+    product with few rows may then read it while that kernel runs.
+    The bfloat16 tensor-core kernels always do: their w must not be what the library's kernel right before writes."""
     require_cuda(x, w, residual, out)
     if x.dim() != 2 or w.dim() != 2 or x.shape[1] != w.shape[1]:
         raise KernelLibraryError(f"linear: x {tuple(x.shape)} does not match w {tuple(w.shape)}")
@@ -272,7 +277,7 @@ def linear(
     if x.dtype == torch.float32:
         if out_dtype != torch.float32:
             raise KernelLibraryError("linear: float32 operands give float32 results")
-        return gemm_simt(x, w, residual, torch.float32, out)
+        return gemm_simt(x, w, residual, torch.float32, out, weights_stored)
     if out_dtype == torch.float32 and residual is not None:
         return gemm_simt(x, w, residual, torch.float32, out)
     if BACKEND == "tcgen05" and tcgen05_supported(x, w):

@@ -144,7 +144,7 @@ class GQAttention(Mixer):
                 cache: CacheView | None, write_cache: bool = True) -> torch.Tensor:  # fmt: skip
         # (no residual: a block that sums in float32 itself, and the product stays float32)
         return ops.linear(self.attend(h, ctx, cache, write_cache), self.o_proj, residual,
-                          out_dtype=torch.float32 if residual is None else None)  # fmt: skip
+                          out_dtype=torch.float32 if residual is None else None, weights_stored=True)  # fmt: skip
 
     def forward_then(self, h: torch.Tensor, residual: torch.Tensor, ctx: StepContext, cache: CacheView | None,
                      write_cache: bool, then: Norm) -> tuple[torch.Tensor, torch.Tensor]:  # fmt: skip
@@ -166,7 +166,7 @@ class GQAttention(Mixer):
         return self.qkv_proj
 
     def forward_from(self, proj: torch.Tensor, col: int, ctx: StepContext, cache: CacheView, write_cache: bool = True) -> torch.Tensor:
-        return ops.linear(self.attend_from(proj, col, ctx, cache, write_cache), self.o_proj, out_dtype=torch.float32)
+        return ops.linear(self.attend_from(proj, col, ctx, cache, write_cache), self.o_proj, out_dtype=torch.float32, weights_stored=True)
 
     def attend_from(self, proj: torch.Tensor, col: int, ctx: StepContext, cache: CacheView, write_cache: bool) -> torch.Tensor:
         """`attend` for queries and keys normed over the whole projection, from a product that holds this
@@ -186,7 +186,7 @@ class GQAttention(Mixer):
         H, KV, hd = self.num_heads, self.num_kv_heads, self.head_dim
         if self.norm_over == "projection":
             weight = self.qkv_proj if write_cache else self.qkv_proj[: H * self.key_dim]
-            return self.attend_from(ops.linear(h, weight), 0, ctx, cache, write_cache)
+            return self.attend_from(ops.linear(h, weight, weights_stored=True), 0, ctx, cache, write_cache)
         # the position encoding says how it is applied: by the fused kernel below (a rotation by
         # position x frequency), or by its own `encode` on the normalised queries and keys
         rotary = self.position.fused_rotary() if self.position is not None else None
@@ -197,7 +197,7 @@ class GQAttention(Mixer):
         elif self.query_temperature is not None:
             # unnormed queries scaled by position: the kernel for heads of several maps, with one map
             # (the padded rows of the stacked weight give the zeros of the wider head size)
-            qkv = ops.linear(h, self.qkv_proj if write_cache else self.qkv_proj[: H * hd])
+            qkv = ops.linear(h, self.qkv_proj if write_cache else self.qkv_proj[: H * hd], weights_stored=True)
             q = ops.qk_prepare_store(
                 qkv, H, KV, 1, hd, hd, hd, ctx.positions,
                 inv_freq=rotary.inv_freq if rotary else None, rotary_dim=rotary.rotary_dim if rotary else 0,
@@ -212,7 +212,7 @@ class GQAttention(Mixer):
                 # with few tokens the product stays as the GEMM's partial sums and the next kernel adds them up
                 qkv = ops.linear_partial(h, weight)
             if qkv is None:
-                qkv = ops.linear(h, weight)
+                qkv = ops.linear(h, weight, weights_stored=True)
             q = ops.qk_norm_rope_store(
                 qkv, H, kv_heads, hd, ctx.positions,
                 q_gain=self.q_gain, k_gain=self.k_gain, eps=self.kernel_eps or 0.0,
@@ -238,7 +238,7 @@ class GQAttention(Mixer):
         H, KV, hd = self.num_heads, self.num_kv_heads, self.head_dim
         T = h.shape[0]
         kv_heads = KV if write_cache else 0
-        qkv = ops.linear(h, self.qkv_proj if write_cache else self.qkv_proj[: H * hd])
+        qkv = ops.linear(h, self.qkv_proj if write_cache else self.qkv_proj[: H * hd], weights_stored=True)
         normed = qkv
         if self.qk_norm_eps is not None:
             heads = qkv.view(T, H + 2 * kv_heads, hd)

@@ -135,7 +135,7 @@ class LMHead(Part):
         self.weight = embedding.table
 
     def forward(self, hidden: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
-        logits = ops.linear(hidden, self.weight, out_dtype=torch.float32, out=out)
+        logits = ops.linear(hidden, self.weight, out_dtype=torch.float32, out=out, weights_stored=True)
         return ops.softcap_(logits, self.softcap) if self.softcap else logits
 
 

@@ -39,10 +39,10 @@ class SwiGLU(FeedForward):
     def hidden(self, h: torch.Tensor) -> torch.Tensor:
         if self.fused:
             return ops.linear_swiglu(h, self.gate_up_proj)
-        return ops.silu_mul(ops.linear(h, self.gate_up_proj))
+        return ops.silu_mul(ops.linear(h, self.gate_up_proj, weights_stored=True))
 
     def forward(self, h: torch.Tensor, residual: torch.Tensor, ctx: StepContext) -> torch.Tensor:
-        return ops.linear(self.hidden(h), self.down_proj, residual)
+        return ops.linear(self.hidden(h), self.down_proj, residual, weights_stored=True)
 
     def forward_then(self, h: torch.Tensor, residual: torch.Tensor, ctx: StepContext,
                      then: Norm) -> tuple[torch.Tensor, torch.Tensor]:  # fmt: skip
@@ -97,10 +97,10 @@ class GatedMLP(FeedForward):
     def inner(self, h: torch.Tensor) -> torch.Tensor:
         if self.fused:
             return ops.linear_glu(h, self.gate_up, self.gate_up_bias, self.activation)
-        return ops.bias_glu(ops.linear(h, self.gate_up), self.gate_up_bias, self.activation)
+        return ops.bias_glu(ops.linear(h, self.gate_up, weights_stored=True), self.gate_up_bias, self.activation)
 
     def forward(self, h: torch.Tensor, residual: torch.Tensor | None, ctx: StepContext) -> torch.Tensor:
-        out = ops.linear(self.inner(h), self.down, None, out_dtype=torch.float32)
+        out = ops.linear(self.inner(h), self.down, None, out_dtype=torch.float32, weights_stored=True)
         if self.output_bias is not None:
             out += self.output_bias
         return out if residual is None else residual + out.to(residual.dtype)

@@ -39,7 +39,7 @@ class RMSNorm(Norm):
             product = ops.linear_partial(x, weight)
             if product is not None:
                 return ops.partial_add_rms_norm(product, residual, self.gain, self.eps)
-        total = ops.linear(x, weight, residual)
+        total = ops.linear(x, weight, residual, weights_stored=True)
         return total, self.forward(total)
 
 

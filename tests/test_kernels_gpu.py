@@ -109,6 +109,19 @@ def test_float32_linear_in_both_kernels(ops, N, K):
         assert torch.equal(ops.linear(off[:M], w), whole[:M])
 
 
+@pytest.mark.parametrize("M", [1, 4, 7, 16, 17])
+def test_float32_linear_waits_for_the_matrix_that_the_previous_kernel_writes(ops, M):
+    """A matrix that comes from the library kernel right before (which lets its successor start early) is read when that
+    kernel has completed, with as few rows as well."""
+    g = torch.Generator().manual_seed(M)
+    x, b = torch.randn(M, 2048, generator=g).cuda(), torch.randn(2048, 1024, generator=g).cuda()
+    for i in range(6):
+        a = torch.randn(512, 1024, generator=g).cuda()
+        ref = ops.linear(x, ops.linear(a, b).clone())
+        torch.cuda.synchronize()
+        assert torch.equal(ops.linear(x, ops.linear(a, b)), ref), i
+
+
 def rope_reference(x, positions, hd, theta, rotary_dim=None):
     rd = rotary_dim or hd
     angles = plain.rope_angles(positions, rd, theta)
