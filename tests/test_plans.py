@@ -39,6 +39,25 @@ def test_decode_attention_partition_plans_cover_every_context(monkeypatch):
     attention.plan_decode_partitions.cache_clear()
 
 
+def test_portions_are_planned_for_their_own_contexts():
+    """A short prompt beside one long decode is not divided for the decode's context; without the positions the step's
+    longest context stands in, and one part is the answer where the lengths are not told at all."""
+    from atomserve_b200.ops.attention import plan_portion_parts, portions_context
+
+    assert portions_context([40, 1], [0, 12000], 12001) == 40
+    assert portions_context([40, 1, 200], [5000, 12000, 100], 12001) == 5040
+    assert portions_context([40, 1], None, 12001) == portions_context(None, None, 12001) == 12001
+    assert plan_portion_parts([40, 1], 8, 4, portions_context([40, 1], [0, 12000], 12001), 0) == 1
+    assert plan_portion_parts(None, 8, 4, 12001, 0) == 1
+    for lens in ([512], [100], [9], [300, 200, 64], [2048]):
+        for kv, group in ((8, 4), (8, 5), (1, 16), (2, 1)):
+            for context in (64, 449, 512, 7000, 40000):
+                for window in (0, 100, 4096):
+                    parts = plan_portion_parts(lens, kv, group, max(context, max(lens)), window)
+                    tiles = -(-(min(max(context, max(lens)), window + 128 // group) if window else max(context, max(lens))) // 64)
+                    assert parts in (1, 2, 4) and (parts == 1 or tiles >= 8)
+
+
 def test_gemm_plans_keep_every_tile_within_its_partial_sum_slots():
     """The tensor-core GEMM's schedule is host arithmetic inside the library (it needs no GPU):
     whatever the shape, the tiles cover the product, only swapped operands cut K, every block has
