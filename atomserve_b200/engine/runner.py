@@ -390,7 +390,7 @@ class ModelRunner:
         if device_tokens is not None:  # behind the upload, before anything reads the ids
             ctx.token_ids[: len(rows)].copy_(device_tokens)
         ctx.max_context = context_bucket(ctx.max_context)
-        key = (*key, ctx.max_context, ctx.earlier_keys_stored)
+        key = (*key, ctx.earlier_keys_stored, ctx.max_context)
         self._bind(groups)
         out_rows = key[3]
         if self._graph_logits is None or self._graph_logits.shape[0] < out_rows:
