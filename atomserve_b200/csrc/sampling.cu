@@ -1,4 +1,4 @@
-// Sampling on the device: a cluster of eight blocks per row of float32 logits [B, V].
+// Sampling on the device: a cluster of up to eight blocks per row of float32 logits [B, V].
 //
 // The rules are the reference sampler's (atomserve/sampler.py:82-129): top-k on the raw
 // logits (0 or >= V keeps all; temperature 0 is the single best), divide by the temperature,
@@ -16,7 +16,7 @@
 // candidates they are gathered into one block's shared memory and ranked there.
 //
 // What bounds it: a row of 151,936 logits is 600 KB, and with one block a row every one of
-// seven passes over it moved at the rate of one SM. Here each block of the cluster brings its eighth of the row
+// seven passes over it moved at the rate of one SM. Here each block of the cluster brings its share of the row
 // into shared memory once (76 KB, two blocks an SM) and all passes read it there; what is left is the
 // chain of passes with two cluster barriers each. Measured, 1 / 48 rows of 151,936: temperature 0.6, top-k 20, top-p
 // 0.95 122 / 124 -> 17 / 40 us; top-p 0.95 alone 371 / 480 -> 35 / 87 us; argmax 8.8 / 8.8 -> 3.8 / 6.5 us. An eighth and not a quarter, because rows in flight on the
@@ -35,11 +35,11 @@ namespace {
 
 constexpr int kThreads = 512;
 constexpr int kWarps = kThreads / 32;
-constexpr int kCluster = 8;                      // blocks a row
+constexpr int kMostBlocks = 8;                   // blocks a row: 8, 4, 2 or 1 (the kernels' C)
 constexpr int kBins = 2048;                      // an 11-bit digit
-constexpr int kSegment = kBins / kCluster;       // bins whose totals one block forms
+constexpr int kSegment = 256;                    // bins that are searched together
+constexpr int kSegments = kBins / kSegment;      // a block of C forms the totals of kSegments / C of them
 constexpr int kCompact = 1024;
-constexpr int kMaxSlice = 48 * 1024;             // floats of a row that a block can hold in shared memory
 constexpr int kSplitSlice = 65535;               // most elements whose masses two 32-bit words can add up (see Scratch)
 
 __device__ __forceinline__ uint32_t order_key(float f) {
@@ -81,7 +81,9 @@ struct Best {
   }
 };
 
+template <int C>
 struct Scratch {
+  static constexpr int kOwn = kSegments / C;
   // A digit's histogram. Counts: word[0]. Masses, at most 2^32 each: the low 16 bits of each are added up in
   // word[0] and the rest in word[1] (both native 32-bit atomics; 64-bit ones in shared memory are loops), which
   // holds for up to kSplitSlice elements; otherwise, and where a mass may be out of that range (a row with an
@@ -89,19 +91,26 @@ struct Scratch {
   union {
     unsigned int word[2][kBins];
     unsigned long long wide[kBins];
+    struct {  // the candidates in order, once the selects are over in every block
+      uint32_t key[kCompact];
+      int id[kCompact];
+    } sorted;
   } hist;
-  unsigned long long total[kSegment];  // over the cluster, of this block's segment of the bins
-  unsigned long long segment_sum;
-  unsigned long long warp_part[kWarps];  // a sum being formed over the block
+  unsigned long long total[kOwn * kSegment];  // over the cluster, of this block's segments of the bins
+  unsigned long long segment_sum[kOwn];
+  unsigned long long warp_part[kOwn > 2 ? kOwn * kSegment / 32 : kWarps];  // a sum being formed over the block
   int odd;                               // this block's slice holds a NaN
   Best best[2], warp_best[kWarps];  // [0]: the largest logit, [1]: the winner of the race
   unsigned long long found[4];
   int cand_n;
   __align__(16) uint32_t cand_key[kCompact];
   __align__(16) int cand_id[kCompact];
-  uint32_t sorted_key[kCompact];
-  int sorted_id[kCompact];
 };
+
+constexpr int kMaxSmem = 227 * 1024;
+// Floats of a row that a block of C can hold in shared memory.
+template <int C>
+constexpr int kMaxSlice = (kMaxSmem - (int)sizeof(Scratch<C>)) / 16 * 4 < 48 * 1024 ? (kMaxSmem - (int)sizeof(Scratch<C>)) / 16 * 4 : 48 * 1024;
 
 __device__ __forceinline__ float key_value(uint32_t key) {
   return __uint_as_float((key & 0x80000000u) ? (key & 0x7fffffffu) : ~key);
@@ -128,9 +137,27 @@ __device__ __forceinline__ void for_each_value(const Slice& row, F f) {
   for (int i = done + threadIdx.x; i < row.n; i += kThreads) f(row.first + i, row.val[i]);
 }
 
+// `p` of block `c` of the cluster.
+template <int C, typename T>
+__device__ __forceinline__ T* peer(T* p, int c) {
+  if constexpr (C == 1) return p;
+  else return cg::this_cluster().map_shared_rank(p, c);
+}
+template <int C>
+__device__ __forceinline__ void row_sync() {
+  if constexpr (C == 1) __syncthreads();
+  else cg::this_cluster().sync();
+}
+template <int C>
+__device__ __forceinline__ int row_rank() {
+  if constexpr (C == 1) return 0;
+  else return (int)cg::this_cluster().block_rank();
+}
+
 // The best over the block, then over the cluster: every thread of every block gets it. `slot`: which of the
 // scratch's two (each is used once a kernel, so no barrier keeps a second use from a slow reader).
-__device__ Best cluster_best(const cg::cluster_group& cluster, Scratch& s, Best b, int slot) {
+template <int C>
+__device__ Best cluster_best(Scratch<C>& s, Best b, int slot) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     const float os = __shfl_xor_sync(0xffffffffu, b.score, o);
@@ -144,11 +171,11 @@ __device__ Best cluster_best(const cg::cluster_group& cluster, Scratch& s, Best 
     for (int w = 1; w < kWarps; ++w) b.take(s.warp_best[w].score, s.warp_best[w].token);
     s.best[slot] = b;
   }
-  cluster.sync();
+  row_sync<C>();
   b = s.best[slot];
 #pragma unroll
-  for (int c = 0; c < kCluster; ++c) {
-    const Best o = *cluster.map_shared_rank(&s.best[slot], c);
+  for (int c = 0; c < C; ++c) {
+    const Best o = *peer<C>(&s.best[slot], c);
     b.take(o.score, o.token);
   }
   return b;
@@ -167,13 +194,14 @@ __device__ Best cluster_best(const cg::cluster_group& cluster, Scratch& s, Best 
 // `above` and `equal` counting what lies above and inside it.
 //
 // kUnit: every weight is 1 (a count). `wide`: weights added up in 64-bit words (see Scratch).
-template <bool kUnit, typename Item, typename Weight, typename Target>
-__device__ uint32_t cluster_select(const cg::cluster_group& cluster, const Slice& row, Scratch& s, Target target_of,
+template <bool kUnit, int C, typename Item, typename Weight, typename Target>
+__device__ uint32_t cluster_select(const Slice& row, Scratch<C>& s, Target target_of,
                                    unsigned long long* above, unsigned long long* equal, bool wide, int digits, Item item,
                                    Weight weight) {
   uint32_t prefix = 0, mask = 0;
   unsigned long long acc = 0, target = 0;
-  const int rank = (int)cluster.block_rank(), lane = threadIdx.x & 31;
+  constexpr int kOwn = Scratch<C>::kOwn;
+  const int rank = row_rank<C>(), lane = threadIdx.x & 31;
   for (int digit = 0; digit < digits; ++digit) {
     const int shift = digit == 0 ? 21 : (digit == 1 ? 10 : 0);
     const uint32_t bins = digit == 2 ? 1024u : 2048u;
@@ -196,45 +224,45 @@ __device__ uint32_t cluster_select(const cg::cluster_group& cluster, const Slice
         if (hi) atomicAdd(&s.hist.word[1][bin], hi);
       }
     });
-    cluster.sync();
-    // this block's segment of the bins, over the cluster
-    if (threadIdx.x < kSegment) {
-      const int bin = rank * kSegment + threadIdx.x;
+    row_sync<C>();
+    // this block's segments of the bins, over the cluster (a warp's 32 bins lie in one of them)
+    for (int i = threadIdx.x; i < kOwn * kSegment; i += kThreads) {
+      const int bin = rank * kOwn * kSegment + i;
       unsigned long long t = 0;
 #pragma unroll
-      for (int c = 0; c < kCluster; ++c) {
-        const Scratch* o = cluster.map_shared_rank(&s, c);
+      for (int c = 0; c < C; ++c) {
+        const Scratch<C>* o = peer<C>(&s, c);
         if (kUnit) t += o->hist.word[0][bin];
         else if (wide) t += o->hist.wide[bin];
         else t += (unsigned long long)o->hist.word[0][bin] + ((unsigned long long)o->hist.word[1][bin] << 16);
       }
-      s.total[threadIdx.x] = t;
+      s.total[i] = t;
       for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-      if (lane == 0) s.warp_part[threadIdx.x >> 5] = t;
+      if (lane == 0) s.warp_part[i >> 5] = t;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < kOwn) {
       unsigned long long t = 0;
-      for (int w = 0; w < kSegment / 32; ++w) t += s.warp_part[w];
-      s.segment_sum = t;
+      for (int w = 0; w < kSegment / 32; ++w) t += s.warp_part[threadIdx.x * (kSegment / 32) + w];
+      s.segment_sum[threadIdx.x] = t;
     }
-    cluster.sync();
+    row_sync<C>();
     if (threadIdx.x < 32) {
       // the segment, from the top, in which the weight so far reaches the target, then the bin within it: lane l
       // walks eight of its bins downwards, after a scan over the lanes has told it the weight above them
-      unsigned long long sums[kCluster], a = acc;
+      unsigned long long sums[kSegments], a = acc;
 #pragma unroll
-      for (int c = 0; c < kCluster; ++c) sums[c] = *cluster.map_shared_rank(&s.segment_sum, c);
+      for (int c = 0; c < kSegments; ++c) sums[c] = *peer<C>(&s.segment_sum[c % kOwn], c / kOwn);
       if (digit == 0) {
         unsigned long long total = 0;
 #pragma unroll
-        for (int c = 0; c < kCluster; ++c) total += sums[c];
+        for (int c = 0; c < kSegments; ++c) total += sums[c];
         target = target_of(total);
         if (lane == 0) s.found[3] = target;
       }
       int segment = -1;
 #pragma unroll
-      for (int c = kCluster - 1; c >= 0; --c)
+      for (int c = kSegments - 1; c >= 0; --c)
         if (segment < 0) {
           if (a + sums[c] >= target) segment = c;
           else a += sums[c];
@@ -246,7 +274,7 @@ __device__ uint32_t cluster_select(const cg::cluster_group& cluster, const Slice
           s.found[2] = 0ull;
         }
       } else {
-        const unsigned long long* totals = cluster.map_shared_rank(&s.total[0], segment);
+        const unsigned long long* totals = peer<C>(&s.total[segment % kOwn * kSegment], segment / kOwn);
         constexpr int kEach = kSegment / 32;
         unsigned long long mine[kEach], lane_sum = 0;
 #pragma unroll
@@ -314,8 +342,8 @@ struct Cut {
 
 // After a select that found `key` with `need` more units wanted among the ties: the id below
 // which ties are kept. Unit weights (top-k) keep exactly `need` ties.
-template <typename Item>
-__device__ Cut cut_with_ties(const cg::cluster_group& cluster, const Slice& row, Scratch& s, uint32_t key, unsigned long long need,
+template <int C, typename Item>
+__device__ Cut cut_with_ties(const Slice& row, Scratch<C>& s, uint32_t key, unsigned long long need,
                              unsigned long long equal, unsigned long long unit, Item item) {
   Cut cut{key, 0x7fffffff};
   if (key == 0u || unit == 0ull) return cut;
@@ -323,7 +351,7 @@ __device__ Cut cut_with_ties(const cg::cluster_group& cluster, const Slice& row,
   const unsigned long long want = (need + unit - 1) / unit;
   if (want * unit >= equal) return cut;  // all of them: no pass over the ids
   unsigned long long dummy, dummy2;
-  const uint32_t idk = cluster_select<true>(cluster, row, s, Count{want}, &dummy, &dummy2, false, 3,
+  const uint32_t idk = cluster_select<true>(row, s, Count{want}, &dummy, &dummy2, false, 3,
                                             [&](int token, float v, uint32_t& k2) {
     uint32_t k;
     if (!item(token, v, k) || k != key) return false;
@@ -360,7 +388,8 @@ __device__ __forceinline__ unsigned long long mass_target(float p, unsigned long
 // each is ranked by counting those before it, the k best fall into their places, masses are added up along
 // them, and the kept ones race. A token is kept while the mass before it is below top-p's target: the cut that the
 // selects above find, ties (equal keys, equal masses) by ascending id included.
-__device__ int finish_candidates(Scratch& s, int k, float p, float vmax, float inv_t, uint64_t seed, uint64_t counter, int best) {
+template <int C>
+__device__ int finish_candidates(Scratch<C>& s, int k, float p, float vmax, float inv_t, uint64_t seed, uint64_t counter, int best) {
   const int n = min(s.cand_n, kCompact), keep = min(k, n);
   for (int i = threadIdx.x; i < n; i += kThreads) {
     const uint32_t key = s.cand_key[i];
@@ -373,8 +402,8 @@ __device__ int finish_candidates(Scratch& s, int k, float p, float vmax, float i
                 (kk.z > key || (kk.z == key && ii.z < id)) + (kk.w > key || (kk.w == key && ii.w < id));
     }
     for (; j < n; ++j) before += s.cand_key[j] > key || (s.cand_key[j] == key && s.cand_id[j] < id);
-    s.sorted_key[before] = key;
-    s.sorted_id[before] = id;
+    s.hist.sorted.key[before] = key;
+    s.hist.sorted.id[before] = id;
   }
   __syncthreads();
   // two neighbouring places a thread: their masses, and the mass before them
@@ -384,7 +413,7 @@ __device__ int finish_candidates(Scratch& s, int k, float p, float vmax, float i
 #pragma unroll
   for (int u = 0; u < 2; ++u)
     if (at + u < keep) {
-      const float v = key_value(s.sorted_key[at + u]);
+      const float v = key_value(s.hist.sorted.key[at + u]);
       m[u] = v == v ? mass_of(v, vmax, inv_t) : 0ull;  // a NaN takes a place among the k and has no mass
     }
   unsigned long long upto = m[0] + m[1];
@@ -406,8 +435,8 @@ __device__ int finish_candidates(Scratch& s, int k, float p, float vmax, float i
 #pragma unroll
   for (int u = 0; u < 2; ++u) {
     if (at + u < keep && (!cuts || before < target)) {
-      const int token = s.sorted_id[at + u];
-      mine.take(race_score(key_value(s.sorted_key[at + u]), vmax, inv_t, seed, counter, token), token);
+      const int token = s.hist.sorted.id[at + u];
+      mine.take(race_score(key_value(s.hist.sorted.key[at + u]), vmax, inv_t, seed, counter, token), token);
     }
     before += m[u];
   }
@@ -425,10 +454,10 @@ __device__ int finish_candidates(Scratch& s, int k, float p, float vmax, float i
 }
 
 // This block's share of the cluster's row, brought into shared memory where it fits, and the best of it.
-__device__ Slice take_slice(const cg::cluster_group& cluster, const float* logits, int V, float* room, int room_floats, Best* best,
-                            bool* nan) {
-  const int each = ((V + kCluster - 1) / kCluster + 3) & ~3;
-  const int first = min(V, (int)cluster.block_rank() * each), n = min(each, V - first);
+template <int C>
+__device__ Slice take_slice(const float* logits, int V, float* room, int room_floats, Best* best, bool* nan) {
+  const int each = ((V + C - 1) / C + 3) & ~3;
+  const int first = min(V, row_rank<C>() * each), n = min(each, V - first);
   const float* from = logits + first;
   const bool keep = n <= room_floats;
   *best = Best{-INFINITY, 0x7fffffff};
@@ -475,33 +504,33 @@ __device__ Slice take_slice(const cg::cluster_group& cluster, const float* logit
   return Slice{keep ? room : from, first, n};
 }
 
-__global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads, 2)
+template <int C>
+__global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(kThreads, 2)
 sample_rows_kernel(int* __restrict__ out, const float* __restrict__ logits, int V,
                    const float* __restrict__ temperature, const int* __restrict__ top_k,
                    const float* __restrict__ top_p, const unsigned long long* __restrict__ seed,
                    const unsigned long long* __restrict__ counter, int room_floats) {
   asb::pdl_wait();  // the stream's previous kernel has completed (programmatic dependent launch)
   asb::pdl_launch_dependents();
-  __shared__ Scratch s;
+  __shared__ Scratch<C> s;
   extern __shared__ __align__(16) float room[];
-  const cg::cluster_group cluster = cg::this_cluster();
-  const int b = blockIdx.x / kCluster;
-  const bool leads = cluster.block_rank() == 0;
+  const int b = blockIdx.x / C;
+  const bool leads = row_rank<C>() == 0;
   const float temp = temperature[b];
 
   if (threadIdx.x == 0) s.cand_n = 0;
   Best top;
   bool odd;
-  const Slice row = take_slice(cluster, logits + (size_t)b * V, V, room, room_floats, &top, &odd);
+  const Slice row = take_slice<C>(logits + (size_t)b * V, V, room, room_floats, &top, &odd);
   s.odd = 0;
   __syncthreads();
   if (odd) s.odd = 1;
-  top = cluster_best(cluster, s, top, 0);
+  top = cluster_best(s, top, 0);
   const float vmax = top.score;
   const int best = top.token == 0x7fffffff ? 0 : top.token;  // a row of NaN or -inf only
   if (!(temp > 0.f)) {  // greedy: the single best, lowest id among equals
     if (leads && threadIdx.x == 0) out[b] = best;
-    cluster.sync();  // nobody leaves while a neighbour may still read its best
+    row_sync<C>();  // nobody leaves while a neighbour may still read its best
     return;
   }
   const float inv_t = 1.f / temp;
@@ -509,9 +538,9 @@ sample_rows_kernel(int* __restrict__ out, const float* __restrict__ logits, int 
   const float p = top_p[b];
   // masses are added up in 64-bit words where a slice has more elements than two 32-bit words can hold, or where a
   // mass may lie outside [0, 2^32]
-  bool wide = V > kCluster * (kSplitSlice - 3) || isinf(vmax);
+  bool wide = V > C * (kSplitSlice - 3) || isinf(vmax);
 #pragma unroll
-  for (int c = 0; c < kCluster; ++c) wide |= *cluster.map_shared_rank(&s.odd, c) != 0;
+  for (int c = 0; c < C; ++c) wide |= *peer<C>(&s.odd, c) != 0;
 
   // top-k
   const int k = top_k[b];
@@ -534,7 +563,7 @@ sample_rows_kernel(int* __restrict__ out, const float* __restrict__ logits, int 
       const uint32_t top_bin = order_key(vmax) >> 24;
       const uint32_t floor_key = top_bin >= 3u ? (top_bin - 3u) << 24 : 0u;
       for (int digits = 1; digits <= 2 && !few; ++digits) {
-        from = cluster_select<true>(cluster, row, s, kth, &above, &equal, false, digits, [&](int token, float v, uint32_t& key) {
+        from = cluster_select<true>(row, s, kth, &above, &equal, false, digits, [&](int token, float v, uint32_t& key) {
           key = order_key(v);
           return key >= floor_key;
         }, One{});
@@ -543,12 +572,12 @@ sample_rows_kernel(int* __restrict__ out, const float* __restrict__ logits, int 
       }
     }
     if (!few) {
-      const uint32_t key = cluster_select<true>(cluster, row, s, kth, &above, &equal, false, 3, any, One{});
-      kcut = cut_with_ties(cluster, row, s, key, (unsigned long long)k - above, equal, 1ull, any);
+      const uint32_t key = cluster_select<true>(row, s, kth, &above, &equal, false, 3, any, One{});
+      kcut = cut_with_ties(row, s, key, (unsigned long long)k - above, equal, 1ull, any);
     }
     if (k <= kCompact) {
       // to the first block, which ends the row alone (the order they arrive in does not matter)
-      Scratch* lead = cluster.map_shared_rank(&s, 0);
+      Scratch<C>* lead = peer<C>(&s, 0);
       for_each_value(row, [&](int token, float v) {
         const uint32_t key = order_key(v);
         if (few ? key >= from : kcut.keeps(key, token)) {
@@ -556,7 +585,7 @@ sample_rows_kernel(int* __restrict__ out, const float* __restrict__ logits, int 
           if (at < kCompact) { lead->cand_key[at] = key; lead->cand_id[at] = token; }
         }
       });
-      cluster.sync();
+      row_sync<C>();
       if (!leads) return;  // (and the first block reads nothing of its neighbours from here on)
       const int token = finish_candidates(s, k, p, vmax, inv_t, sd, ctr, best);
       if (threadIdx.x == 0) out[b] = token;
@@ -575,11 +604,11 @@ sample_rows_kernel(int* __restrict__ out, const float* __restrict__ logits, int 
     // keep a token while the mass ranked above it is < p * total: find the first key whose
     // cumulative mass (itself included) exceeds p * total, ties by ascending id
     unsigned long long above, equal, target = 0;
-    const uint32_t key = cluster_select<false>(cluster, row, s, [&](unsigned long long total) { return mass_target(p, total); },
+    const uint32_t key = cluster_select<false>(row, s, [&](unsigned long long total) { return mass_target(p, total); },
                                                &above, &equal, wide, 3, kept, mass);
     target = s.found[3];
     // mass of one tied token (all ties share the key, hence the value)
-    pcut = cut_with_ties(cluster, row, s, key, target - above, equal, mass_of(key_value(key), vmax, inv_t), kept);
+    pcut = cut_with_ties(row, s, key, target - above, equal, mass_of(key_value(key), vmax, inv_t), kept);
   }
 
   // exponential race among the kept
@@ -589,21 +618,21 @@ sample_rows_kernel(int* __restrict__ out, const float* __restrict__ logits, int 
     if (!kcut.keeps(key, token) || !pcut.keeps(key, token)) return;
     winner.take(race_score(v, vmax, inv_t, sd, ctr, token), token);
   });
-  winner = cluster_best(cluster, s, winner, 1);
+  winner = cluster_best(s, winner, 1);
   if (leads && threadIdx.x == 0) out[b] = winner.token == 0x7fffffff ? best : winner.token;
-  cluster.sync();  // nobody leaves while a neighbour may still read its best
+  row_sync<C>();  // nobody leaves while a neighbour may still read its best
 }
 
-__global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads, 2)
+template <int C>
+__global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(kThreads, 2)
 argmax_rows_kernel(int* __restrict__ out, const float* __restrict__ logits, int V) {
   asb::pdl_wait();  // the stream's previous kernel has completed (programmatic dependent launch)
   asb::pdl_launch_dependents();
   __shared__ Best slots[1 + kWarps];  // this block's best, and its warps'
-  const cg::cluster_group cluster = cg::this_cluster();
-  const int b = blockIdx.x / kCluster;
+  const int b = blockIdx.x / C;
   Best top;
   bool nan;
-  take_slice(cluster, logits + (size_t)b * V, V, nullptr, -1, &top, &nan);
+  take_slice<C>(logits + (size_t)b * V, V, nullptr, -1, &top, &nan);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     const float os = __shfl_xor_sync(0xffffffffu, top.score, o);
@@ -616,15 +645,15 @@ argmax_rows_kernel(int* __restrict__ out, const float* __restrict__ logits, int 
     for (int w = 1; w < kWarps; ++w) top.take(slots[1 + w].score, slots[1 + w].token);
     slots[0] = top;
   }
-  cluster.sync();
-  if (cluster.block_rank() == 0 && threadIdx.x == 0) {
-    for (int c = 1; c < kCluster; ++c) {
-      const Best o = *cluster.map_shared_rank(&slots[0], c);
+  row_sync<C>();
+  if (row_rank<C>() == 0 && threadIdx.x == 0) {
+    for (int c = 1; c < C; ++c) {
+      const Best o = *peer<C>(&slots[0], c);
       top.take(o.score, o.token);
     }
     out[b] = top.token == 0x7fffffff ? 0 : top.token;  // a row of NaN or -inf only
   }
-  cluster.sync();  // nobody leaves while the first block reads its best
+  row_sync<C>();  // nobody leaves while the first block reads its best
 }
 
 __global__ void presence_penalty_kernel(float* __restrict__ logits, const int* __restrict__ rows,
@@ -636,13 +665,60 @@ __global__ void presence_penalty_kernel(float* __restrict__ logits, const int* _
   if (i < n && tokens[i] >= 0 && tokens[i] < V) logits[(size_t)rows[i] * V + tokens[i]] -= amounts[i];
 }
 
+// Floats of a row that a block of C has.
+int slice_floats(int V, int C) { return ((V + C - 1) / C + 3) & ~3; }
+
+// Blocks a row, starting from what a row of this length is worth: what it takes per element against what the barriers
+// of a cluster cost (top-p alone, one row of 4,000: 20.3 us in eight blocks, 13.6 in one; of 32,000: 24.4, 44.4). Half as
+// many while all rows' blocks are more than run well at once (clusters of eight leave SMs out early) and, where rows are
+// held in shared memory, while two blocks of the longer slice share an SM. 256 rows, top-p alone, eight blocks and those
+// taken here: of 500 216 -> 13 us, of 32,000 260 -> 93, of 64,000 297 -> 193; 48 rows of 32,000 62 -> 33, of 151,936
+// eight as before (108; in four 116).
+int blocks_a_row(int B, int V, int one_below, int four_below, bool held) {
+  constexpr int kTwoAnSM = 18 * 1024;  // floats
+  int C = V <= one_below ? 1 : (V <= four_below ? 4 : 8);
+  const int most8 = held ? 74 : 148;
+  while (C > 1) {
+    if ((long long)B * C <= (C == 8 ? most8 : (C == 4 ? 256 : 296))) break;
+    if (held && slice_floats(V, C / 2) > kTwoAnSM) break;
+    C /= 2;
+  }
+  return C;
+}
+int sample_blocks(int B, int V) { return blocks_a_row(B, V, 7000, 30000, true); }
+// The same for the largest logit alone, which every block reads in place (256 rows of 32,000: 12.7 us in eight, 4.9 in
+// one; of 151,936: 39 and 31).
+int argmax_blocks(int B, int V) { return blocks_a_row(B, V, 16000, 16000, false); }
+
+template <int C>
+int launch_argmax(int* out, const float* logits, int B, int V, cudaStream_t stream) {
+  asb::launch(argmax_rows_kernel<C>, C * B, kThreads, 0, stream, out, logits, V);
+  return asb::check_launch("argmax_rows");
+}
+
+template <int C>
+int launch_sample(int* out, const float* logits, int B, int V, const float* temperature, const int* top_k, const float* top_p,
+                  const unsigned long long* seed, const unsigned long long* counter, cudaStream_t stream) {
+  // a slice too long for shared memory is read in place in every pass
+  const int each = slice_floats(V, C), room = each <= kMaxSlice<C> ? each : 0;
+  cudaError_t e = cudaFuncSetAttribute(sample_rows_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(room * sizeof(float)));
+  if (e != cudaSuccess) return asb::fail("sample_rows: shared memory of %d floats: %s", room, cudaGetErrorString(e));
+  asb::launch(sample_rows_kernel<C>, C * B, kThreads, room * sizeof(float), stream, out, logits, V, temperature, top_k, top_p,
+              seed, counter, room);
+  return asb::check_launch("sample_rows");
+}
+
 }  // namespace
 
 extern "C" int asb_argmax_rows(int* out, const float* logits, int B, int V, cudaStream_t stream) {
   if (B == 0) return 0;
-  if (B > 0x7fffffff / kCluster) return asb::fail("argmax_rows: %d rows", B);
-  asb::launch(argmax_rows_kernel, kCluster * B, kThreads, 0, stream, out, logits, V);
-  return asb::check_launch("argmax_rows");
+  if (B > 0x7fffffff / kMostBlocks) return asb::fail("argmax_rows: %d rows", B);
+  switch (argmax_blocks(B, V)) {
+    case 1: return launch_argmax<1>(out, logits, B, V, stream);
+    case 2: return launch_argmax<2>(out, logits, B, V, stream);
+    case 4: return launch_argmax<4>(out, logits, B, V, stream);
+    default: return launch_argmax<8>(out, logits, B, V, stream);
+  }
 }
 
 // Each (row, token) pair must appear once: the penalty is subtracted once per distinct token.
@@ -659,12 +735,11 @@ extern "C" int asb_sample_rows(int* out, const float* logits, int B, int V,
                                cudaStream_t stream) {
   if (B == 0) return 0;
   if (V < 1) return asb::fail("sample_rows: vocabulary %d", V);
-  if (B > 0x7fffffff / kCluster) return asb::fail("sample_rows: %d rows", B);
-  // a slice too long for shared memory is read in place in every pass
-  const int each = ((V + kCluster - 1) / kCluster + 3) & ~3, room = each <= kMaxSlice ? each : 0;
-  cudaError_t e = cudaFuncSetAttribute(sample_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(room * sizeof(float)));
-  if (e != cudaSuccess) return asb::fail("sample_rows: shared memory of %d floats: %s", room, cudaGetErrorString(e));
-  asb::launch(sample_rows_kernel, kCluster * B, kThreads, room * sizeof(float), stream, out, logits, V, temperature, top_k, top_p,
-              seed, counter, room);
-  return asb::check_launch("sample_rows");
+  if (B > 0x7fffffff / kMostBlocks) return asb::fail("sample_rows: %d rows", B);
+  switch (sample_blocks(B, V)) {
+    case 1: return launch_sample<1>(out, logits, B, V, temperature, top_k, top_p, seed, counter, stream);
+    case 2: return launch_sample<2>(out, logits, B, V, temperature, top_k, top_p, seed, counter, stream);
+    case 4: return launch_sample<4>(out, logits, B, V, temperature, top_k, top_p, seed, counter, stream);
+    default: return launch_sample<8>(out, logits, B, V, temperature, top_k, top_p, seed, counter, stream);
+  }
 }

@@ -570,6 +570,39 @@ def test_sampled_token_wins_the_plain_race(ops, V, k, p, temp):
         assert score[out[r]] >= score[kept].max() * (1 - 1e-5)
 
 
+@pytest.mark.parametrize("V", [5, 500, 4099, 50001, 151936])
+@pytest.mark.parametrize("k,p,temp", [(20, 0.95, 0.6), (0, 0.95, 0.8), (2000, 0.9, 1.0), (0, 1.0, 1.0), (3, 1.0, 1.0), (0, 1.0, 0.0)])
+def test_a_rows_token_does_not_depend_on_how_many_rows_there_are(ops, V, k, p, temp):
+    """How many blocks share a row goes by the number of rows: the same row, seed and counter draw the same token in a
+    batch of one and of hundreds, with masked tokens, infinities and NaN among the logits and with ties at every cut."""
+    g = torch.Generator().manual_seed(V)
+    rows = torch.randn(7, V, generator=g) * 3
+    rows[1] = (rows[1] * 2).round() / 2
+    rows[2, torch.randperm(V, generator=g)[: V // 2]] = -math.inf
+    rows[3, V // 3] = math.nan
+    rows[4, V // 2] = math.inf
+    rows[5], rows[6] = -math.inf, math.nan
+
+    def draw(logits, seeds):
+        n = logits.shape[0]
+        setting = lambda v, dt: torch.full((n,), v, dtype=dt, device="cuda")  # noqa: E731
+        args = setting(temp, torch.float32), setting(k, torch.int32), setting(p, torch.float32), seeds, seeds * 3
+        return ops.sample_rows(logits, *args).cpu(), ops.argmax_rows(logits).cpu()
+
+    seeds = torch.arange(7, device="cuda") + 11
+    alone = [draw(rows[r : r + 1].cuda(), seeds[r : r + 1]) for r in range(7)]
+    sampled, best = (torch.cat(t) for t in zip(*alone))
+    assert sampled[5] == sampled[6] == 0 and sampled[3] != V // 3  # nothing to choose from; a NaN is not chosen
+    finite = [torch.where(torch.isnan(r), -math.inf, r) for r in rows]
+    assert best.tolist() == [int(torch.nonzero(r == r.max())[0]) for r in finite]
+    if p < 1:
+        assert sampled[4] == V // 2
+    for n in (30, 70, 140, 290, 600):
+        which = torch.arange(n) % 7
+        got = draw(rows[which].cuda(), seeds[which.cuda()])
+        assert torch.equal(got[0], sampled[which]) and torch.equal(got[1], best[which]), n
+
+
 def test_presence_penalty(ops):
     logits = torch.zeros(2, 10, device="cuda")
     ops.presence_penalty(
