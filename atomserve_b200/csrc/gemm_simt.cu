@@ -30,6 +30,7 @@ constexpr int kWarps = kThreads / 32;
 constexpr int kRun = 256;   // k per chain
 constexpr int kQuarters = 4;
 constexpr int BK = 16;      // k per stage; kRun is a multiple
+constexpr int kSMs = 148;
 
 // Two multiply-adds in one instruction, each rounded as fmaf rounds: d = a * b + d on both halves.
 __device__ __forceinline__ void fma2(unsigned long long& d, unsigned long long a, unsigned long long b) {
@@ -368,9 +369,13 @@ template <typename TIn, typename TOut>
 int tiles(void* out, const void* x, const void* w, const void* residual, int M, int N, int K, cudaStream_t stream) {
   const bool vec = K % 4 == 0 && ((((uintptr_t)x) | ((uintptr_t)w)) & (4 * sizeof(TIn) - 1)) == 0;
   const bool cut = K > (kQuarters - 1) * kRun;  // a run for every block of a cluster
-  // tiles of 32 rows for up to 32: half the multiply-adds would be padding in the other
+  // Tiles of 32 rows for up to 32 (half the multiply-adds would be padding in the other), and where they come to one block
+  // an SM: a block's chain of stages is then what counts, and half as long (300 rows of 96 over 512: 9.8 us with 64 rows a
+  // tile, 7.3 with 32; of 2,048 over 2,048, 64 rows: 36.3 and 34.9; just beyond one block an SM, 1,000 rows of 256 over
+  // 640: 19.6 and 22.8).
+  const long long blocks = (long long)(cut ? kQuarters : 1) * ((M + 31) / 32) * ((N + BN - 1) / BN);
 #define ASB_TILE(BM_, C_, V_) return launch_tile<TIn, TOut, BM_, C_, V_>(out, x, w, residual, M, N, K, stream)
-  if (M <= 32) {
+  if (M <= 32 || blocks <= kSMs) {
     if (cut) { if (vec) ASB_TILE(32, kQuarters, true); ASB_TILE(32, kQuarters, false); }
     if (vec) ASB_TILE(32, 1, true);
     ASB_TILE(32, 1, false);

@@ -85,12 +85,15 @@ def test_linear_rows_do_not_depend_on_the_batch(ops):
 
 
 @pytest.mark.parametrize("K", [1, 12, 30, 256, 260, 771, 772, 1028, 8192, 8460, 12288])
-@pytest.mark.parametrize("N", [1, 63, 130, 384])
+@pytest.mark.parametrize("N", [1, 63, 130, 384, 1600, 4800])
 def test_float32_linear_in_both_kernels(ops, N, K):
     """The float32 product on either side of each of its dispatch's lines (4, 8, 16 and 32 rows; K by a multiple of 4,
-    by fewer runs of 256 than quarters, by more than eight runs a block; rows off 16 bytes): against float64, within the
+    by fewer runs of 256 than quarters, by more than eight runs a block; rows off 16 bytes; matrices whose tiles of 32 rows
+    are fewer than the SMs with some of these numbers of rows and more with others): against float64, within the
     bound of a sum cut into chains of 256, and each row the same bits whatever the number of rows beside it."""
     g = torch.Generator().manual_seed(N + K)
+    if N > 384 and K > 1028:
+        K = 4096 + K % 7  # (as many blocks, fewer multiply-adds for the float64 product)
     x = torch.randn(131, K, generator=g).cuda()
     w = torch.randn(N, K, generator=g).cuda()
     res = torch.randn(131, N, generator=g).cuda()
@@ -107,6 +110,20 @@ def test_float32_linear_in_both_kernels(ops, N, K):
     off = torch.empty(131 * K + 1, device="cuda")[1:].view(131, K).copy_(x)  # rows that start off 16 bytes
     for M in (3, 20, 131):
         assert torch.equal(ops.linear(off[:M], w), whole[:M])
+
+
+@pytest.mark.parametrize("M", [3, 8, 13, 30, 70, 131])
+@pytest.mark.parametrize("N,K", [(130, 772), (63, 771), (384, 8460), (5, 96)])
+def test_float32_linear_keeps_what_is_not_finite_in_its_row_and_column(ops, M, N, K):
+    """A NaN among the inputs of one row, an infinity in one row of the matrix: that row, that column, and no other."""
+    g = torch.Generator().manual_seed(M + N + K)
+    x, w = torch.randn(M, K, generator=g).cuda(), torch.randn(N, K, generator=g).cuda()
+    plain_out = ops.linear(x, w)
+    x[M // 2, K - 1], w[N // 2, K // 3] = math.nan, math.inf
+    bad = torch.zeros(M, N, dtype=torch.bool, device="cuda")
+    bad[M // 2], bad[:, N // 2] = True, True
+    out = ops.linear(x, w)
+    assert torch.equal(~torch.isfinite(out), bad) and torch.equal(out[~bad], plain_out[~bad])
 
 
 @pytest.mark.parametrize("M", [1, 4, 7, 16, 17])
