@@ -1039,31 +1039,37 @@ int launch_decode(const DecodeParams& p, cudaStream_t stream) {
   return asb::check_launch("decode_merge");
 }
 
-template <int HD>
+template <int HD, bool Half>
 int resident_blocks(int sms) {
   int per_sm = 0;
-  auto kern = decode_attention_kernel<HD, false>;
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, decode_smem(HD, 16));
+  auto kern = decode_attention_kernel<HD, Half>;
+  const int smem = decode_smem(HD, Half ? 8 : 16);
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   asb::prefer_shared_carveout((const void*)kern);
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, decode_smem(HD, 16)) != cudaSuccess) return 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, smem) != cudaSuccess) return 0;
   return per_sm * sms;
 }
 
 }  // namespace
 
-// How many blocks of the decode kernel the device holds at once (blocks per SM x SMs), which is
-// what the caller's choice of ranges aims to fill; 0 for a head size not served.
-extern "C" int asb_decode_attention_resident_blocks(int hd) {
+// How many blocks of the decode kernel for `group` heads a kv head the device holds at once (blocks per SM x SMs), which
+// is what the caller's choice of ranges aims to fill; 0 for a head size not served. (Head size 64 with up to 8 heads: four
+// an SM; with three counted, 128 rows of 2,048 keys, 32 heads over 8, took 100 us instead of 97.)
+extern "C" int asb_decode_attention_resident(int hd, int group) {
   if (hd != 64 && hd != 128) return 0;
-  static int cached[2] = {0, 0};
-  int& slot = cached[hd == 128];
+  static int cached[4] = {0, 0, 0, 0};
+  int& slot = cached[2 * (hd == 128) + (group <= 8)];
   if (slot) return slot;
   int device = 0, sms = 0;
   if (cudaGetDevice(&device) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
     return 0;
-  return slot = hd == 64 ? resident_blocks<64>(sms) : resident_blocks<128>(sms);
+  if (group <= 8) return slot = hd == 64 ? resident_blocks<64, true>(sms) : resident_blocks<128, true>(sms);
+  return slot = hd == 64 ? resident_blocks<64, false>(sms) : resident_blocks<128, false>(sms);
 }
+
+// The same for more than 8 heads a kv head, the least of them.
+extern "C" int asb_decode_attention_resident_blocks(int hd) { return asb_decode_attention_resident(hd, 16); }
 
 // 1 if this (head size, group) is served by the tensor-core kernels.
 extern "C" int asb_attention_mma_supported(int hd, int group) {

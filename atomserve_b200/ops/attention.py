@@ -66,14 +66,10 @@ def plan_partitions(num_tokens: int, num_requests: int, num_kv_heads: int, group
 @functools.lru_cache(maxsize=4096)
 def plan_decode_partitions(rows: int, num_kv_heads: int, group: int, max_context: int, window: int,
                            head_dim: int = 128) -> tuple[int, int]:  # fmt: skip
-    """(partition size, partitions) for the tensor-core decode kernel, one block per (row, kv
-    head, partition). The device holds a fixed number of its blocks at once, so the blocks run in
-    waves; the choice minimises waves x (64-key tiles per block + 3 tiles' worth of start-up) plus
-    half a tile per partition for the merge, which is what a sweep over batch 4-128 and context
-    1k-8k fitted: small batches want one nearly full wave, large ones two to five, and a count
-    that spills a few blocks into one more wave is the worst. Never below one tile of 64 keys a
-    block (which only short contexts at small batches choose: batch 1 at 512 keys runs 8.2 us with
-    four partitions of 128 against 10.3 us with two of 256)."""
+    """(partition size, partitions) that even out the waves of blocks, one per (row, kv head, partition), if every row
+    had the longest context: the fewest of waves x (64-key tiles per block + 3 tiles' worth of start-up) plus half a tile
+    per partition for a merge. `plan_decode_ranges` asks it whether rows of several waves are worth cutting at all; how
+    they are cut the decode kernel works out from the rows' own lengths."""
     blocks = rows * num_kv_heads * -(-group // 16)
     span = max_context if window <= 0 else min(max_context, window)
     resident = lib().asb_decode_attention_resident_blocks(head_dim) or 3 * 148
@@ -97,25 +93,43 @@ def plan_decode_partitions(rows: int, num_kv_heads: int, group: int, max_context
 def plan_decode_ranges(rows: int, num_kv_heads: int, group: int, max_context: int, window: int, head_dim: int = 128,
                        partitions: tuple[int, int] | None = None) -> int:  # fmt: skip
     """Equal ranges into which the decode kernel cuts the keys of all rows, each for a block per kv head (and 16 of its
-    heads); 0: each row is a range, and there is no merge. Where rows of the longest context would not be split, nothing
-    is, nor where rows of up to 24 key tiles make blocks for half of what the device holds at once (64 rows of 100 to 300
-    keys, 8 kv heads: 25.6 -> 16.5 us). Otherwise as many ranges as the device holds at once, three blocks an SM, if that
-    leaves a block eight key tiles of the longest context; with less work three quarters of them, and no more than there
-    are tiles: a merge of more shares then costs more than the shorter walk saves (one request of 12,288 keys and 8 kv
-    heads: 18.7 us in 16 ranges, 16.3 in 40, 19.3 in 55; of 2,048 keys: 10.8 us in 8, 9.4 in 32, 8.4 in 40; 64 requests
-    of 300 to 3,000 keys: 90.3 us in 24, 78.4 in 55)."""
-    size, parts = partitions or plan_decode_partitions(rows, num_kv_heads, group, max_context, window, head_dim)
-    if parts <= 1:
-        return 0
+    heads); 0: each row is a range, and there is no merge. `partitions` (size, parts) asks for rows x parts of them.
+
+    Nothing is cut where `plan_decode_partitions` would not split rows of the longest context (unless all rows run at once
+    and walk more than 64 tiles, so that the longest row's end is worth a merge: 32 rows of 6,000 to 12,000 keys, 12 heads
+    over 12 of size 64: 161 -> 136 us), nor where rows of up to 24 key tiles make blocks for half of what the device holds at once
+    (64 rows of 100 to 300 keys, 8 kv heads: 25.6 -> 16.5 us). Otherwise as many ranges as the device holds blocks at
+    once, if that leaves a block eight key tiles of the longest context; with less work three quarters of them, and no
+    more than there are tiles: a merge of more shares then costs more than the shorter walk saves (one request of 12,288
+    keys and 8 kv heads: 18.7 us in 16 ranges, 16.3 in 40, 19.3 in 55; of 2,048 keys: 10.8 us in 8, 9.4 in 32, 8.4 in 40;
+    64 requests of 300 to 3,000 keys: 90.3 us in 24, 78.4 in 55).
+
+    The merge costs about five tiles' time of a kernel with up to 8 heads a kv head (three with more, whose tiles take
+    longer): rows that all run at once and walk no more than that further than a range would stay whole, and so do rows of
+    up to eight tiles that would be cut in two (5 rows of 100 to 300 keys, 32 heads over 8: 7.7 -> 6.3 us; 16 of 500, 12 heads over 12 of size 64:
+    12.6 -> 8.7; 128 of 500, 16 heads over one: 22.7 -> 16.7)."""
     if partitions:
-        return rows * parts
-    resident = lib().asb_decode_attention_resident_blocks(head_dim) or 3 * 148
+        return rows * partitions[1] if partitions[1] > 1 else 0
+    resident = lib().asb_decode_attention_resident(head_dim, group) or 3 * 148
     lanes = num_kv_heads * -(-group // 16)
     longest = -(-(min(max_context, window) if window > 0 else max_context) // 64)
+    one_wave = rows * lanes <= resident
+    if not (one_wave and longest > 64) and plan_decode_partitions(rows, num_kv_heads, group, max_context, window, head_dim)[1] <= 1:
+        return 0
     if longest <= 24 and 2 * rows * lanes >= resident:
         return 0
     full, tiles = max(1, resident // lanes), rows * longest
-    return full if tiles >= 8 * full else max(1, min(3 * full // 4, tiles))
+    ranges = full if tiles >= 8 * full else max(1, min(3 * full // 4, tiles))
+    walk = -(-tiles // ranges)
+    if one_wave and longest <= max(walk + (5 if group <= 8 else 3), min(2 * walk, 8)):
+        return 0
+    return ranges
+
+
+def decode_scratch_floats(rows: int, ranges: int, num_kv_heads: int, group: int, head_dim: int) -> int:
+    """float32 elements of the decode kernel's scratch: four words a row, and per block (a range and a kv head, or 16 of its
+    heads) two shares of up to 16 heads, each its output, maximum and sum."""
+    return 4 * rows + 2 * ranges * num_kv_heads * -(-group // 16) * min(group, 16) * (head_dim + 2)
 
 
 def plan_portion_parts(q_lens: list[int] | None, num_kv_heads: int, group: int, max_context: int, window: int) -> int:
@@ -266,8 +280,7 @@ def _paged_attention_mma(q, out, k_cache, v_cache, block_tables, req_q_start, re
         that holds longer portions too. Its scratch belongs to the stream that is current now."""
         group = H // KV
         ranges = plan_decode_ranges(short_rows, KV, group, max_context, span, hd, partitions)
-        floats = 4 * (compact or T) + 2 * ranges * KV * -(-group // 16) * min(group, 16) * (hd + 2)
-        scratch = torch.empty(floats, device=q.device, dtype=torch.float32) if ranges else None
+        scratch = torch.empty(decode_scratch_floats(compact or T, ranges, KV, group, hd), device=q.device, dtype=torch.float32) if ranges else None
 
         def launch():
             check(lib().asb_decode_attention(

@@ -39,6 +39,50 @@ def test_decode_attention_partition_plans_cover_every_context(monkeypatch):
     attention.plan_decode_partitions.cache_clear()
 
 
+def test_decode_attention_ranges_fill_the_device_and_their_scratch(monkeypatch):
+    """Whatever the batch, context and window: no more ranges than the device holds blocks at once or than there are
+    tiles, none where a cut would not shorten the walk by more than the merge costs; and the scratch holds every share a
+    block can leave (its first row's and its last row's, for each of its heads)."""
+    import random
+
+    import atomserve_b200.ops.attention as attention
+
+    class FakeLibrary:
+        def asb_decode_attention_resident(self, head_dim, group):
+            return 592 if head_dim == 64 and group <= 8 else 444
+
+        def asb_decode_attention_resident_blocks(self, head_dim):
+            return 444
+
+    monkeypatch.setattr(attention, "lib", lambda: FakeLibrary())
+    attention.plan_decode_partitions.cache_clear()
+    rng = random.Random(2)
+    cut = 0
+    for _ in range(4000):
+        rows = rng.choice([1, 2, 3, 8, 17, 64, 128, 200])
+        kv, group = rng.choice([(1, 1), (2, 4), (8, 4), (8, 8), (4, 20), (1, 16), (12, 1)])
+        context, window, hd = rng.choice([1, 63, 64, 65, 300, 512, 1500, 2048, 8191, 40000]), rng.choice([0, 0, 100, 4096]), rng.choice([64, 128])
+        ranges = attention.plan_decode_ranges(rows, kv, group, context, window, hd)
+        lanes, longest = kv * -(-group // 16), -(-(min(context, window) if window else context) // 64)
+        resident = FakeLibrary().asb_decode_attention_resident(hd, group)
+        assert 0 <= ranges and ranges * lanes <= max(resident, lanes) and ranges <= rows * longest
+        if ranges:
+            cut += 1
+            # the walk is shorter by more than a merge, unless whole rows would run in several waves
+            assert rows * lanes > resident or longest > -(-rows * longest // ranges) + 3
+        # the kernel: shares 2 * block and 2 * block + 1 of GC heads, outputs first, then (max, sum) pairs, behind int4 a row
+        blocks, heads = ranges * lanes, min(group, 16)
+        outputs = 4 * rows + 2 * blocks * heads * hd
+        last_pair = outputs + ((2 * blocks - 1) * heads + heads - 1) * 2 + 1 if blocks else outputs - 1
+        assert attention.decode_scratch_floats(rows, ranges, kv, group, hd) == last_pair + 1
+        assert attention.plan_decode_ranges(rows, kv, group, context, window, hd, (64, 3)) == 3 * rows
+        assert attention.plan_decode_ranges(rows, kv, group, context, window, hd, (1 << 30, 1)) == 0
+    assert cut > 500
+    assert attention.plan_decode_ranges(1, 8, 4, 2048, 0) == 32 and attention.plan_decode_ranges(64, 8, 4, 3000, 0) == 55
+    assert attention.plan_decode_ranges(64, 8, 4, 300, 0) == 0 and attention.plan_decode_ranges(5, 8, 4, 300, 0) == 0
+    attention.plan_decode_partitions.cache_clear()
+
+
 def test_portions_are_planned_for_their_own_contexts():
     """A short prompt beside one long decode is not divided for the decode's context; without the positions the step's
     longest context stands in, and one part is the answer where the lengths are not told at all."""
