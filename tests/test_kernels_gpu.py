@@ -916,20 +916,40 @@ def test_gemm_tcgen05_on_pairs_of_sms(ops, M, N, K, rows):
         assert torch.allclose(fused.double().cpu(), gate / (1 + torch.exp(-gate)) * up, atol=3e-2, rtol=3e-2)
 
 
-@pytest.mark.parametrize("lens,H,KV,hd,bs,window,ranges", [
-    ([1], 8, 2, 128, 16, None, 7),                                    # more ranges than tiles
-    ([1, 64, 65, 129, 4000], 8, 2, 128, 16, None, 13),                # ranges over several rows and within one
-    ([1 + (53 * i) % 700 for i in range(300)], 4, 2, 64, 8, None, 50),  # more rows than a round of the scan, rows of 1 to 11 tiles
-    ([500, 3, 2000, 777], 40, 2, 128, 16, 300, 31),                   # twenty heads a kv head: two chunks; a window
-    ([900] * 6, 16, 1, 64, 4, None, 64),                              # sixteen heads; every range ends inside a row
+def ranges_end_with_rows(tiles, ranges):
+    """Whether the decode kernel cuts these rows (of so many 64-key tiles) one by one, each into equal ranges of its own,
+    or all of them as one sequence whose ranges run from one row into the next (tiles_a_range in csrc/attention_mma.cu)."""
+    least = -(-sum(tiles) // ranges)
+    return len(tiles) <= 128 and any(sum(-(-t // c) for t in tiles) <= ranges for c in range(max(1, least), least + 3))
+
+
+def tiles_of(lens, q_lens, window):
+    """64-key tiles of each row of the requests that bring at most eight tokens."""
+    at = [p for n, m in zip(lens, q_lens) if m <= 8 for p in range(n - m, n)]
+    return [p // 64 - (max(0, p - window + 1) if window else 0) // 64 + 1 for p in at]
+
+
+@pytest.mark.parametrize("lens,H,KV,hd,bs,window,ranges,by_row", [
+    ([1], 8, 2, 128, 16, None, 7, True),                                # more ranges than tiles
+    ([1, 64, 65, 129, 4000], 8, 2, 128, 16, None, 13, True),            # most ranges within one row
+    ([1, 64, 65, 129, 4000], 8, 2, 128, 16, None, 3, False),            # a range over several rows, then two within one
+    ([1 + (53 * i) % 700 for i in range(300)], 4, 2, 64, 8, None, 50, False),  # more rows than a round of the scan, rows of 1 to 11 tiles
+    ([500, 3, 2000, 777], 40, 2, 128, 16, 300, 31, True),               # twenty heads a kv head: two chunks; a window
+    ([500, 3, 2000, 777], 40, 2, 128, 16, 300, 3, False),               # the same, ranges across rows
+    ([900] * 6, 16, 1, 64, 4, None, 64, True),                          # sixteen heads, two tiles a range
+    ([900] * 6, 16, 1, 64, 4, None, 4, False),                          # sixteen heads, every range but the last ends inside a row
+    ([900, 130, 64, 1500, 70, 333], 16, 1, 128, 16, None, 5, False),
+    ([900, 130, 64, 1500, 70, 333], 9, 1, 128, 16, None, 4, False),     # nine heads
+    ([40 + 97 * i % 600 for i in range(128)], 8, 8, 128, 16, None, 37, False),  # as many rows as threads, one head a kv head
 ])  # fmt: skip
 @pytest.mark.parametrize("stored", [False, True])
-def test_decode_attention_ranges(ops, monkeypatch, lens, H, KV, hd, bs, window, ranges, stored):
+def test_decode_attention_ranges(ops, monkeypatch, lens, H, KV, hd, bs, window, ranges, by_row, stored):
     """The decode kernel's equal ranges of all rows' key tiles, for numbers of ranges that the planner would not take,
     against the plain attention. bfloat16 values and probabilities: 2^-8 of values of size one, a few times over."""
     import atomserve_b200.ops.attention as attention
 
     rows = len(lens)
+    assert ranges_end_with_rows(tiles_of(lens, [1] * rows, window), ranges) == by_row
     dev, dense, qs = paged_setup(lens, [1] * rows, H, KV, hd, bs, torch.bfloat16)
     ref = attention_reference(qs, dense, lens, [1] * rows, window)
     monkeypatch.setattr(attention, "plan_decode_ranges", lambda *a: ranges)
@@ -938,17 +958,20 @@ def test_decode_attention_ranges(ops, monkeypatch, lens, H, KV, hd, bs, window, 
     assert torch.allclose(out.float().cpu(), ref, atol=2e-2, rtol=2e-2), float((out.float().cpu() - ref).abs().max())
 
 
-@pytest.mark.parametrize("lens,q_lens,ranges", [
-    ([900, 1200, 64, 700, 2100, 33], [2, 300, 1, 8, 1, 1], 11),       # short rows of one to eight tokens around a portion
-    ([70 + i for i in range(140)] + [400], [1] * 140 + [64], 29),     # more rows than a round of the scan, beside a portion
+@pytest.mark.parametrize("lens,q_lens,ranges,by_row", [
+    ([900, 1200, 64, 700, 2100, 33], [2, 300, 1, 8, 1, 1], 11, False),  # short rows of one to eight tokens around a portion
+    ([900, 1200, 64, 700, 2100, 33], [2, 300, 1, 8, 1, 1], 40, True),
+    ([70 + i for i in range(140)] + [400], [1] * 140 + [64], 29, False),  # more rows than a round of the scan, beside a portion
 ])  # fmt: skip
+@pytest.mark.parametrize("H", [10, 40])
 @pytest.mark.parametrize("known", [True, False])
-def test_decode_attention_ranges_in_mixed_steps(ops, monkeypatch, lens, q_lens, ranges, known):
+def test_decode_attention_ranges_in_mixed_steps(ops, monkeypatch, lens, q_lens, ranges, by_row, H, known):
     """The same beside prompt portions, whose rows the decode kernel leaves alone, with and without host knowledge of
-    what each request brings."""
+    what each request brings (without it all rows of the step are more than one round of the scan)."""
     import atomserve_b200.ops.attention as attention
 
-    dev, dense, qs = paged_setup(lens, q_lens, 10, 2, 128, 16, torch.bfloat16)
+    assert ranges_end_with_rows(tiles_of(lens, q_lens, None), ranges) == by_row
+    dev, dense, qs = paged_setup(lens, q_lens, H, 2, 128, 16, torch.bfloat16)
     ref = attention_reference(qs, dense, lens, q_lens, None)
     monkeypatch.setattr(attention, "plan_decode_ranges", lambda *a: ranges)
     out = ops.paged_attention(**dev, num_requests=len(lens), max_context=max(lens), window=None, scale=128**-0.5,
@@ -1044,15 +1067,16 @@ def test_portions_launch_without_tiles_keeps_the_order_of_kernels(ops, monkeypat
     ([1200, 300], [200, 100], 16, 1, 150),          # a window: parts in which a row sees nothing
 ])  # fmt: skip
 @pytest.mark.parametrize("parts", [1, 2, 4])
-@pytest.mark.parametrize("with_sink", [False, True])
-def test_prefill_attention_tcgen05_in_parts(ops, monkeypatch, lens, q_lens, H, KV, window, parts, with_sink):
+@pytest.mark.parametrize("with_sink,chunk,softcap", [(False, None, None), (True, None, None), (False, 256, None), (True, 333, 2.0)])
+def test_prefill_attention_tcgen05_in_parts(ops, monkeypatch, lens, q_lens, H, KV, window, parts, with_sink, chunk, softcap):
     """Prompt portions whose key tiles are divided among the blocks of a cluster, against the general kernel in float32."""
     import atomserve_b200.ops.attention as attention
     from atomserve_b200.ops.linear import check_gemm_status
 
     dev, dense, qs = paged_setup(lens, q_lens, H, KV, 128, 16, torch.bfloat16)
     sink = torch.linspace(-2, 3, H, device="cuda") if with_sink else None
-    common = dict(num_requests=len(lens), max_context=max(lens), window=window, scale=128**-0.5, host_q_lens=q_lens, sink=sink)
+    common = dict(num_requests=len(lens), max_context=max(lens), window=window, scale=128**-0.5, host_q_lens=q_lens, sink=sink,
+                  chunk=chunk, softcap=softcap)  # fmt: skip
     wide = {k: (v.float() if v.dtype == torch.bfloat16 else v) for k, v in dev.items()}
     ref = ops.paged_attention(**wide, **common, generic=True)
     monkeypatch.setattr(attention, "plan_portion_parts", lambda *a: parts)
