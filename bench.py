@@ -357,14 +357,16 @@ def time_gemms(which: str, tokens: list[int], steps: int) -> None:
         del ws
 
 
-def attention_partition_sweep(batches: list[int], contexts: list[int]) -> None:
-    """Device time of the decode attention kernel plus its partition merge for every number of key
-    partitions, per (batch, context), at the 8B shape's heads; one JSON line each, with the plan
-    that the engine's planner picks. CUDA-graph loop, microseconds."""
+def attention_range_sweep(batches: list[int], contexts: list[int]) -> None:
+    """Device time of the decode attention kernel plus its merge against the number of ranges that all rows' keys are cut
+    into (0: whole rows, no merge), per (batch, context), at the 8B shape's heads; one JSON line each, with what the
+    engine's planner picks. CUDA-graph loop, microseconds."""
+    from unittest import mock
+
     import torch
 
     from atomserve_b200 import ops
-    from atomserve_b200.ops.attention import plan_decode_partitions
+    from atomserve_b200.ops import attention
 
     c = QWEN3_8B
     H, KV, hd, bs = c["num_attention_heads"], c["num_key_value_heads"], c["head_dim"], BLOCK_SIZE
@@ -381,16 +383,12 @@ def attention_partition_sweep(batches: list[int], contexts: list[int]) -> None:
             q_start = torch.arange(B + 1, dtype=torch.int32, device="cuda")
             pos = torch.full((B,), ctx - 1, dtype=torch.int32, device="cuda")
             times = {}
-            for want in range(1, 33):
-                size = max(256, -(-(-(-ctx // want)) // 64) * 64)
-                parts = (ctx - 1) // size + 1
-                if parts in times:
-                    continue
-                plan = (size, parts) if parts > 1 else (1 << 30, 1)
-
+            planned = attention.plan_decode_ranges(B, KV, H // KV, ctx, 0, hd)
+            for ranges in sorted({0, 4, 8, 16, 24, 32, 40, 48, 55, 64, 74, 110, planned}):
                 def run():
-                    return ops.paged_attention(q, k, v, tables, q_start, pos, num_requests=B, max_context=ctx, window=None,
-                                               scale=hd**-0.5, partitions=plan, host_q_lens=[1] * B)  # fmt: skip
+                    with mock.patch.object(attention, "plan_decode_ranges", return_value=ranges):
+                        return ops.paged_attention(q, k, v, tables, q_start, pos, num_requests=B, max_context=ctx, window=None,
+                                                   scale=hd**-0.5, host_q_lens=[1] * B, earlier_keys_stored=True)  # fmt: skip
 
                 run()
                 torch.cuda.synchronize()
@@ -405,11 +403,10 @@ def attention_partition_sweep(batches: list[int], contexts: list[int]) -> None:
                 graph.replay()
                 end.record()
                 torch.cuda.synchronize()
-                times[parts] = round(start.elapsed_time(end) * 100, 1)
-            planned = plan_decode_partitions(B, KV, H // KV, ctx, 0, hd)
+                times[ranges] = round(start.elapsed_time(end) * 100, 1)
             print(json.dumps({"attention": "decode", "batch": B, "context": ctx,
                               "ideal_us": round(B * ctx * KV * hd * 2 * 2 / 7.3e12 * 1e6, 1),
-                              "planned_parts": planned[1], "us_by_parts": times}))  # fmt: skip
+                              "planned_ranges": planned, "us_by_ranges": times}))  # fmt: skip
             del k, v
 
 
@@ -1450,7 +1447,7 @@ def main() -> int:
     require_device()
     pk = peaks()
     if args.only == "attention":
-        attention_partition_sweep([4, 8, 16, 32, 64, 128], [2048, 8192])
+        attention_range_sweep([1, 4, 8, 16, 32, 64, 128], [512, 2048, 8192])
         return 0
     if args.only == "sampling":
         time_sampling([1, 8, 64], SHAPES[args.shape]["vocab_size"])
