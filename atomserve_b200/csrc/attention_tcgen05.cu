@@ -436,7 +436,6 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
 #pragma unroll 1
       for (int c = 0; c < HD; c += 32) {
         uint32_t raw[32];
-        __syncwarp();  // the read takes the whole warp, and padding rows come from the store's branch early
         tmem_ld32(tmem_o + lane_addr + (uint32_t)c, raw);
         if (real) {
           uint4 v[4];

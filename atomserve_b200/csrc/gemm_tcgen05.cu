@@ -344,7 +344,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
         if (q0 + c >= p.q_rows) break;  // uniform: depends on the segment and c only
         uint32_t raw[kChunk];
         const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + buf * C::kAccCols + (uint32_t)c;
-        __syncwarp();  // the read takes the whole warp, and lanes beyond the matrix come from the store's branch early
         tmem_ld(taddr, raw);
         // the other issuing threads' accumulators, as far as the segment gave them K blocks
 #pragma unroll
