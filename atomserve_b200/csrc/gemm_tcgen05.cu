@@ -620,13 +620,17 @@ int stage_room(int bn_kernel) {
 //     epilogue that writes 64 bytes a token and warp: gate/up at 302 tokens 66.2 us in three rounds, 67.9 without.)
 //   swapped operands with the flattened K-block sequence cut into equal ranges, up to 512 tokens:
 //     the partial sums cost about 14 us, which only long K over few tokens repays (down at 200).
-// With 17 to 64 tokens and more than one round of those pair tiles whose rest can be cut (gate/up), the pair tiles also
-// take the place of the other two forms: gate/up of Qwen3-8B at 32 tokens 44.6 -> 40.8 us, at 64 44.0 -> 42.4 (at 8 tokens
-// 39.3 against 40.8, at 96 44.4 against 46.2).
+// With 17 to 32 tokens and more than one round of those pair tiles whose rest can be cut (gate/up), the pair tiles also
+// take the place of the swapped single-SM form: gate/up of Qwen3-8B at 32 tokens 41.9 -> 39.2 us, 151,936 rows of 2,048 110.3
+// -> 101.0 (at 16 tokens nothing is gained). With 33 to 64 tokens they do so only for the activated form (`glu`), whose
+// epilogue the narrow unswapped tiles take longer over, from 5/4 rounds of tiles and 4,096 elements of K on: 24,576 rows
+// of 4,096 at 48 tokens 42.0 -> 40.2 us (a step of Qwen3-8B with 64 requests 6,660 -> 6,525), 32,768 of 5,120 60.0 -> 57.3.
+// Below, the unswapped tiles are narrower still (20,480 of 4,096 at 64: 37.4 against 40.2 us; 24,576 of 2,048: 25.7, 28.0), and without
+// the activation they win throughout (20,480 of 4,096: 33.0 against 36.3; 24,576: 36.7 against 39.5).
 // With swapped operands, whole tiles are dealt round-robin unless cutting the flattened K-block
 // sequence into equal ranges shortens the busiest SM's share of the operand stream by more than
 // the partial sums cost to write and read back; unswapped single-SM tiles are never cut.
-Plan make_plan(int M, int N, int K) {
+Plan make_plan(int M, int N, int K, bool glu) {
   Plan pl;
   const int sms_now = sm_count();
   const int unswapped_tiles = ((M + BM - 1) / BM) * ((N + 255) / 256);
@@ -645,7 +649,8 @@ Plan make_plan(int M, int N, int K) {
       if (cost < best) { best = cost; pl.bn = bn; pl.bn_kernel = bn <= 128 ? 128 : 256; }
     }
   }
-  if (M > 16 && M <= 64 && g_force_swap < 0 && (N + 255) / 256 > sms_now / 2) {
+  const int wide_tiles = (N + 255) / 256, all_pairs = sms_now / 2;
+  if (M > 16 && g_force_swap < 0 && (M <= 32 ? wide_tiles > all_pairs : M <= 64 && glu && 4 * wide_tiles >= 5 * all_pairs && K >= 4096)) {
     int cut[3];
     const int bn = M <= 32 ? 32 : 64;
     if (asb_gemm_tcgen05_pair_swapped_cut(M, N, K, bn, cut) > 0) pl.wide = bn;
@@ -779,21 +784,22 @@ extern "C" int asb_gemm_tcgen05_pair_swapped(void* out, const void* x, const voi
                                              int K, int mode, int bn, float* workspace, int* status,
                                              const float* glu_bias, int glu_act, cudaStream_t stream);
 
-// Float32 workspace elements a call needs (0 when every tile is computed whole).
+// Float32 workspace elements a call of any mode needs (0 when every tile is computed whole).
 extern "C" long long asb_gemm_tcgen05_workspace(int M, int N, int K, int* stream_out) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  const Plan pl = make_plan(M, N, K);
+  const Plan pl = make_plan(M, N, K, false);
+  const long long activated = make_plan(M, N, K, true).workspace;
   if (stream_out) *stream_out = pl.stream;
-  return pl.workspace;
+  return pl.workspace > activated ? pl.workspace : activated;
 }
 
 // Whether a call runs on pairs of SMs with swapped operands: tiles of 256 weight rows by out4[0] tokens (0: not that form),
 // of which out4[1] run whole, and each of the others in out4[2] pieces of out4[3] stages (two K blocks).
-// Returns its workspace's float32 elements, which asb_gemm_tcgen05_workspace tells too.
-extern "C" long long asb_gemm_tcgen05_wide_plan(int M, int N, int K, int* out4) {
+// Returns its workspace's float32 elements. glu: for mode 2 of asb_gemm_tcgen05, else for the others.
+extern "C" long long asb_gemm_tcgen05_wide_plan(int M, int N, int K, int glu, int* out4) {
   out4[0] = out4[1] = out4[2] = out4[3] = 0;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  const Plan pl = make_plan(M, N, K);
+  const Plan pl = make_plan(M, N, K, glu != 0);
   if (!pl.wide) return 0;
   out4[0] = pl.wide;
   return asb_gemm_tcgen05_pair_swapped_cut(M, N, K, pl.wide, out4 + 1);
@@ -815,10 +821,10 @@ extern "C" void asb_gemm_tcgen05_tune(int swap, int bn) { g_force_swap = swap; g
 // tiles is cut along K, asb_gemm_tcgen05_pair_cut tells. Swapped operands on pairs of SMs (whole tiles of
 // 256 weight rows) are told apart by asb_gemm_tcgen05_wide_plan. A shape that cuts K with
 // swapped operands can leave its product as partial sums (mode 3 of asb_gemm_tcgen05), which
-// csrc/gemm_partials.cuh describes.
+// csrc/gemm_partials.cuh describes. (Mode 2 with 33 to 64 tokens may run as asb_gemm_tcgen05_wide_plan tells for it.)
 extern "C" int asb_gemm_tcgen05_plan(int M, int N, int K, int* out8) {
   if (M <= 0 || N <= 0 || K <= 0) return asb::fail("gemm_tcgen05_plan: empty shape");
-  const Plan pl = make_plan(M, N, K);
+  const Plan pl = make_plan(M, N, K, false);
   out8[0] = pl.stream; out8[1] = pl.swap; out8[2] = pl.max_slots; out8[3] = pl.bn;
   out8[4] = pl.kb_per_tile; out8[5] = pl.tiles_p * pl.tiles_q; out8[6] = pl.blocks;
   out8[7] = pl.pair;
@@ -854,7 +860,7 @@ static int gemm_tcgen05_run(void* out, const void* x, const void* w, const void*
   if (((uintptr_t)x & 15) || ((uintptr_t)w & 15)) return asb::fail("gemm_tcgen05: operands must be 16-byte aligned");
   if (out_f32 && residual) return asb::fail("gemm_tcgen05: the float32 result form takes no residual");
   if (!status) return asb::fail("gemm_tcgen05: a status word is required");
-  const Plan pl = make_plan(M, N, K);
+  const Plan pl = make_plan(M, N, K, mode == 2);
   if (mode == 3 && !(pl.stream && pl.swap && pl.tiles_q == 1))
     return asb::fail("gemm_tcgen05: [%d, %d] x [%d, %d] does not run with partial sums", M, K, N, K);
   if (pl.wide)

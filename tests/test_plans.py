@@ -122,10 +122,10 @@ def test_gemm_plans_keep_every_tile_within_its_partial_sum_slots():
     pair_cut.argtypes, pair_cut.restype = [ctypes.c_int] * 4 + [ctypes.POINTER(ctypes.c_int)], ctypes.c_longlong
     workspace.argtypes, workspace.restype = [ctypes.c_int] * 3 + [ctypes.POINTER(ctypes.c_int)], ctypes.c_longlong
     wide_plan, wide_cut = lib().asb_gemm_tcgen05_wide_plan, lib().asb_gemm_tcgen05_pair_swapped_cut
-    wide_plan.argtypes, wide_plan.restype = [ctypes.c_int] * 3 + [ctypes.POINTER(ctypes.c_int)], ctypes.c_longlong
+    wide_plan.argtypes, wide_plan.restype = [ctypes.c_int] * 4 + [ctypes.POINTER(ctypes.c_int)], ctypes.c_longlong
     wide_cut.argtypes, wide_cut.restype = [ctypes.c_int] * 4 + [ctypes.POINTER(ctypes.c_int)], ctypes.c_longlong
     out, cut, wide = (ctypes.c_int * 8)(), (ctypes.c_int * 3)(), (ctypes.c_int * 4)()
-    cut_plans = wide_plans = wide_cut_plans = 0
+    cut_plans = wide_plans = wide_cut_plans = only_wide = 0
     rng = random.Random(1)
     shapes = [(8, 4096, 4096), (1, 151936, 4096), (512, 4096, 12288), (2048, 24576, 4096), (300, 5120, 17408)]
     for _ in range(3000):
@@ -136,9 +136,18 @@ def test_gemm_plans_keep_every_tile_within_its_partial_sum_slots():
         plan(M, N, K, out)
         cuts_k, swap, max_slots, bn, kb, tiles, blocks, pair = list(out)
         assert kb == -(-K // 64) and 1 <= blocks <= 148, (M, N, K)
-        floats = wide_plan(M, N, K, wide)
+        activated = wide_plan(M, N, K, 1, wide)  # the form of a product with an activation may be another
+        if wide[0]:
+            tokens, whole, split, piece = list(wide)
+            left = -(-N // 256) * -(-M // tokens) - whole
+            slot = 256 * next(s for s in (64, 128, 192, 256) if s >= tokens)
+            assert activated == (left * split * slot if split > 1 else 0) <= workspace(M, N, K, None), (M, N, K)
+            assert left * split <= 74 and (split - 1) * piece < -(-kb // 2) <= split * piece, (M, N, K)
+        only_activated = wide[0]
+        floats = wide_plan(M, N, K, 0, wide)
         if wide[0]:  # tiles of 256 weight rows by wide[0] tokens, a pair of SMs on each; the plan and the workspace are this form's
             wide_plans += 1
+            assert only_activated == wide[0]
             tokens, whole, split, piece = list(wide)
             stages = -(-kb // 2)
             assert tokens % 32 == 0 and 32 <= tokens <= 256 and bn == tokens and swap and not cuts_k and not pair and not max_slots, (M, N, K)
@@ -154,7 +163,8 @@ def test_gemm_plans_keep_every_tile_within_its_partial_sum_slots():
                 assert (split - 1) * piece < stages <= split * piece, (M, N, K)
                 assert blocks == 2 * (74 if whole else tiles * split), (M, N, K)
             continue
-        assert floats == 0
+        assert floats == 0 and (not only_activated or 32 < M <= 64)
+        only_wide += only_activated > 0
         if pair:  # tiles of 256 tokens by `pair` weight rows, two blocks (a pair of SMs) on each
             assert pair in (128, 160, 192, 224, 256) and bn == pair and not swap and not cuts_k and M > 128, (M, N, K)
             assert tiles == -(-M // 256) * -(-N // pair), (M, N, K)
@@ -191,7 +201,7 @@ def test_gemm_plans_keep_every_tile_within_its_partial_sum_slots():
             first = bisect.bisect_right(begins, tile * kb) - 1
             last = bisect.bisect_right(begins, tile * kb + kb - 1) - 1
             assert last - first + 1 <= max_slots, (M, N, K, tile)
-    assert cut_plans > 20 and wide_plans > 50 and wide_cut_plans > 20
+    assert cut_plans > 20 and wide_plans > 50 and wide_cut_plans > 20 and only_wide > 10
 
 
 def test_decode_graph_keys_are_few_and_the_cache_of_graphs_is_bounded():
