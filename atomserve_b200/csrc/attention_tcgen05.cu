@@ -94,6 +94,9 @@ __device__ __forceinline__ float fast_exp2(float x) {
   return y;
 }
 
+// Shared: a tile's keys are divided among `parts` blocks. (In one kernel for both, tiles of one block took 2 to 5 % longer:
+// 512 tokens, 32 heads over 8, 12.8 -> 13.5 us, 2,048 47.4 -> 49.3.)
+template <bool Shared>
 __global__ void __launch_bounds__(kThreads, 2)
 prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                                  const __grid_constant__ CUtensorMap map_v, const AttnParams p) {
@@ -128,7 +131,8 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
   // numbers, so every kv head's block of a request's last tile (the one that sees the most keys)
   // starts before any block of an earlier tile. (Numbered tile fastest, the long blocks of the
   // last kv heads started when half the kernel's time had passed: 64.8 us at 2,048 tokens.)
-  const int unit = blockIdx.x / p.parts, part = blockIdx.x - unit * p.parts;
+  const int parts = Shared ? p.parts : 1;
+  const int unit = blockIdx.x / parts, part = blockIdx.x - unit * parts;
   int tile = unit / p.KV, r = 0, q_len = 0;
   for (; r < p.R; ++r) {
     q_len = p.req_q_start[r + 1] - p.req_q_start[r];
@@ -155,9 +159,9 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
   if (p.chunk > 0) key_lo = max(key_lo, pos0 - pos0 % p.chunk);
   const int key_hi = pos0 + nq;  // exclusive
   const int all_tiles = (key_hi - (key_lo / kKeys) * kKeys + kKeys - 1) / kKeys;
-  const int first_tile = all_tiles * part / p.parts;  // this block's share of the key tiles: none, if there are fewer than parts
+  const int first_tile = all_tiles * part / parts;  // this block's share of the key tiles: none, if there are fewer than parts
   const int kt_begin = (key_lo / kKeys + first_tile) * kKeys;
-  const int num_tiles = all_tiles * (part + 1) / p.parts - first_tile;
+  const int num_tiles = all_tiles * (part + 1) / parts - first_tile;
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
@@ -196,7 +200,7 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
     // The whole warp looks up the pages of a key tile (one page per lane, the loads in flight
     // together); lane 0 waits for the stage, and the lanes issue the tile's TMA loads together.
     const bool keys = warp == 0;
-    if (keys && lane == 0 && num_tiles > 0) {
+    if (keys && lane == 0 && (!Shared || num_tiles > 0)) {
       // the box is QT tokens by G heads: 128 rows when G divides 128, fewer otherwise (the rows
       // after them are padding: never real, masked out, stored nowhere)
       mbar_expect_tx(q_full, (uint32_t)(2 * p.QT * p.G * 128));
@@ -257,7 +261,7 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
         umma_commit(s_full(j & 1));
         umma_commit(k_empty(s));  // the keys' stage, once this product has read it
       };
-      bool ok = num_tiles > 0 && mbar_wait(q_full, 0, p.status, 12);
+      bool ok = (!Shared || num_tiles > 0) && mbar_wait(q_full, 0, p.status, 12);
       if (ok) ok = mbar_wait(k_full(0), 0, p.status, 13);
       if (ok) {
         fence_after_sync();
@@ -407,12 +411,12 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
       if (lane == 0) mbar_arrive(p_full(j & 1));
     }
     // epilogue: O / sum, rounded once
-    if (ok && num_tiles > 0) {
+    if (ok && (!Shared || num_tiles > 0)) {
       int ok_i = 1;
       if (lane == 0) ok_i = mbar_wait(pv_done((num_tiles - 1) & 1), ((uint32_t)(num_tiles - 1) >> 1) & 1u, p.status, 18) ? 1 : 0;
       ok = __shfl_sync(0xffffffffu, ok_i, 0) != 0;
     }
-    if (p.parts > 1) {
+    if constexpr (Shared) {
       // This part's O, column by column, and (max, sum), over the queries and keys, which have been read. A part
       // without key tiles leaves a sum of zero.
       if (num_tiles > 0 && ok) {
@@ -456,7 +460,7 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
     fence_after_sync();
     tmem_dealloc(tmem_base, kTmemCols);
   }
-  if (p.parts > 1) {
+  if constexpr (Shared) {
     const cg::cluster_group cluster = cg::this_cluster();
     cluster.sync();
     if (warp >= 2 && warp < 6) {
@@ -466,7 +470,7 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
 #pragma unroll
       for (int s = 0; s < kMaxParts; ++s) {
         ml[s] = make_float2(-INFINITY, 0.f);
-        if (s < p.parts) ml[s] = reinterpret_cast<const float2*>(cluster.map_shared_rank(smem_raw + kPartBytes, s))[row];
+        if (s < parts) ml[s] = reinterpret_cast<const float2*>(cluster.map_shared_rank(smem_raw + kPartBytes, s))[row];
         if (ml[s].y != 0.f) m = fmaxf(m, ml[s].x);  // (a sum of zero: no key seen there; one that is NaN counts)
       }
       if (qi < nq) {
@@ -479,7 +483,7 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
         }
         if (p.sink) l += exp2f(p.sink[head] * 1.4426950408889634f - m);
         const float inv = 1.f / l;
-        const int columns = HD / p.parts, c0 = part * columns;
+        const int columns = HD / parts, c0 = part * columns;
         __nv_bfloat16* to = p.out + ((size_t)(row0 + qi) * p.H + head) * HD;
 #pragma unroll 1
         for (int c = c0; c < c0 + columns; c += 8) {
@@ -562,7 +566,7 @@ extern "C" int asb_prefill_attention_tcgen05_masked(void* out, const void* q, co
     if (int rc = make_bf16_map(&mk, k_cache, 2, dims, strides, box)) return rc;
     if (int rc = make_bf16_map(&mv, v_cache, 2, dims, strides, box)) return rc;
   }
-  auto kern = prefill_attention_tcgen05_kernel;
+  auto kern = parts == 1 ? prefill_attention_tcgen05_kernel<false> : prefill_attention_tcgen05_kernel<true>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
   if (e != cudaSuccess) return asb::fail("prefill_attention_tcgen05: shared memory %d: %s", kSmem, cudaGetErrorString(e));
   const long long blocks = (long long)((num_tokens + p.QT - 1) / p.QT + R) * KV * parts;
