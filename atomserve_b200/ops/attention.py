@@ -145,13 +145,6 @@ def plan_portion_parts(q_lens: list[int] | None, num_kv_heads: int, group: int, 
     return _portion_parts(sum(-(-n // tokens) for n in q_lens if n > SHORT_ROWS) * num_kv_heads, tiles)
 
 
-def portions_context(q_lens: list[int] | None, pos_start: list[int] | None, max_context: int) -> int:
-    """The longest context of the requests that bring portions (single tokens beside them may have longer ones)."""
-    if q_lens is None or pos_start is None:
-        return max_context
-    return max((p + n for p, n in zip(pos_start, q_lens, strict=True) if n > SHORT_ROWS), default=max_context)
-
-
 @functools.lru_cache(maxsize=4096)
 def _portion_parts(blocks: int, tiles: int) -> int:
     def cost(parts):
@@ -183,7 +176,7 @@ def paged_attention(
     softcap: float | None = None,
     keep_first: int = 0,
     earlier_keys_stored: bool = False,
-    host_pos_start: list[int] | None = None,
+    portions_context: int | None = None,
 ) -> torch.Tensor:
     """softmax(q k^T * scale) v for every new token, keys read in place from the pages.
 
@@ -210,8 +203,8 @@ def paged_attention(
 
     bfloat16 with head size 64 or 128 runs the tensor-core kernels (decode kernel for requests
     that bring at most 8 tokens, prefill kernel for longer portions; `host_q_lens`, the tokens
-    each request brings, tells which are needed, and with `host_pos_start`, where each begins, a
-    portion's blocks are planned for the portions' own contexts; heads with a vector per key head have kernels of
+    each request brings, tells which are needed; `portions_context`, as max_context but of the
+    requests that bring portions, is what these are planned for; heads with a vector per key head have kernels of
     their own); everything else, and `generic=True`, runs the
     general CUDA-core kernel.
     """
@@ -242,7 +235,7 @@ def paged_attention(
     if q.dtype == torch.bfloat16 and not generic and not summed and not keep and lib().asb_attention_mma_supported(hd, H // KV):
         return _paged_attention_mma(q, out, k_cache, v_cache, block_tables, req_q_start, req_pos_start,
                                     num_requests, max_context, win, scale, partitions, host_q_lens, sink, chunk, softcap, span,
-                                    earlier_keys_stored, host_pos_start)  # fmt: skip
+                                    earlier_keys_stored, portions_context)  # fmt: skip
     if q.dtype == torch.bfloat16 and not generic and summed and not chunk and not softcap and sink is None and lib().asb_attention_parts_supported(hd, H, KV):
         return _paged_attention_parts(q, out, k_cache, v_cache, block_tables, req_q_start, req_pos_start, num_requests, max_context,
                                       win, keep, scale, partitions, host_q_lens, earlier_keys_stored)  # fmt: skip
@@ -261,7 +254,7 @@ def paged_attention(
 
 def _paged_attention_mma(q, out, k_cache, v_cache, block_tables, req_q_start, req_pos_start, num_requests,
                          max_context, win, scale, partitions, host_q_lens, sink=None, chunk=0, softcap=0.0, span=None, earlier_keys_stored=False,
-                         host_pos_start=None):  # fmt: skip
+                         portions_context=None):  # fmt: skip
     span = win if span is None else span  # what bounds the keys of a row, for the planner
     T, H, hd = q.shape
     KV, bs = k_cache.shape[1], k_cache.shape[2]
@@ -293,7 +286,7 @@ def _paged_attention_mma(q, out, k_cache, v_cache, block_tables, req_q_start, re
     if has_long and PREFILL_KERNEL == "tcgen05" and lib().asb_attention_tcgen05_supported(hd, H // KV, bs):
         from atomserve_b200.ops.linear import gemm_status
 
-        parts = plan_portion_parts(host_q_lens, KV, H // KV, portions_context(host_q_lens, host_pos_start, max_context), span)
+        parts = plan_portion_parts(host_q_lens, KV, H // KV, portions_context or max_context, span)
 
         def portions():
             check(lib().asb_prefill_attention_tcgen05_masked(

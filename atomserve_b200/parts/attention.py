@@ -227,7 +227,7 @@ class GQAttention(Mixer):
             q, cache.k, cache.v, cache.block_tables, ctx.req_q_start, ctx.req_pos_start,
             num_requests=ctx.num_requests, max_context=ctx.max_context, window=self.window,
             scale=self.scale, host_q_lens=ctx.host_q_lens or None, sink=self.sink, chunk=self.chunk, softcap=self.softcap,
-            earlier_keys_stored=ctx.earlier_keys_stored, host_pos_start=ctx.host_pos_start or None,
+            earlier_keys_stored=ctx.earlier_keys_stored, portions_context=ctx.portions_context(),
         )  # fmt: skip
         return out.view(-1, self.num_heads * self.head_dim)
 

@@ -122,6 +122,9 @@ class CacheView:
 # ---- the step's batch as parts see it -------------------------------------------------------
 
 
+PORTION_TOKENS = 8  # a request that brings more is a portion to the attention kernels
+
+
 @dataclass
 class StepContext:
     """One step's flat batch: T new tokens of R requests, each request's tokens contiguous.
@@ -147,6 +150,15 @@ class StepContext:
     # what a part works out once per step for all layers of its kind (a cut of the step's requests
     # into segments, say), under a name of the part's choosing
     plans: dict[str, Any] = field(default_factory=dict)
+
+    def portions_context(self) -> int:
+        """The longest context of the requests that bring more than a few tokens (single tokens beside them may have longer
+        ones), worked out once per step; the longest of all where none does or the host does not know."""
+        known = self.plans.get("portions_context")
+        if known is None:
+            ends = (p + n for p, n in zip(self.host_pos_start, self.host_q_lens) if n > PORTION_TOKENS)
+            known = self.plans["portions_context"] = max(ends, default=self.max_context)
+        return known
 
 
 # ---- interfaces -----------------------------------------------------------------------------

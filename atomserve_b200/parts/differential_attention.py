@@ -83,7 +83,7 @@ class DifferentialAttention(Mixer):
             q, cache.k, cache.v, cache.block_tables, ctx.req_q_start, ctx.req_pos_start,
             num_requests=ctx.num_requests, max_context=ctx.max_context, window=self.window, scale=self.scale,
             host_q_lens=ctx.host_q_lens or None, chunk=self.chunk, earlier_keys_stored=ctx.earlier_keys_stored,
-            host_pos_start=ctx.host_pos_start or None,
+            portions_context=ctx.portions_context(),
         )  # fmt: skip
         return ops.differential_combine(maps, self.value_dim, self.lam, 1.0 - self.diff, self.eps)
 

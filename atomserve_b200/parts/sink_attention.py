@@ -63,7 +63,7 @@ class SinkAttention(Mixer):
         out = ops.paged_attention(q, cache.k, cache.v, cache.block_tables, ctx.req_q_start, ctx.req_pos_start,
                                   num_requests=ctx.num_requests, max_context=ctx.max_context, window=self.window,
                                   scale=self.scale, host_q_lens=ctx.host_q_lens or None, sink=self.sink,
-                                  earlier_keys_stored=ctx.earlier_keys_stored, host_pos_start=ctx.host_pos_start or None)  # fmt: skip
+                                  earlier_keys_stored=ctx.earlier_keys_stored, portions_context=ctx.portions_context())  # fmt: skip
         return ops.head_norm_gate(out.view(-1, qw), proj[:, col + qw + kw : col + 2 * qw + kw], 1)
 
     def forward_from(self, proj: torch.Tensor, col: int, ctx: StepContext, cache: CacheView, write_cache: bool = True) -> torch.Tensor:

@@ -86,11 +86,19 @@ def test_decode_attention_ranges_fill_the_device_and_their_scratch(monkeypatch):
 def test_portions_are_planned_for_their_own_contexts():
     """A short prompt beside one long decode is not divided for the decode's context; without the positions the step's
     longest context stands in, and one part is the answer where the lengths are not told at all."""
-    from atomserve_b200.ops.attention import plan_portion_parts, portions_context
+    from atomserve_b200.ops.attention import SHORT_ROWS, plan_portion_parts
+    from atomserve_b200.parts.base import PORTION_TOKENS, StepContext
+
+    def portions_context(q_lens, starts, longest):
+        ctx = StepContext(1, 1, *[None] * 6, max_context=longest, host_q_lens=q_lens, host_pos_start=starts)
+        assert ctx.portions_context() == ctx.portions_context()
+        return ctx.portions_context()
+
+    assert PORTION_TOKENS == SHORT_ROWS
 
     assert portions_context([40, 1], [0, 12000], 12001) == 40
     assert portions_context([40, 1, 200], [5000, 12000, 100], 12001) == 5040
-    assert portions_context([40, 1], None, 12001) == portions_context(None, None, 12001) == 12001
+    assert portions_context([8, 1], [0, 12000], 12001) == portions_context([], [], 12001) == 12001
     assert plan_portion_parts([40, 1], 8, 4, portions_context([40, 1], [0, 12000], 12001), 0) == 1
     assert plan_portion_parts(None, 8, 4, 12001, 0) == 1
     for lens in ([512], [100], [9], [300, 200, 64], [2048]):
