@@ -59,6 +59,28 @@ inline void launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
   cudaLaunchKernelEx(&config, kernel, std::forward<Args>(args)...);
 }
 
+// The same for a kernel whose blocks wait for one another: the launch is refused unless all of them fit the device at
+// once, and none of them starts before there is room for all.
+template <typename... KArgs, typename... Args>
+inline int launch_cooperative(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+  cudaLaunchConfig_t config = {};
+  config.gridDim = grid;
+  config.blockDim = block;
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  cudaLaunchAttribute attribute[2];
+  attribute[0].id = cudaLaunchAttributeCooperative;
+  attribute[0].val.cooperative = 1;
+  attribute[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attribute[1].val.programmaticStreamSerializationAllowed = 1;
+  config.attrs = attribute;
+  config.numAttrs = pdl_enabled() ? 2 : 1;
+  prefer_shared_carveout((const void*)kernel);
+  count_launch();
+  const cudaError_t error = cudaLaunchKernelEx(&config, kernel, std::forward<Args>(args)...);
+  return error == cudaSuccess ? 0 : fail("cooperative launch: %s", cudaGetErrorString(error));
+}
+
 // Among the rows of the requests that bring at most `limit` tokens, counted in request order,
 // the flat row of number `index` (its request in *request); -1 if there are fewer such rows.
 __device__ __forceinline__ int nth_short_row(const int* req_q_start, int R, int limit, int index, int* request) {

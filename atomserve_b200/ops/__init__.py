@@ -3,6 +3,7 @@ and launches on the current stream. float32 tensors run the true 32-bit kernels,
 tensors the serving kernels; nothing here computes on the CPU."""
 
 from atomserve_b200.ops.attention import attention_tile_shape, paged_attention
+from atomserve_b200.ops.chain import decode_chain, decode_chain_takes
 from atomserve_b200.ops.delta import delta_rule, plan_delta
 from atomserve_b200.ops.elementwise import (
     embedding,
@@ -40,6 +41,7 @@ __all__ = [
     "cast_rows", "clamped_glu", "combine", "embedding_scaled", "experts_down", "experts_glu", "gated_rms_norm", "gelu",
     "group_by_expert", "linear_for_stream", "head_matmul", "head_matmul_on_tensor_cores", "latent_attention", "latent_prepare", "lightning_attention", "plan_segments", "route",
     "scaled_add_rms_norm",
+    "decode_chain", "decode_chain_takes",
     "DeviceStatus",
     "KernelLibraryError",
     "PartialSums",

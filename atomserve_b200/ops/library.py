@@ -74,6 +74,10 @@ _SIGNATURES = {
     "asb_partial_add_normed": [_P, _P, _P, _I, _I, _I, _I, _I, _P, _P, _P, _P, _I, _I, _F, _F, _P],
     "asb_bias_glu": [_P, _P, _P, _I, _I, _I, _I, _P],
     "asb_softcap": [_P, ctypes.c_longlong, _F, _P],
+    # the projections between one layer's attention and the next one's in one kernel
+    "asb_decode_chain": [_P] * 5 + [_F] + [_P] * 5 + [_F] + [_P] * 4 + [_I] * 5 + [_P, _P],
+    "asb_decode_chain_blocks": [],
+    "asb_decode_chain_limits": [_P, _P],
     # attention with a sink in the softmax's denominator
     "asb_paged_attention_sink": [_P] * 11 + [_I] * 10 + [_F, _I, _P],
     "asb_prefill_attention_tcgen05_sink": [_P] * 8 + [_I] * 9 + [_F, _P, _P],

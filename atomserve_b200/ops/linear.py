@@ -37,6 +37,12 @@ def gemm_simt(x: torch.Tensor, w: torch.Tensor, residual: torch.Tensor | None, o
 # unaligned operands) go to the library either way.
 BACKEND = os.environ.get("ATOMSERVE_B200_GEMM", "tcgen05")
 
+
+def own_kernels() -> bool:
+    """Whether bfloat16 products run this package's kernels."""
+    return BACKEND == "tcgen05"
+
+
 def gemm_status(device: torch.device) -> torch.Tensor:
     """The device word a tcgen05 kernel sets if one of its pipeline waits runs out."""
     return status_for(device).pipeline

@@ -16,6 +16,7 @@ import torch
 PIPELINE, EMBEDDING = 0, 1
 _ROLES = {
     1: "GEMM: operand loads", 2: "GEMM: MMA issue", 3: "GEMM: epilogue", 4: "GEMM: accumulator hand-back",
+    31: "decode chain: free stage", 32: "decode chain: weights", 33: "decode chain: grid barrier",
 }  # fmt: skip
 
 
@@ -24,7 +25,7 @@ def describe(words: list[int]) -> str | None:
     if words[PIPELINE]:
         code = words[PIPELINE]
         who = _ROLES.get(code, f"prefill attention, wait {code}" if 10 <= code <= 29 else ("the self-test" if code == 90 else f"wait {code}"))
-        parts.append(f"a tcgen05 kernel gave up a bounded wait ({who}); its output is incomplete")
+        parts.append(f"a kernel gave up a bounded wait ({who}); its output is incomplete")
     if words[EMBEDDING]:
         parts.append("the embedding met a token id outside the vocabulary")
     return "; ".join(parts) or None

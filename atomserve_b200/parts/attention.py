@@ -18,7 +18,7 @@ from __future__ import annotations
 import torch
 
 from atomserve_b200 import ops
-from atomserve_b200.parts.base import CacheView, KVCacheSpec, Mixer, Norm, PageSpec, StepContext, build_part, register_part
+from atomserve_b200.parts.base import CacheView, KVCacheSpec, Mixer, Norm, PageSpec, ProjectedInput, StepContext, build_part, register_part
 from atomserve_b200.parts.spec import PartSpec, TensorSpec
 
 
@@ -165,6 +165,19 @@ class GQAttention(Mixer):
             raise NotImplementedError("attention beside another mixer norms its queries over the whole projection")
         return self.qkv_proj
 
+    def input_projection(self, write_cache: bool) -> torch.Tensor | None:
+        """The weight of the product that `attend` begins with, for a kernel that runs it at the end of the layer before and
+        hands on a `ProjectedInput`; None where `attend` does not take one."""
+        rotary = self.position.fused_rotary() if self.position is not None else None
+        if self.norm_over == "projection" or self.query_temperature is not None or (self.position is not None and rotary is None):
+            return None
+        # reading another entry's keys and values, only queries are projected
+        return self.qkv_proj if write_cache else self.qkv_proj[: self.num_heads * self.head_dim]
+
+    def output_projection(self) -> torch.Tensor:
+        """The weight of the product that follows `attend`, for a kernel that runs it with what comes next."""
+        return self.o_proj
+
     def forward_from(self, proj: torch.Tensor, col: int, ctx: StepContext, cache: CacheView, write_cache: bool = True) -> torch.Tensor:
         return ops.linear(self.attend_from(proj, col, ctx, cache, write_cache), self.o_proj, out_dtype=torch.float32, weights_stored=True)
 
@@ -181,7 +194,7 @@ class GQAttention(Mixer):
         )  # fmt: skip
         return self._over_pages(q, ctx, cache)
 
-    def attend(self, h: torch.Tensor, ctx: StepContext, cache: CacheView | None, write_cache: bool) -> torch.Tensor:
+    def attend(self, h: torch.Tensor | ProjectedInput, ctx: StepContext, cache: CacheView | None, write_cache: bool) -> torch.Tensor:
         """The heads' outputs side by side, [T, H * hd], before the output projection."""
         H, KV, hd = self.num_heads, self.num_kv_heads, self.head_dim
         if self.norm_over == "projection":
@@ -207,8 +220,8 @@ class GQAttention(Mixer):
         else:
             # reading another entry's keys and values, only queries are projected
             weight, kv_heads = (self.qkv_proj, KV) if write_cache else (self.qkv_proj[: H * hd], 0)
-            qkv = None
-            if ops.qk_norm_rope_store_takes_partial(hd, rotary.rotary_dim if rotary else None):
+            qkv = h.product if isinstance(h, ProjectedInput) else None
+            if qkv is None and ops.qk_norm_rope_store_takes_partial(hd, rotary.rotary_dim if rotary else None):
                 # with few tokens the product stays as the GEMM's partial sums and the next kernel adds them up
                 qkv = ops.linear_partial(h, weight)
             if qkv is None:

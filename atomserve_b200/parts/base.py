@@ -151,6 +151,10 @@ class StepContext:
     # into segments, say), under a name of the part's choosing
     plans: dict[str, Any] = field(default_factory=dict)
 
+    # the block that runs right after this one, and whether it writes keys and values of its own: None where the run order
+    # ends or something else comes between
+    following: tuple["Block", bool] | None = None
+
     def portions_context(self) -> int:
         """The longest context of the requests that bring more than a few tokens (single tokens beside them may have longer
         ones), worked out once per step; the longest of all where none does or the host does not know."""
@@ -159,6 +163,14 @@ class StepContext:
             ends = (p + n for p, n in zip(self.host_pos_start, self.host_q_lens) if n > PORTION_TOKENS)
             known = self.plans["portions_context"] = max(ends, default=self.max_context)
         return known
+
+
+@dataclass(frozen=True)
+class ProjectedInput:
+    """A mixer's input that has been through the mixer's first projection already (`Mixer.input_projection`), handed on by
+    the block before in the place of the normed input."""
+
+    product: torch.Tensor
 
 
 # ---- interfaces -----------------------------------------------------------------------------

@@ -44,6 +44,11 @@ class SwiGLU(FeedForward):
     def forward(self, h: torch.Tensor, residual: torch.Tensor, ctx: StepContext) -> torch.Tensor:
         return ops.linear(self.hidden(h), self.down_proj, residual, weights_stored=True)
 
+    def gated_weights(self) -> tuple[torch.Tensor, torch.Tensor] | None:
+        """(gate and up rows alternating, down), for a kernel that runs the whole feed-forward; None where the rows do not
+        alternate."""
+        return (self.gate_up_proj, self.down_proj) if self.fused else None
+
     def forward_then(self, h: torch.Tensor, residual: torch.Tensor, ctx: StepContext,
                      then: Norm) -> tuple[torch.Tensor, torch.Tensor]:  # fmt: skip
         after_linear = getattr(then, "after_linear", None)

@@ -110,7 +110,9 @@ class DecoderModel:
                 else:
                     x, normed = step.forward(x, x0, call.before[1], ctx), None
             last = i + 1 == len(self.schedule) or self.schedule[i + 1].before is not None  # (a stream step norms nothing)
-            then = None if last else self.blocks[self.schedule[i + 1].layer].mixer_norm
+            following = None if last else self.blocks[self.schedule[i + 1].layer]
+            then = None if last else following.mixer_norm
+            ctx.following = None if last else (following, self.schedule[i + 1].cache_from is None)
             x, normed = self.blocks[call.layer].forward_chain(
                 x, normed, ctx, views[i if own else call.cache_from], own, then
             )

@@ -14,6 +14,8 @@ class RMSNorm(Norm):
     """`centre`: what the gain is stored less of (1 for a checkpoint that keeps gains around zero); the
     gain the kernels read is made once at load, in float32."""
 
+    plain = True  # `forward` is the norm itself, in x's own dtype: a kernel that knows `gain` and `eps` may stand in for it
+
     def __init__(self, hidden_size: int, prefix: str, eps: float, width: int | None = None, tensor: str | None = None,
                  centre: float = 0.0):  # fmt: skip
         self.width = width or hidden_size
@@ -58,6 +60,8 @@ class StreamRMSNorm(RMSNorm):
     blocks whose norm follows the sum: `add_forward(x, y)` is norm(alpha x + y), returned both as
     the new float32 stream and in the compute dtype (what the next products read); `forward` is
     the plain norm of (rows of) the stream in the compute dtype, as a final norm before the head."""
+
+    plain = False
 
     def __init__(self, hidden_size: int, prefix: str, eps: float, alpha: float = 1.0, width: int | None = None,
                  tensor: str | None = None, centre: float = 0.0):  # fmt: skip

@@ -1,0 +1,87 @@
+"""The projections from one layer's attention to the next one's as one kernel, against plain products with the same
+roundings."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _inputs(tokens, hidden, attn_k, ff, next_rows, seed=0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+
+    def normal(*shape, std=1.0):
+        return (torch.randn(*shape, generator=g, device="cuda") * std).bfloat16()
+
+    gains = [1 + 0.1 * torch.randn(hidden, generator=g, device="cuda") for _ in range(2)]
+    return dict(attn=normal(tokens, attn_k), o=normal(hidden, attn_k, std=attn_k**-0.5), x=normal(tokens, hidden), gains=gains,
+                gate=normal(ff, hidden, std=hidden**-0.5), up=normal(ff, hidden, std=hidden**-0.5),
+                down=normal(hidden, ff, std=ff**-0.5), proj=normal(next_rows, hidden, std=hidden**-0.5) if next_rows else None)  # fmt: skip
+
+
+def _normed_product(x, gain, eps, *matrices):
+    """N(x) . w^T in float64: the operand is x times the gain rounded to bfloat16, the norm's factor multiplies the sums."""
+    d = torch.float64
+    factor = torch.rsqrt((x.to(d) ** 2).mean(-1, keepdim=True) + eps)
+    operand = (x.float() * gain).bfloat16().to(d)
+    return [factor * (operand @ w.to(d).T) for w in matrices]
+
+
+def _plain(v, eps):
+    """Every stored value rounded to bfloat16 once, all else in float64."""
+    d = torch.float64
+    x1 = (v["attn"].to(d) @ v["o"].to(d).T + v["x"].to(d)).bfloat16()
+    gate, up = _normed_product(x1, v["gains"][0], eps, v["gate"], v["up"])
+    act = (torch.nn.functional.silu(gate) * up).bfloat16()
+    x2 = (act.to(d) @ v["down"].to(d).T + x1.to(d)).bfloat16()
+    return x2, (_normed_product(x2, v["gains"][1], eps, v["proj"])[0].bfloat16() if v["proj"] is not None else None)
+
+
+def _close(got, want):
+    # A stored value may be the neighbour of the plain one where the sum lies at a rounding boundary (float32 sums against
+    # float64: one element in a few thousand); each such step of 2^-8 in x1 or the gated values moves the products behind it
+    # by far less than their own rounding, 2^-9 of a value at most: 4e-3 of the norm holds both, with room for neither wrong
+    # rows, nor wrong tokens, nor a product left out.
+    got, want = got.double(), want.double()
+    assert torch.isfinite(got).all()
+    assert (got - want).norm() <= 4e-3 * want.norm()
+    assert (got - want).abs().max() <= 2**-6 * want.abs().max()
+
+
+# rows a block: fewer than blocks, a part of a row tile, one tile and a part, several passes; K of one step and of several
+@pytest.mark.parametrize("hidden,attn_k,ff,next_rows", [
+    (512, 512, 512, 130), (1024, 2048, 1536, 1536), (4096, 4096, 12288, 6144), (5120, 8192, 25600, 10240), (2048, 512, 6144, 0),
+])  # fmt: skip
+@pytest.mark.parametrize("tokens", [1, 2, 3, 7, 8])
+def test_against_plain_products(hidden, attn_k, ff, next_rows, tokens):
+    from atomserve_b200 import ops
+    from atomserve_b200.ops.linear import check_gemm_status
+
+    v = _inputs(tokens, hidden, attn_k, ff, next_rows, seed=tokens)
+    gate_up = ops.interleave_gate_up(v["gate"], v["up"])
+    assert ops.decode_chain_takes(v["x"], v["o"], gate_up, v["down"])
+    want = _plain(v, 1e-6)
+    for _ in range(2):  # (what a call leaves behind is not met by the next)
+        got = ops.decode_chain(v["attn"], v["o"], v["x"], v["gains"][0], 1e-6, gate_up, v["down"], torch.zeros(4, dtype=torch.int32, device="cuda"),
+                               next_gain=v["gains"][1], next_eps=1e-6, next_proj=v["proj"])  # fmt: skip
+        check_gemm_status()
+        _close(got[0], want[0])
+        assert (got[1] is None) == (next_rows == 0)
+        if next_rows:
+            _close(got[1], want[1])
+
+
+def test_a_row_does_not_depend_on_the_others():
+    from atomserve_b200 import ops
+
+    v = _inputs(8, 1024, 2048, 1536, 1536)
+    gate_up = ops.interleave_gate_up(v["gate"], v["up"])
+
+    def run(rows):
+        return ops.decode_chain(v["attn"][rows].contiguous(), v["o"], v["x"][rows].contiguous(), v["gains"][0], 1e-6, gate_up, v["down"],
+                                torch.zeros(4, dtype=torch.int32, device="cuda"), v["gains"][1], 1e-6, v["proj"])  # fmt: skip
+
+    whole = run(slice(0, 8))
+    for rows in (slice(0, 1), slice(2, 5), slice(7, 8)):
+        for part, all_rows in zip(run(rows), whole):
+            assert torch.equal(part, all_rows[rows])
