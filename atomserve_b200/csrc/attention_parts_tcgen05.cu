@@ -205,7 +205,7 @@ parts_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __
     }
   } else if (warp == 1) {
     // S = Q K^T, a tile ahead of the softmax
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_qk = instr_desc_bf16(kRows, kKeys, false);
       bool ok = kStreamQ || mbar_wait(q_full, 0, p.status, 12);
       const int total = num_tiles * p.KV;
@@ -234,7 +234,7 @@ parts_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __
     }
   } else if (warp == 6) {
     // O += P V as soon as the softmax has written a tile's P
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_pv = instr_desc_bf16(kRows, HD, true);
       bool ok = true;
       Ring ring;

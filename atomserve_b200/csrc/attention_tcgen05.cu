@@ -247,7 +247,7 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
   } else if (warp == 1) {
     // Q K^T, one tile ahead of the softmax. (Issuing a tcgen05.mma takes its thread 60-80 cycles
     // whatever its shape, so the two products have a thread each: warp 6 issues P V.)
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_qk = instr_desc_bf16(kRows, kKeys, false);
       auto issue_qk = [&](int j) {
         const int s = j % kKStages;
@@ -279,7 +279,7 @@ prefill_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
     }
   } else if (warp == 6) {
     // O += P V as soon as the softmax has written a tile's P
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_pv = instr_desc_bf16(kRows, HD, true);
       bool ok = true;
       for (int j = 0; j < num_tiles && ok; ++j) {

@@ -227,7 +227,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
 
   constexpr int kFirstExtraLoader = 6 + C::kIssuers - 1;  // warps 0 and kFirstExtraLoader.. load
   if (warp == 0 || warp >= kFirstExtraLoader) {
-    if (lane == 0) {
+    if (asb::t5::elect_one()) {
       // Loader `me` of kLoaders brings every kLoaders-th K block of the block's sequence. The
       // weights are operand P when swapped, Q otherwise. Before waiting for the previous kernel,
       // the first `stages` stages are filled with the weight half; the activation half follows.
@@ -278,7 +278,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
     }
   } else if (warp == 1 || (warp >= 6 && warp < kFirstExtraLoader)) {
     asb::pdl_wait();
-    if (lane == 0) {
+    if (asb::t5::elect_one()) {
       const int me = warp == 1 ? 0 : warp - 5;  // which of the kIssuers issuing threads
       const uint32_t idesc = instr_desc(BM, bn);
       SegmentWalk walk(p);

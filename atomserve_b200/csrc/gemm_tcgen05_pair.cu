@@ -190,7 +190,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   auto item_len = [&](int i) { return i < n_whole ? stages_per_tile : (i < n_items ? piece_len : 0x3fffffff); };
 
   if (warp == 0 || warp >= 6) {
-    if (lane == 0 && (warp == 0 ? 0 : warp - 5) < C::kLoaders) {  // a spare loader warp has nothing to do
+    if ((warp == 0 ? 0 : warp - 5) < C::kLoaders && elect_one()) {  // a spare loader warp has nothing to do
       // Loader `me` of kLoaders (warps 0, 6, 7, ...) brings every kLoaders-th stage: this CTA's 128
       // token rows and its half of the weight rows; the bytes are counted in the even CTA. One
       // thread's chain of wait, announcement and requests takes about 700 cycles per stage,
@@ -270,7 +270,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     }
   } else if (warp == 1) {
     asb::pdl_wait();
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       const uint32_t idesc = instr_desc_bf16(256, p.bn, false);
       int s = 0;
       uint32_t phase = 0;

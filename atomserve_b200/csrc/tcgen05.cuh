@@ -60,6 +60,20 @@ __device__ __forceinline__ uint32_t mbar_try(uint32_t bar, uint32_t parity) {
   return done;
 }
 
+// True in one lane of the (whole, converged) warp. A role that issues tcgen05.mma or TMA from one thread begins with this and
+// not with a lane's number: the instructions take warp-uniform operands, and here the compiler knows that one lane runs. With
+// a branch on the lane the products bound by their issuing thread took longer: o [4096, 4096] on pairs at 512 tokens 18.3
+// -> 16.5 us, down [4096, 12288] 45.9 -> 42.7, gate/up [51200, 5120] at 302 172.6 -> 158.9; the others stay as they were.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t elected;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(elected));
+  return elected != 0;
+}
+
 // TMA tile loads (no multicast). Coordinates are element offsets, innermost first; the innermost
 // must be a multiple of 16 bytes.
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
