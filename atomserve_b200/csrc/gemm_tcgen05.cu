@@ -630,6 +630,42 @@ int stage_room(int bn_kernel) {
 // With swapped operands, whole tiles are dealt round-robin unless cutting the flattened K-block
 // sequence into equal ranges shortens the busiest SM's share of the operand stream by more than
 // the partial sums cost to write and read back; unswapped single-SM tiles are never cut.
+// What a product with the activated epilogue takes in a form, in microseconds, as fitted to the calls of a sweep of every
+// form and width (gate/up of 12,288 to 51,200 rows, the other projections with an epilogue of their own, 136 to 2,048
+// tokens; off by 7 % in the mean): a start, the busiest SM's K blocks, what each round's epilogue adds, and where the last
+// round is cut along K its reduction and sums; no less than the weights' bytes and 9 us. `swapped`: tiles of 256 weight rows
+// by bn tokens on pairs of SMs; else `pair`: of 256 tokens by bn weight rows on pairs, or of 128 tokens on single SMs.
+double activated_us(bool swapped, bool pair, int bn, int M, int N, int K) {
+  static const double kPerBlock[3][7] = {  // by width: 64, 96, .., 256
+      {0.1890, 0.2076, 0.2294, 0.2712, 0.2937, 0.3127, 0.3873},
+      {0.1956, 0.1956, 0.1956, 0.2574, 0.2864, 0.3189, 0.3580},
+      {0.1352, 0.1686, 0.1918, 0.2221, 0.2546, 0.2994, 0.3366}};
+  static const double kStart[3] = {5.26, 5.62, 5.74}, kEpilogue[3] = {1.23, 0.83, 3.73};  // (the latter a round of 128 columns)
+  const int form = swapped ? 2 : (pair ? 1 : 0);
+  const double kb = (K + BK - 1) / BK;
+  double blocks, rounds, more = 0.0;
+  if (form == 0) {
+    rounds = (double)((((M + BM - 1) / BM) * ((N + bn - 1) / bn) + sm_count() - 1) / sm_count());
+    blocks = rounds * kb;
+  } else {
+    const int pairs = sm_count() / 2;
+    int cut[3];
+    const long long floats = swapped ? asb_gemm_tcgen05_pair_swapped_cut(M, N, K, bn, cut) : asb_gemm_tcgen05_pair_cut(M, N, K, bn, cut);
+    const int tiles = swapped ? ((N + 255) / 256) * ((M + bn - 1) / bn) : ((M + 255) / 256) * ((N + bn - 1) / bn);
+    if (floats > 0) {
+      rounds = cut[0] / pairs + 1;
+      blocks = (cut[0] / pairs) * kb + 2.0 * cut[2];
+      more = (swapped ? 3.45 : 3.17) + (swapped ? 0.51 : 1.66) * (double)(tiles - cut[0]) * cut[1] * 256 * bn / 1e6;
+    } else {
+      rounds = (tiles + pairs - 1) / pairs;
+      blocks = rounds * kb;
+    }
+  }
+  const double us = kStart[form] + kPerBlock[form][(bn - 64) / 32] * blocks + kEpilogue[form] * rounds * bn / 128.0 + more;
+  const double memory = 9.0 + (double)N * K * 2 / 6.5e6;
+  return us > memory ? us : memory;
+}
+
 Plan make_plan(int M, int N, int K, bool glu) {
   Plan pl;
   const int sms_now = sm_count();
@@ -697,6 +733,19 @@ Plan make_plan(int M, int N, int K, bool glu) {
       const double share = (double)((N + BM - 1) / BM) * ((M + 255) / 256) * kb / sms_now;  // K blocks per SM
       const double cost = 14.0 + (share < 4 ? 4 : share) * 0.457;
       if (cost < best) { best = cost; pl.swap = 1; pl.pair = pl.wide = 0; pl.bn = pl.bn_kernel = 256; }
+    }
+  }
+  // Matrices of more than a round of weight tiles (gate/up): swapped pair tiles of several rounds too, where they save 5 % by the finer estimate: gate/up
+  // of Qwen3-14B at 302 tokens 112.3 -> 96.8 us, of 32B at 136 105.8 -> 97.0; whole steps at 280 and 302 tokens of 14B 1.05 and
+  // 1.07 times as fast, at 136 of 32B 1.03, and no size between 136 and 350 tokens of 8B, 14B and 32B slower. (Not with fewer
+  // rows: o, down and qkv at 256 to 1,000 tokens won up to 15 % call by call and lost up to 5 % in whole steps, as
+  // a product with a residual reads and writes 64 bytes a token and warp in this form; and at 400 tokens gate/up of
+  // 32B won 6 % alone and nothing in a step.)
+  if (M > BM && M <= kWideTokens && wide_tiles > all_pairs && !pl.swap && g_force_swap < 0) {
+    double best = 0.95 * activated_us(pl.wide > 0, pl.pair > 0, pl.wide ? pl.wide : (pl.pair ? pl.pair : pl.bn), M, N, K);
+    for (int bn = 64; bn <= 256; bn += 32) {
+      const double us = activated_us(true, false, bn, M, N, K);
+      if (us < best) { best = us; pl.pair = 0; pl.wide = bn; }
     }
   }
   if (g_force_swap >= 0) {  // the tuning aid's choice

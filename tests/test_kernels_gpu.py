@@ -709,7 +709,8 @@ def test_prefill_attention_tcgen05(ops, case):
 
 
 @pytest.mark.parametrize("M,I,K", [(1, 64, 64), (5, 200, 72), (16, 1024, 512), (40, 352, 256), (64, 12288, 4096),
-                                   (100, 176, 80), (300, 704, 256), (2048, 512, 512)])  # fmt: skip
+                                   (100, 176, 80), (300, 704, 256), (2048, 512, 512),
+                                   (130, 25600, 5120), (302, 17408, 5120), (281, 17410, 5128)])  # fmt: skip
 def test_gemm_tcgen05_swiglu(ops, M, I, K):
     """silu(x gate^T) * (x up^T) from the GEMM's own epilogue (and, where K is cut, from the
     reduction of its partial sums) against float64."""
