@@ -395,7 +395,8 @@ __global__ void __launch_bounds__(kThreads, 1) decode_chain_kernel(const __grid_
     load_matrices(c, s, ring, warp - kWarps, lane);  // weights: no kernel writes them, so nothing is waited for
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
-    for (int p = 0; p < c.phases; ++p)  // the gains are on their way into L2 before their first product
+    // the gains are on their way into L2 before their first product, which reads every line of them
+    for (int p = 0; p < c.phases; ++p)
       if (c.phase[p].gain)
         for (int i = threadIdx.x * 32; i < c.phase[p].k; i += kWarps * 32 * 32)
           asm volatile("prefetch.global.L2 [%0];" ::"l"(c.phase[p].gain + i));
