@@ -586,6 +586,31 @@ def test_sampled_token_wins_the_plain_race(ops, V, k, p, temp):
         assert score[out[r]] >= score[kept].max() * (1 - 1e-5)
 
 
+@pytest.mark.parametrize("V", [2, 1024, 1025, 4099, 32000])
+@pytest.mark.parametrize("spread,k,p,temp", [(0.0, 0, 0.5, 1.0), (1e-6, 0, 0.9, 0.8), (1e-3, 1500, 0.3, 1.0), (3.0, 0, 0.5, 50.0),
+                                             (3.0, 0, 0.99, 0.02), (30.0, 0, 0.9, 1.0)])  # fmt: skip
+def test_the_cut_of_top_p_wherever_the_mass_lies(ops, V, spread, k, p, temp):
+    """The steps below the largest logit in which the walk over masses begins: all logits in one step (as many as the buffer
+    of candidates holds, and one more), steps of a few neighbouring floats, nearly all mass in the first or far down."""
+    g = torch.Generator().manual_seed(V + k)
+    logits = (torch.randn(2, V, generator=g) * spread + 7).float()
+    seeds, counters = [5, (1 << 40) + 3], [0, 9]
+    out = ops.sample_rows(
+        logits.cuda(), torch.full((2,), temp, device="cuda"), torch.full((2,), k, dtype=torch.int32, device="cuda"),
+        torch.full((2,), p, device="cuda"), torch.tensor(seeds, device="cuda"), torch.tensor(counters, device="cuda"),
+    ).tolist()  # fmt: skip
+    for r in range(2):
+        x = logits[r].double().numpy()
+        order = np.lexsort((np.arange(V), -x))[: k if 0 < k < V else V]
+        mass = np.exp((x[order] - x[order[0]]) / np.float64(np.float32(temp)))
+        before, p32 = np.cumsum(mass) - mass, np.float64(np.float32(p))
+        # float32 masses (a few units of 2^-24 each) may keep one token more or fewer at the cut
+        kept, edge = order[before < p32 * mass.sum() * (1 - 1e-6)], order[before < p32 * mass.sum() * (1 + 1e-6)]
+        score = np.exp((x - x.max()) / np.float64(np.float32(temp))) / np.maximum(-np.log(philox_uniforms(seeds[r], counters[r], V)), 1e-10)
+        assert out[r] in edge
+        assert score[out[r]] >= score[kept].max() * (1 - 1e-5)
+
+
 @pytest.mark.parametrize("V", [5, 500, 4099, 50001, 151936])
 @pytest.mark.parametrize("k,p,temp", [(20, 0.95, 0.6), (0, 0.95, 0.8), (2000, 0.9, 1.0), (0, 1.0, 1.0), (3, 1.0, 1.0), (0, 1.0, 0.0)])
 def test_a_rows_token_does_not_depend_on_how_many_rows_there_are(ops, V, k, p, temp):
