@@ -150,7 +150,7 @@ __device__ void load_matrices(const Chain& c, Shared& s, uint32_t ring, int load
         for (int r = r0; r < r1; r += kTileRows) {
           if (turn == loader) {
             const uint32_t full = smem_u32(&s.full[stage]);
-            wait_or_give_up(s, smem_u32(&s.empty[stage]), (round & 1) ^ 1, c.status, 31);
+            wait_or_give_up(s, smem_u32(&s.empty[stage]), (round & 1) ^ 1, c.status, 41);
             if (__any_sync(0xffffffffu, given_up(s))) return;
             const int n = min(kTileRows, r1 - r);
             if (lane == 0) mbar_expect_tx(full, (uint32_t)n * kStepK * 2);
@@ -263,7 +263,7 @@ __device__ void multiply_phase(const Chain& c, const Phase& ph, Shared& s, uint3
 #pragma unroll
       for (int m = 0; m < kMaxTiles; ++m) {
         if (m >= tiles) break;
-        wait_or_give_up(s, smem_u32(&s.full[walk.stage]), walk.parity, c.status, 32);
+        wait_or_give_up(s, smem_u32(&s.full[walk.stage]), walk.parity, c.status, 42);
         const uint32_t at = ring + walk.stage * kStageBytes + lane_at;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -367,7 +367,7 @@ __device__ void grid_barrier(const Chain& c, Shared& s, int index, int tid) {
       done = seen >= gridDim.x;
     }
     if (!done && !given_up(s)) {
-      atomicExch(c.status, 33);
+      atomicExch(c.status, 43);
       *(volatile int*)&s.dead = 1;
     }
   }

@@ -1,7 +1,7 @@
 """The device's status words: how a kernel tells the host that it could not finish its work.
 
-Kernels here never trap and never spin without end. A wait in a tcgen05 kernel that runs out of
-polls writes which role gave up into word 0 and lets its block wind down (tensor memory freed,
+Kernels here never trap and never spin without end. A wait in a kernel that runs out of
+polls writes which role gave up into word 0 (each kernel has codes of its own) and lets its block wind down (tensor memory freed,
 output incomplete); the embedding gather writes 1 into word 1 when it meets a token id outside
 the table. There is one set of words per device. The serving path copies them to pinned host
 memory behind each step's kernels (`send_to_host`, no wait of its own) and looks at the copy once
@@ -14,9 +14,11 @@ from __future__ import annotations
 import torch
 
 PIPELINE, EMBEDDING = 0, 1
-_ROLES = {
+_ROLES = {  # 10 to 29: prefill attention; 90: the self-test
     1: "GEMM: operand loads", 2: "GEMM: MMA issue", 3: "GEMM: epilogue", 4: "GEMM: accumulator hand-back",
-    31: "decode chain: free stage", 32: "decode chain: weights", 33: "decode chain: grid barrier",
+    31: "GEMM on pairs of SMs: free stage", 32: "GEMM on pairs of SMs: operands", 33: "GEMM on pairs of SMs: accumulator",
+    34: "GEMM on pairs of SMs: accumulator hand-back", 38: "GEMM on pairs of SMs: last stages",
+    41: "decode chain: free stage", 42: "decode chain: weights", 43: "decode chain: grid barrier",
 }  # fmt: skip
 
 
