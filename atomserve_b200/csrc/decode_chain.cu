@@ -22,7 +22,7 @@
 // multiplies by the norm's factor of the token, rounds and stores them.
 //
 // The norms' sums of squares: every block leaves its rows' share per token, and all blocks add up the shares of all
-// blocks in one order, so that each token's factor is the same everywhere.
+// blocks in one order, so that each token's factor is the same everywhere, and the same for any number of tokens.
 //
 // Measured in a CUDA graph of such layers, 1 and 8 tokens, in us, as separate kernels and as one, beside the matrices' time
 // at 6,546 GB/s: Qwen3-8B's sizes 80.3, 82.5 -> 70.9, 73.7 (59.0); 14B's 120.3, 123.3 -> 107.1, 110.7 (100.9); 32B's 165.9,
@@ -217,7 +217,9 @@ template <int NT>
 __device__ void multiply_phase(const Chain& c, const Phase& ph, Shared& s, uint32_t ring, float* sums, Walk& walk, float4 (&gains)[2][2],
                                int warp, int lane) {
   const int T = c.tokens, tid = warp * 32 + lane;
-  int columns = 1;  // tokens to a power of two: how the epilogue's threads divide
+  // Tokens to a power of two: how the epilogue's threads divide. Where they add up squares, always the most tokens there are:
+  // the order of a token's sum is then the same whatever else is in the step (and a block has few rows there: 14 to 18 pairs).
+  int columns = ph.epilogue == kResidual ? kMaxTokens : 1;
   while (columns < T) columns *= 2;
   constexpr int TP = NT * 8;                                      // token columns
   constexpr int kGroup = kSumFloats / (kWarps * kTileRows * TP);  // row tiles whose sums meet at once

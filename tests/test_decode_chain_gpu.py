@@ -71,17 +71,32 @@ def test_against_plain_products(hidden, attn_k, ff, next_rows, tokens):
             _close(got[1], want[1])
 
 
-def test_a_row_does_not_depend_on_the_others():
+# 2 to 18 pairs of rows a block in the sums of squares: one thread a pair, several threads and several warps of a token. (The
+# sums are read too: a factor that differs in its last bit changes one bfloat16 value in some ten thousand.)
+@pytest.mark.parametrize("hidden", [512, 1024, 4096, 5120])
+def test_a_row_does_not_depend_on_the_others(hidden):
+    from atomserve_b200.ops.library import check, lib, ptr, stream
+    from atomserve_b200.ops.linear import check_gemm_status, gemm_status
     from atomserve_b200 import ops
 
-    v = _inputs(8, 1024, 2048, 1536, 1536)
+    attn_k, ff, next_rows = 2048, 1536, 1536
+    v = _inputs(8, hidden, attn_k, ff, next_rows)
     gate_up = ops.interleave_gate_up(v["gate"], v["up"])
+    blocks = lib().asb_decode_chain_blocks()
 
     def run(rows):
-        return ops.decode_chain(v["attn"][rows].contiguous(), v["o"], v["x"][rows].contiguous(), v["gains"][0], 1e-6, gate_up, v["down"],
-                                torch.zeros(4, dtype=torch.int32, device="cuda"), v["gains"][1], 1e-6, v["proj"])  # fmt: skip
+        attn, x = v["attn"][rows].contiguous(), v["x"][rows].contiguous()
+        T = x.shape[0]
+        x1, x2, act, out = (torch.empty(T, n, device="cuda", dtype=torch.bfloat16) for n in (hidden, hidden, ff, next_rows))
+        squares, arrived = torch.empty(2, T, blocks, device="cuda"), torch.zeros(4, dtype=torch.int32, device="cuda")
+        check(lib().asb_decode_chain(
+            ptr(attn), ptr(v["o"]), ptr(x), ptr(x1), ptr(v["gains"][0]), 1e-6, ptr(gate_up), ptr(act), ptr(v["down"]), ptr(x2),
+            ptr(v["gains"][1]), 1e-6, ptr(v["proj"]), ptr(out), ptr(squares), ptr(arrived), T, hidden, attn_k, ff, next_rows,
+            ptr(gemm_status(x.device)), stream()))  # fmt: skip
+        check_gemm_status()
+        return x1, act, x2, out, squares[0], squares[1]
 
     whole = run(slice(0, 8))
-    for rows in (slice(0, 1), slice(2, 5), slice(7, 8)):
+    for rows in (slice(0, 1), slice(7, 8), slice(2, 4), slice(2, 5), slice(1, 5), slice(3, 8)):
         for part, all_rows in zip(run(rows), whole):
             assert torch.equal(part, all_rows[rows])
