@@ -735,13 +735,14 @@ Plan make_plan(int M, int N, int K, bool glu) {
       if (cost < best) { best = cost; pl.swap = 1; pl.pair = pl.wide = 0; pl.bn = pl.bn_kernel = 256; }
     }
   }
-  // Matrices of more than a round of weight tiles (gate/up): swapped pair tiles of several rounds too, where they save 5 % by the finer estimate: gate/up
+  // Activated products of more than a round of weight tiles (gate/up): swapped pair tiles of several rounds too, where they save 5 % by the finer
+  // estimate, which knows this epilogue only (plain and float32 results, as an output head's, were not measured in this form): gate/up
   // of Qwen3-14B at 302 tokens 112.3 -> 96.8 us, of 32B at 136 105.8 -> 97.0; whole steps at 280 and 302 tokens of 14B 1.05 and
   // 1.07 times as fast, at 136 of 32B 1.03, and no size between 136 and 350 tokens of 8B, 14B and 32B slower. (Not with fewer
   // rows: o, down and qkv at 256 to 1,000 tokens won up to 15 % call by call and lost up to 5 % in whole steps, as
   // a product with a residual reads and writes 64 bytes a token and warp in this form; and at 400 tokens gate/up of
   // 32B won 6 % alone and nothing in a step.)
-  if (M > BM && M <= kWideTokens && wide_tiles > all_pairs && !pl.swap && g_force_swap < 0) {
+  if (glu && M > BM && M <= kWideTokens && wide_tiles > all_pairs && !pl.swap && g_force_swap < 0) {
     double best = 0.95 * activated_us(pl.wide > 0, pl.pair > 0, pl.wide ? pl.wide : (pl.pair ? pl.pair : pl.bn), M, N, K);
     for (int bn = 64; bn <= 256; bn += 32) {
       const double us = activated_us(true, false, bn, M, N, K);
@@ -870,7 +871,7 @@ extern "C" void asb_gemm_tcgen05_tune(int swap, int bn) { g_force_swap = swap; g
 // tiles is cut along K, asb_gemm_tcgen05_pair_cut tells. Swapped operands on pairs of SMs (whole tiles of
 // 256 weight rows) are told apart by asb_gemm_tcgen05_wide_plan. A shape that cuts K with
 // swapped operands can leave its product as partial sums (mode 3 of asb_gemm_tcgen05), which
-// csrc/gemm_partials.cuh describes. (Mode 2 with 33 to 64 tokens may run as asb_gemm_tcgen05_wide_plan tells for it.)
+// csrc/gemm_partials.cuh describes. (Mode 2 with 33 to 64 and 129 to 400 tokens may run as asb_gemm_tcgen05_wide_plan tells for it.)
 extern "C" int asb_gemm_tcgen05_plan(int M, int N, int K, int* out8) {
   if (M <= 0 || N <= 0 || K <= 0) return asb::fail("gemm_tcgen05_plan: empty shape");
   const Plan pl = make_plan(M, N, K, false);

@@ -171,7 +171,8 @@ def test_gemm_plans_keep_every_tile_within_its_partial_sum_slots():
                 assert (split - 1) * piece < stages <= split * piece, (M, N, K)
                 assert blocks == 2 * (74 if whole else tiles * split), (M, N, K)
             continue
-        assert floats == 0 and (not only_activated or 32 < M <= 64)
+        # (the activated form alone: at 33 to 64 tokens, and at 129 to 400 with more weight tiles than pairs of SMs)
+        assert floats == 0 and (not only_activated or 32 < M <= 64 or 128 < M <= 400 and N > 256 * 74)
         only_wide += only_activated > 0
         if pair:  # tiles of 256 tokens by `pair` weight rows, two blocks (a pair of SMs) on each
             assert pair in (128, 160, 192, 224, 256) and bn == pair and not swap and not cuts_k and M > 128, (M, N, K)
@@ -182,7 +183,8 @@ def test_gemm_plans_keep_every_tile_within_its_partial_sum_slots():
             whole, split, piece = list(cut)
             stages = -(-kb // 2)
             slot = 256 * (128 if pair == 128 else 256)  # a slot is as wide as the widest tile of the kernel that runs it
-            assert workspace(M, N, K, None) == floats == ((tiles - whole) * split * slot if split > 1 else 0), (M, N, K)
+            assert floats == ((tiles - whole) * split * slot if split > 1 else 0), (M, N, K)
+            assert workspace(M, N, K, None) == max(floats, activated), (M, N, K)  # (the activated form's, where that is another)
             if split == 1:
                 assert whole == tiles and blocks == 2 * min(tiles, 74), (M, N, K)
             else:
@@ -210,6 +212,29 @@ def test_gemm_plans_keep_every_tile_within_its_partial_sum_slots():
             last = bisect.bisect_right(begins, tile * kb + kb - 1) - 1
             assert last - first + 1 <= max_slots, (M, N, K, tile)
     assert cut_plans > 20 and wide_plans > 50 and wide_cut_plans > 20 and only_wide > 10
+
+
+def test_swapped_pair_tiles_of_several_rounds_are_for_activated_products():
+    """Tiles of 256 weight rows on pairs of SMs in several rounds were fitted to and measured on the activated epilogue: at
+    129 to 400 tokens an output head, or any product without an activation, keeps the forms it had."""
+    import ctypes
+
+    try:
+        from atomserve_b200.ops.library import lib
+
+        wide_plan = lib().asb_gemm_tcgen05_wide_plan
+    except Exception as error:  # no compiler here, or the library does not load without a driver
+        pytest.skip(f"the kernel library is not available: {error}")
+    wide_plan.argtypes, wide_plan.restype = [ctypes.c_int] * 4 + [ctypes.POINTER(ctypes.c_int)], ctypes.c_longlong
+    wide, activated = (ctypes.c_int * 4)(), 0
+    for rows in (18_945, 24_576, 34_816, 51_200, 151_936):
+        for hidden in (1024, 4096, 5120):
+            for tokens in range(129, 401, 7):
+                wide_plan(tokens, rows, hidden, 0, wide)
+                assert wide[0] == 0, (tokens, rows, hidden)
+                wide_plan(tokens, rows, hidden, 1, wide)
+                activated += wide[0] > 0
+    assert activated > 50
 
 
 def test_decode_graph_keys_are_few_and_the_cache_of_graphs_is_bounded():
