@@ -15,6 +15,7 @@ neighbours, and a preempted request that is recomputed draws the same tokens aga
 from __future__ import annotations
 
 import os
+from array import array
 
 import numpy as np
 import torch
@@ -33,6 +34,15 @@ class Picked:
 
     def __init__(self, device_ids: torch.Tensor, host_ids: torch.Tensor, arrived):
         self.device_ids, self.host_ids, self.arrived = device_ids, host_ids, arrived
+
+
+def _numbers(code: str, values: list):
+    """The values as C numbers of `array`'s type code. A number of another kind (20.0 for a count) is converted as torch does,
+    and what is none (None, a text) raises; numpy's own conversion would make a NaN of None and a number of a text."""
+    try:
+        return array(code, values)
+    except TypeError:
+        return torch.tensor(values, dtype={"q": torch.int64, "i": torch.int32, "f": torch.float32}[code]).numpy()
 
 
 class Sampler:
@@ -85,12 +95,12 @@ class Sampler:
             # (filled through numpy: a small tensor a setting, and its copy, took the host 40 us a step)
             host, dev = self._host[turn][: 4 * n], self._dev[: 4 * n]
             words = host.numpy().reshape(4, n)
-            words[0] = [self.seed_of(s) for s in seqs]
-            words[1] = [len(s.token_ids) - s.num_prompt_tokens + ahead for s in seqs]
             floats, ints = words[2].view(np.float32), words[3].view(np.int32)
-            floats[:n] = [s.params.temperature for s in seqs]
-            floats[n:] = [s.params.top_p for s in seqs]
-            ints[:n] = [s.params.top_k for s in seqs]
+            words[0] = _numbers("q", [self.seed_of(s) for s in seqs])
+            words[1] = _numbers("q", [len(s.token_ids) - s.num_prompt_tokens + ahead for s in seqs])
+            floats[:n] = _numbers("f", [s.params.temperature for s in seqs])
+            floats[n:] = _numbers("f", [s.params.top_p for s in seqs])
+            ints[:n] = _numbers("i", [s.params.top_k for s in seqs])
             dev.copy_(host, non_blocking=True)
             dev_floats, dev_ints = dev[2 * n : 3 * n].view(torch.float32), dev[3 * n :].view(torch.int32)
             out = ops.sample_rows(logits, dev_floats[:n], dev_ints[:n], dev_floats[n:], dev[:n], dev[n : 2 * n])
