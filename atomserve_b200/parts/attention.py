@@ -18,7 +18,7 @@ from __future__ import annotations
 import torch
 
 from atomserve_b200 import ops
-from atomserve_b200.parts.base import CacheView, KVCacheSpec, Mixer, Norm, PageSpec, ProjectedInput, StepContext, build_part, register_part
+from atomserve_b200.parts.base import CacheView, KVCacheSpec, Mixer, Norm, PageSpec, ProjectedInput, StepContext, build_part, register_part, runs_own
 from atomserve_b200.parts.spec import PartSpec, TensorSpec
 
 
@@ -167,16 +167,19 @@ class GQAttention(Mixer):
 
     def input_projection(self, write_cache: bool) -> torch.Tensor | None:
         """The weight of the product that `attend` begins with, for a kernel that runs it at the end of the layer before and
-        hands on a `ProjectedInput`; None where `attend` does not take one."""
+        hands on a `ProjectedInput`; None where `attend`, or a derived part, does not take one."""
+        if not runs_own(self, GQAttention, "attend", "forward", "forward_then"):
+            return None
         rotary = self.position.fused_rotary() if self.position is not None else None
         if self.norm_over == "projection" or self.query_temperature is not None or (self.position is not None and rotary is None):
             return None
         # reading another entry's keys and values, only queries are projected
         return self.qkv_proj if write_cache else self.qkv_proj[: self.num_heads * self.head_dim]
 
-    def output_projection(self) -> torch.Tensor:
-        """The weight of the product that follows `attend`, for a kernel that runs it with what comes next."""
-        return self.o_proj
+    def output_projection(self) -> torch.Tensor | None:
+        """The weight of the product that follows `attend`, for a kernel that runs it with what comes next; None where a derived
+        part does something else there."""
+        return self.o_proj if runs_own(self, GQAttention, "forward", "forward_then") else None
 
     def forward_from(self, proj: torch.Tensor, col: int, ctx: StepContext, cache: CacheView, write_cache: bool = True) -> torch.Tensor:
         return ops.linear(self.attend_from(proj, col, ctx, cache, write_cache), self.o_proj, out_dtype=torch.float32, weights_stored=True)

@@ -186,6 +186,12 @@ class Part:
         """Receive the tensors named by tensor_specs (on the device, in their final dtype)."""
 
 
+def runs_own(part: Part, owner: type, *methods: str) -> bool:
+    """Whether `part` runs these methods as `owner` wrote them. A class that offers its weights to a kernel which stands in for
+    its methods does so for itself alone: a part that derives from it and changes one of them is run by what it has."""
+    return all(getattr(type(part), m) is getattr(owner, m) and m not in vars(part) for m in methods)
+
+
 class Norm(Part):
     def forward(self, x: torch.Tensor, rows: torch.Tensor | None = None) -> torch.Tensor:
         raise NotImplementedError

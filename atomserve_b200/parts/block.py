@@ -7,7 +7,7 @@ from __future__ import annotations
 import torch
 
 from atomserve_b200 import ops
-from atomserve_b200.parts.base import Block, CacheView, Norm, ProjectedInput, StepContext, register_part
+from atomserve_b200.parts.base import Block, CacheView, Norm, ProjectedInput, StepContext, register_part, runs_own
 
 
 class PreNormBlock(Block):
@@ -32,16 +32,17 @@ class PreNormBlock(Block):
     def _chained(self, x: torch.Tensor, normed, ctx: StepContext, cache: CacheView | None, write_cache: bool, then: Norm | None):
         """With few tokens: all products from the mixer's last to the following block's first as one kernel
         (`ops.decode_chain`), where both blocks are of the kind it knows. None where it does not run."""
-        output = getattr(self.mixer, "output_projection", None)
+        offered = getattr(self.mixer, "output_projection", None)
         gated = getattr(self.feed_forward, "gated_weights", None)
-        weights = gated() if gated is not None else None
+        output, weights = offered() if offered is not None else None, gated() if gated is not None else None
         if output is None or weights is None or not getattr(self.feed_forward_norm, "plain", False):
             return None
-        if not ops.decode_chain_takes(x, output(), *weights):
+        if not ops.decode_chain_takes(x, output, *weights):
             return None
         proj = None
-        if ctx.following is not None and isinstance(ctx.following[0], PreNormBlock) and getattr(then, "plain", False):
-            first = getattr(ctx.following[0].mixer, "input_projection", None)
+        following = ctx.following[0] if ctx.following is not None else None
+        if isinstance(following, PreNormBlock) and runs_own(following, PreNormBlock, "forward_chain") and getattr(then, "plain", False):
+            first = getattr(following.mixer, "input_projection", None)
             proj = first(ctx.following[1]) if first is not None else None
             if proj is not None and not ops.decode_chain_takes(x, proj):
                 proj = None
@@ -51,7 +52,7 @@ class PreNormBlock(Block):
         ctx.plans["chain_arrivals"] = (counters, used + 1)
         norm = self.feed_forward_norm
         x, product = ops.decode_chain(
-            self.mixer.attend(normed, ctx, cache, write_cache), output(), x, norm.gain, norm.eps, *weights, counters[used],
+            self.mixer.attend(normed, ctx, cache, write_cache), output, x, norm.gain, norm.eps, *weights, counters[used],
             next_gain=then.gain if proj is not None else None, next_eps=then.eps if proj is not None else 0.0, next_proj=proj,
         )  # fmt: skip
         if product is not None:

@@ -6,7 +6,7 @@ from __future__ import annotations
 import torch
 
 from atomserve_b200 import ops
-from atomserve_b200.parts.base import FeedForward, Norm, StepContext, register_part
+from atomserve_b200.parts.base import FeedForward, Norm, StepContext, register_part, runs_own
 from atomserve_b200.parts.spec import TensorSpec
 
 
@@ -46,8 +46,9 @@ class SwiGLU(FeedForward):
 
     def gated_weights(self) -> tuple[torch.Tensor, torch.Tensor] | None:
         """(gate and up rows alternating, down), for a kernel that runs the whole feed-forward; None where the rows do not
-        alternate."""
-        return (self.gate_up_proj, self.down_proj) if self.fused else None
+        alternate or a derived part computes something else."""
+        own = self.fused and runs_own(self, SwiGLU, "hidden", "forward", "forward_then")
+        return (self.gate_up_proj, self.down_proj) if own else None
 
     def forward_then(self, h: torch.Tensor, residual: torch.Tensor, ctx: StepContext,
                      then: Norm) -> tuple[torch.Tensor, torch.Tensor]:  # fmt: skip

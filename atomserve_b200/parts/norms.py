@@ -6,7 +6,7 @@ from __future__ import annotations
 import torch
 
 from atomserve_b200 import ops
-from atomserve_b200.parts.base import Norm, register_part
+from atomserve_b200.parts.base import Norm, register_part, runs_own
 from atomserve_b200.parts.spec import TensorSpec
 
 
@@ -14,14 +14,17 @@ class RMSNorm(Norm):
     """`centre`: what the gain is stored less of (1 for a checkpoint that keeps gains around zero); the
     gain the kernels read is made once at load, in float32."""
 
-    plain = True  # `forward` is the norm itself, in x's own dtype: a kernel that knows `gain` and `eps` may stand in for it
-
     def __init__(self, hidden_size: int, prefix: str, eps: float, width: int | None = None, tensor: str | None = None,
                  centre: float = 0.0):  # fmt: skip
         self.width = width or hidden_size
         self.eps, self.centre = float(eps), float(centre)
         self.name = tensor or prefix + "weight"
         self.gain: torch.Tensor | None = None
+
+    @property
+    def plain(self) -> bool:
+        """Whether `forward` is the norm itself, in x's own dtype: a kernel that knows `gain` and `eps` may stand in for it."""
+        return runs_own(self, RMSNorm, "forward", "after_linear")
 
     def tensor_specs(self) -> list[TensorSpec]:
         return [TensorSpec(self.name, (self.width,), kind="gain", init="normal" if self.centre else "gain")]
@@ -60,8 +63,6 @@ class StreamRMSNorm(RMSNorm):
     blocks whose norm follows the sum: `add_forward(x, y)` is norm(alpha x + y), returned both as
     the new float32 stream and in the compute dtype (what the next products read); `forward` is
     the plain norm of (rows of) the stream in the compute dtype, as a final norm before the head."""
-
-    plain = False
 
     def __init__(self, hidden_size: int, prefix: str, eps: float, alpha: float = 1.0, width: int | None = None,
                  tensor: str | None = None, centre: float = 0.0):  # fmt: skip
