@@ -359,9 +359,19 @@ def build_block(kind: str, mixer: Mixer, feed_forward: FeedForward, mixer_norm: 
     return factory(mixer, feed_forward, mixer_norm, feed_forward_norm)
 
 
+_builtin_loaded = False
+
+
 def _ensure_builtin() -> None:
-    if "rms_norm" not in _REGISTRIES["norm"]:
+    """Register the package's own parts before the first build. Some may be registered already (a program that derives from one
+    has imported its module); a kind that the program has registered itself stays the program's."""
+    global _builtin_loaded
+    if not _builtin_loaded:
+        _builtin_loaded = True
+        registered = {family: dict(kinds) for family, kinds in _REGISTRIES.items()}
         from atomserve_b200.parts import (  # noqa: F401
             attention, block, delta_rule, differential_attention, embedding, experts, latent_attention, lightning, matrix_memory, mixed_heads, mlp,
             norms, parallel, rotary, sink_attention, state_space, stream_step, token_input,
         )
+        for family, kinds in registered.items():
+            _REGISTRIES[family].update(kinds)
