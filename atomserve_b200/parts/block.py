@@ -40,7 +40,8 @@ class PreNormBlock(Block):
         if not ops.decode_chain_takes(x, output, *weights):
             return None
         proj = None
-        following = ctx.following[0] if ctx.following is not None else None
+        # (`following` is of the model's run order: a block inside another one is told another norm than that block's)
+        following = ctx.following[0] if ctx.following is not None and then is ctx.following[0].mixer_norm else None
         if isinstance(following, PreNormBlock) and runs_own(following, PreNormBlock, "forward_chain") and getattr(then, "plain", False):
             first = getattr(following.mixer, "input_projection", None)
             proj = first(ctx.following[1]) if first is not None else None

@@ -165,3 +165,33 @@ def test_a_method_set_on_the_part_itself_is_run(chain, monkeypatch):
         monkeypatch.setattr(block.feed_forward, "hidden", lambda h, inner=inner: seen.append(h.shape) or inner(h))
     _run(model, 4)
     assert len(seen) == 2 and chain.calls == 0
+
+
+class PairOfBlocks(PreNormBlock):
+    """Two pre-norm blocks in the place of one (the second one with the first one's sublayers, over a cache of its own)."""
+
+    def load(self, tensors):
+        super().load(tensors)
+        self.first, self.second = (PreNormBlock(self.mixer, self.feed_forward, self.mixer_norm, self.feed_forward_norm) for _ in range(2))
+        self.second.mixer_norm = ShiftedGain(self.mixer_norm)
+        self.inner = View()
+
+    def forward_chain(self, x, normed, ctx, cache, write_cache, then):
+        x, normed = self.first.forward_chain(x, normed, ctx, cache, write_cache, self.second.mixer_norm)
+        return self.second.forward_chain(x, normed, ctx, self.inner, True, then)
+
+
+class ShiftedGain(RMSNorm):
+    def __init__(self, other):
+        self.gain, self.eps, self.width = other.gain + 1, other.eps, other.width
+
+
+def test_a_block_of_blocks_hands_on_between_its_own(chain, monkeypatch):
+    """What follows a block in the run order is not what follows a block inside it: the norm that a block is told to run next
+    says whose input it hands on."""
+    register_part("block", "pair_of_the_test", PairOfBlocks)
+    model = _model(2, block="pair_of_the_test")
+    model.blocks[1] = model.blocks[1].first
+    plain = _off(monkeypatch, model, 4)
+    assert torch.allclose(_run(model, 4), plain, rtol=1e-12, atol=1e-12)
+    assert chain.calls == 3
