@@ -155,6 +155,18 @@ class StepContext:
     # ends or something else comes between
     following: tuple["Block", bool] | None = None
 
+    # zeroed words of this pass for kernels whose blocks count themselves in, and how many rows of them are taken: None at the
+    # start of every pass, so that a captured pass holds their zeroing whatever ran over this context before
+    counters: tuple[torch.Tensor, int] | None = None
+
+    def zeroed_counters(self, device: torch.device) -> torch.Tensor:
+        """Four int32 zeros on the device for one call of a kernel (zeroed a few dozen calls at a time, in the current stream)."""
+        words, used = self.counters or (None, 0)
+        if words is None or used == len(words):
+            words, used = torch.zeros(64, 4, dtype=torch.int32, device=device), 0
+        self.counters = (words, used + 1)
+        return words[used]
+
     def portions_context(self) -> int:
         """The longest context of the requests that bring more than a few tokens (single tokens beside them may have longer
         ones), worked out once per step; the longest of all where none does or the host does not know."""

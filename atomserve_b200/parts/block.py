@@ -47,13 +47,9 @@ class PreNormBlock(Block):
             proj = first(ctx.following[1]) if first is not None else None
             if proj is not None and not ops.decode_chain_takes(x, proj):
                 proj = None
-        counters, used = ctx.plans.get("chain_arrivals", (None, 0))
-        if counters is None or used == len(counters):  # (zeroed a few dozen layers at a time, in the step's own stream)
-            counters, used = torch.zeros(64, 4, dtype=torch.int32, device=x.device), 0
-        ctx.plans["chain_arrivals"] = (counters, used + 1)
         norm = self.feed_forward_norm
         x, product = ops.decode_chain(
-            self.mixer.attend(normed, ctx, cache, write_cache), output, x, norm.gain, norm.eps, *weights, counters[used],
+            self.mixer.attend(normed, ctx, cache, write_cache), output, x, norm.gain, norm.eps, *weights, ctx.zeroed_counters(x.device),
             next_gain=then.gain if proj is not None else None, next_eps=then.eps if proj is not None else 0.0, next_proj=proj,
         )  # fmt: skip
         if product is not None:

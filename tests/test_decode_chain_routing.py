@@ -195,3 +195,19 @@ def test_a_block_of_blocks_hands_on_between_its_own(chain, monkeypatch):
     plain = _off(monkeypatch, model, 4)
     assert torch.allclose(_run(model, 4), plain, rtol=1e-12, atol=1e-12)
     assert chain.calls == 3
+
+
+@pytest.mark.parametrize("layers", [1, 3, 64, 65, 130])
+def test_every_pass_zeroes_counters_of_its_own(chain, layers):
+    """A pass that is captured into a graph after another one over the same context has to hold the zeroing of all its
+    counters: words that an earlier pass zeroed would be met at their end state by the second replay."""
+    model, ctx = _model(layers), _context(4)
+    words = []
+    for _ in range(2):
+        chain.counters.clear()
+        _run(model, 4, ctx)
+        assert chain.calls == layers
+        chain.calls = 0
+        words.append({c.untyped_storage().data_ptr(): c.untyped_storage() for c in chain.counters})
+        assert len({c.data_ptr() for c in chain.counters}) == layers  # a call's own
+    assert not words[0].keys() & words[1].keys()
