@@ -23,15 +23,17 @@ def chain_limits() -> tuple[int, int]:
     return tokens.value, k_multiple.value
 
 
-def decode_chain_takes(x: torch.Tensor, *matrices: torch.Tensor) -> bool:
-    """Whether `decode_chain` runs for this residual stream and these matrices (the output, gated and down projections, and
-    any that follow)."""
+def decode_chain_takes(x: torch.Tensor, *weights: torch.Tensor) -> bool:
+    """Whether `decode_chain` runs for this residual stream and these weights: matrices (the output, gated and down projections,
+    and any that follow) and norms' gains. Its loads are of 16 bytes; what is laid out otherwise, the separate kernels take."""
     if not CHAIN or not own_kernels() or x.dtype != torch.bfloat16 or not x.is_cuda:
         return False
     tokens, k_multiple = chain_limits()
-    return 0 < x.shape[0] <= tokens and all(
-        w.dtype == torch.bfloat16 and w.dim() == 2 and w.is_contiguous() and w.shape[0] % 2 == 0 and w.shape[1] % k_multiple == 0 and w.data_ptr() % 16 == 0
-        for w in matrices
+    if not 0 < x.shape[0] <= tokens or not all(t.is_contiguous() and t.data_ptr() % 16 == 0 for t in (x, *weights)):
+        return False
+    return all(
+        w.dtype == torch.float32 if w.dim() == 1 else w.dim() == 2 and w.dtype == torch.bfloat16 and w.shape[0] % 2 == 0 and w.shape[1] % k_multiple == 0
+        for w in weights
     )
 
 
@@ -57,13 +59,13 @@ def decode_chain(
     The matrices are read before the stream's previous kernel has completed: they must not be what it writes."""
     require_cuda(attn, o_proj, x, gain, gate_up, down, arrived, next_gain, next_proj)
     T, hidden = x.shape
-    if not decode_chain_takes(x, o_proj, gate_up, down, *([next_proj] if next_proj is not None else [])):
+    if next_proj is not None and (next_proj.shape[1] != hidden or next_gain is None):
+        raise KernelLibraryError("decode_chain: the last product reads the normed stream")
+    if not decode_chain_takes(x, o_proj, gate_up, down, gain, *([next_proj, next_gain] if next_proj is not None else [])):
         raise KernelLibraryError("decode_chain: tokens, types or sizes that the kernel does not take")
     ff = down.shape[1]
     if attn.shape != (T, o_proj.shape[1]) or o_proj.shape[0] != hidden or gate_up.shape != (2 * ff, hidden) or down.shape[0] != hidden:
         raise KernelLibraryError("decode_chain: the matrices' sizes do not follow from one another")
-    if next_proj is not None and (next_proj.shape[1] != hidden or next_gain is None):
-        raise KernelLibraryError("decode_chain: the last product reads the normed stream")
     if attn.dtype != x.dtype or not attn.is_contiguous() or not x.is_contiguous():
         raise KernelLibraryError("decode_chain: attn and x must be contiguous bfloat16")
     for g in (gain, next_gain):

@@ -37,7 +37,7 @@ class PreNormBlock(Block):
         output, weights = offered() if offered is not None else None, gated() if gated is not None else None
         if output is None or weights is None or not getattr(self.feed_forward_norm, "plain", False):
             return None
-        if not ops.decode_chain_takes(x, output, *weights):
+        if not ops.decode_chain_takes(x, output, *weights, self.feed_forward_norm.gain):
             return None
         proj = None
         # (`following` is of the model's run order: a block inside another one is told another norm than that block's)
@@ -45,7 +45,7 @@ class PreNormBlock(Block):
         if isinstance(following, PreNormBlock) and runs_own(following, PreNormBlock, "forward_chain") and getattr(then, "plain", False):
             first = getattr(following.mixer, "input_projection", None)
             proj = first(ctx.following[1]) if first is not None else None
-            if proj is not None and not ops.decode_chain_takes(x, proj):
+            if proj is not None and not ops.decode_chain_takes(x, proj, then.gain):
                 proj = None
         norm = self.feed_forward_norm
         x, product = ops.decode_chain(

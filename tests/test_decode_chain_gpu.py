@@ -100,3 +100,44 @@ def test_a_row_does_not_depend_on_the_others(hidden):
     for rows in (slice(0, 1), slice(7, 8), slice(2, 4), slice(2, 5), slice(1, 5), slice(3, 8)):
         for part, all_rows in zip(run(rows), whole):
             assert torch.equal(part, all_rows[rows])
+
+
+def test_what_lies_between_16_byte_boundaries_goes_to_the_separate_kernels():
+    """A stream or a gain that does not begin on one, as a slice of a longer tensor may, in a block wide enough that the
+    separate kernels take it."""
+    from atomserve_b200 import ops
+    from atomserve_b200.ops.linear import check_gemm_status
+    from atomserve_b200.parts.attention import GQAttention
+    from atomserve_b200.parts.base import StepContext
+    from atomserve_b200.parts.block import PreNormBlock
+    from atomserve_b200.parts.mlp import SwiGLU
+    from atomserve_b200.parts.norms import RMSNorm
+
+    tokens, hidden, heads, hd, ff = 3, 8704, 4, 128, 512
+    v = _inputs(tokens, hidden, heads * hd, ff, 0)
+
+    def shifted(t):  # the same values one element further on
+        return torch.cat([t.new_zeros(1), t.flatten()])[1:].view(t.shape)
+
+    attention = GQAttention(hidden, "", heads, heads, hd, None)
+    attention.o_proj = v["o"]
+    mlp = SwiGLU(hidden, "", ff)
+    mlp.load({"gate_proj.weight": v["gate"], "up_proj.weight": v["up"], "down_proj.weight": v["down"]})
+    norms = [RMSNorm(hidden, "", 1e-6) for _ in range(2)]
+    block = PreNormBlock(attention, mlp, *norms)
+    ids = torch.zeros(tokens, dtype=torch.int32, device="cuda")
+    ctx = StepContext(tokens, tokens, ids, ids, ids, ids, ids, ids, 1)
+    attention.attend = lambda h, ctx, cache, write_cache: v["attn"]
+    want = _plain(v, 1e-6)[0]
+    for x, gain in ((v["x"], v["gains"][0]), (shifted(v["x"]), v["gains"][0]), (v["x"], shifted(v["gains"][0]))):
+        norms[0].gain, norms[1].gain = v["gains"][1], gain
+        aligned = x is v["x"] and gain is v["gains"][0]
+        assert ops.decode_chain_takes(x, v["o"], mlp.gate_up_proj, v["down"], gain) == aligned
+        got = block.forward(x, ctx, None)
+        check_gemm_status()
+        _close(got, want)
+        if not aligned:
+            with pytest.raises(ops.KernelLibraryError):
+                ops.decode_chain(v["attn"], v["o"], x, gain, 1e-6, mlp.gate_up_proj, v["down"], torch.zeros(4, dtype=torch.int32, device="cuda"))
+    strided = torch.stack([v["x"], v["x"]], dim=1)[:, 0]
+    assert not ops.decode_chain_takes(strided, v["o"], mlp.gate_up_proj, v["down"], v["gains"][0])
