@@ -141,3 +141,83 @@ def test_what_lies_between_16_byte_boundaries_goes_to_the_separate_kernels():
                 ops.decode_chain(v["attn"], v["o"], x, gain, 1e-6, mlp.gate_up_proj, v["down"], torch.zeros(4, dtype=torch.int32, device="cuda"))
     strided = torch.stack([v["x"], v["x"]], dim=1)[:, 0]
     assert not ops.decode_chain_takes(strided, v["o"], mlp.gate_up_proj, v["down"], v["gains"][0])
+
+
+LAYERS = 66  # more than the calls whose counters are zeroed together
+
+
+def _model(dtype, schedule):
+    import dataclasses
+
+    import plain_qwen3 as plain
+    from atomserve_b200.config.registry import config_from_dict
+    from atomserve_b200.parts import build_model
+
+    cfg = dict(architectures=["Qwen3ForCausalLM"], vocab_size=384, hidden_size=512, intermediate_size=1024, num_hidden_layers=LAYERS,
+               num_attention_heads=4, num_key_value_heads=2, head_dim=128, rms_norm_eps=1e-6, rope_theta=1e6, tie_word_embeddings=False,
+               max_position_embeddings=512)  # fmt: skip
+    arch, config = config_from_dict(cfg)
+    model = build_model(dataclasses.replace(arch.build_spec(config), schedule=schedule))
+    w = plain.random_checkpoint(cfg, 4)
+    model.load({s.name: (w[s.name] if s.kind == "gain" else w[s.name].bfloat16().to(dtype)).cuda() for s in model.tensor_specs()})
+    return model
+
+
+def _steps(model):
+    """Logits of steps of a model: prompts, then single tokens of three requests (from a graph, three times the same step),
+    a portion of five tokens beside two single ones, eight tokens of one request, and one token."""
+    from atomserve_b200.config import EngineConfig
+    from atomserve_b200.engine.engine import create_engine
+    from atomserve_b200.engine.runner import Row
+
+    engine = create_engine(model, EngineConfig(block_size=16, num_blocks=32, max_num_seqs=4, max_num_batched_tokens=64, max_model_len=256))
+    runner, cache = engine.runner, engine.runner.cache
+    requests, at = [cache.new_request() for _ in range(3)], [0, 0, 0]
+    for rc in requests:
+        assert cache.admit(rc) and cache.reserve(rc, 0, 64)
+    g, logits = torch.Generator().manual_seed(9), []
+
+    def step(lengths, times=1):
+        rows = [Row(torch.randint(0, 384, (n,), generator=g).tolist(), at[i], requests[i], list(range(n))) for i, n in lengths]
+        got = [runner.step(rows).clone() for _ in range(times)]
+        assert all(torch.equal(got[0], again) for again in got)
+        for i, n in lengths:
+            at[i] += n
+        logits.append(got[0])
+
+    step([(0, 20), (1, 13), (2, 17)])
+    step([(0, 1), (1, 1), (2, 1)], times=3)
+    step([(0, 1), (1, 1), (2, 1)], times=3)
+    step([(1, 5), (0, 1), (2, 1)], times=2)
+    step([(2, 8)])
+    step([(0, 1)], times=3)
+    return logits
+
+
+def test_a_model_with_and_without_the_chain(monkeypatch):
+    """A model of more layers than share one zeroing of counters, two of which read another one's keys and values, through
+    the runner, eagerly and from graphs. Both forms are draws of the same rounding noise around the float32 path: the chain's
+    may be at most twice the other's, a step's error measured over all its logits (thousands of values)."""
+    from atomserve_b200 import ops
+    from atomserve_b200.ops import chain
+    from atomserve_b200.ops.linear import check_gemm_status
+    from atomserve_b200.parts import LayerCall
+
+    schedule = tuple(LayerCall(i, cache_from={10: 9, 21: 9}.get(i)) for i in range(LAYERS))
+    exact = _steps(_model(torch.float32, schedule))
+    model, calls, run = _model(torch.bfloat16, schedule), [], ops.decode_chain
+    monkeypatch.setattr(ops, "decode_chain", lambda *args, **kwargs: calls.append(kwargs["next_proj"]) or run(*args, **kwargs))
+    with_chain = _steps(model)
+    check_gemm_status()
+    # the graphs' two shapes are run once for warming up and once captured; of the last layer nothing is handed on
+    eager, captured = 3, 2 * 2
+    assert len(calls) == LAYERS * (eager + captured) and sum(p is None for p in calls) == eager + captured
+    assert {p.shape[0] for p in calls if p is not None} == {4 * 128, 8 * 128}
+    calls.clear()
+    monkeypatch.setattr(chain, "CHAIN", False)
+    without = _steps(model)
+    assert not calls
+    for got, other, want in zip(with_chain, without, exact):
+        error, allowed = (got - want).norm(), (other - want).norm()
+        assert torch.isfinite(got).all() and error <= 2 * allowed, (error / want.norm(), allowed / want.norm())
+    assert torch.equal(with_chain[0], without[0])  # (more tokens than the chain takes)

@@ -7,7 +7,7 @@ import torch
 from atomserve_b200 import ops
 from atomserve_b200.parts import LayerCall, LayerSpec, ModelSpec, PartSpec, StepContext, register_part
 from atomserve_b200.parts.attention import GQAttention
-from atomserve_b200.parts.base import ProjectedInput
+from atomserve_b200.parts.base import ProjectedInput, StreamStep
 from atomserve_b200.parts.block import PreNormBlock
 from atomserve_b200.parts.mlp import SwiGLU
 from atomserve_b200.parts.model import DecoderModel
@@ -211,3 +211,40 @@ def test_every_pass_zeroes_counters_of_its_own(chain, layers):
         words.append({c.untyped_storage().data_ptr(): c.untyped_storage() for c in chain.counters})
         assert len({c.data_ptr() for c in chain.counters}) == layers  # a call's own
     assert not words[0].keys() & words[1].keys()
+
+
+class Halfway(StreamStep):
+    def __init__(self, hidden_size, prefix):
+        pass
+
+    def forward(self, x, x0, number, ctx):
+        return (x + x0) / 2
+
+
+@pytest.mark.parametrize("tokens", [1, 8])
+def test_a_run_order_with_shared_caches_repeated_layers_and_stream_steps(chain, monkeypatch, tokens):
+    """An entry that reads another one's keys and values is handed its queries only; nothing is handed over a stream step."""
+    schedule = [LayerCall(0), LayerCall(1, cache_from=0), LayerCall(2), LayerCall(1), LayerCall(0, before=(0, 1)), LayerCall(2, cache_from=4)]
+    register_part("stream_step", "halfway_of_the_test", Halfway)
+    model = _model(3, schedule, stream_steps=(PartSpec("halfway_of_the_test"),))
+    plain = _off(monkeypatch, model, tokens)
+    assert chain.calls == 0
+    assert torch.allclose(_run(model, tokens), plain, rtol=1e-12, atol=1e-12)
+    assert chain.calls == 6 and chain.handed_on == 4  # not before the stream step, nor at the end
+
+
+def test_more_tokens_than_it_takes(chain, monkeypatch):
+    model = _model(2)
+    assert torch.equal(_run(model, 9), _off(monkeypatch, model, 9)) and chain.calls == 0
+
+
+@pytest.mark.parametrize("what", ["next product", "output", "feed-forward"])
+def test_a_matrix_that_is_not_taken(chain, monkeypatch, what):
+    """The layer before hands on its normed output where the next product is not taken; a layer whose own matrices are not
+    taken runs by itself on what it is handed."""
+    model = _model(3)
+    block = model.blocks[1]
+    chain.refused = [{"next product": block.mixer.qkv_proj, "output": block.mixer.o_proj, "feed-forward": block.feed_forward.down_proj}[what]]
+    plain = _off(monkeypatch, model, 5)
+    assert torch.allclose(_run(model, 5), plain, rtol=1e-12, atol=1e-12)
+    assert (chain.calls, chain.handed_on) == ((3, 1) if what == "next product" else (2, 1))
