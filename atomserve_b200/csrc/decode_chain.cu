@@ -2,8 +2,8 @@
 //
 //   x1 = attn . Wo^T + x;  h = SiLU(N(x1) . Wg^T) * (N(x1) . Wu^T);  x2 = h . Wd^T + x1;  p = N'(x2) . Wqkv^T
 //
-// (atomserve/model.py:336, 354-360, 378-382 and the next layer's :326-329), N the RMS norms. With a few dozen tokens at
-// most, each product is a read of its matrix, and as separate kernels a layer's four products left memory idle for 2 to 3
+// (atomserve/model.py:336, 354-360, 378-382 and the next layer's :326-329), N the RMS norms. With up to 8 tokens, one column
+// of tiles, each product is a read of its matrix, and as separate kernels a layer's four products left memory idle for 2 to 3
 // us at each of nine kernel boundaries. Here the matrices are one stream: every block owns 1 / gridDim of each matrix's
 // rows, and its loader warps walk the block's rows of all four matrices in order through one ring of stages, stopping
 // for nothing but a full ring. Where a product needs what all blocks made of the one before (a grid barrier, about 3 us
@@ -14,7 +14,7 @@
 // rows 1088 bytes apart, so that the fragment reads below meet no bank conflict; a loader issues such a copy every 37 ns,
 // so that four of them stay ahead of memory). The eight multiplying warps share a stage along K, 64 elements each, with
 // the weights as the rows of mma.sync's m16n8k16 and the tokens as its columns: per 14 KB of weights and SM, which memory
-// delivers in some 600 cycles, a warp issues 4 shared loads and 4 mma per 8 tokens. (tcgen05's tiles have 64 or 128 rows:
+// delivers in some 600 cycles, a warp issues 4 shared loads and 4 mma. (tcgen05's tiles have 64 or 128 rows:
 // they would have to be cut along K to give every SM its share of 4096 rows, and the cut sums met again behind one
 // barrier more.) K runs outside, the block's row tiles inside: a token's elements are read once per K step from L2 into
 // registers, a step ahead, multiplied there by the norm's gains where the product's input is a norm's output, and serve
@@ -51,13 +51,14 @@ constexpr int kStepK = 512;          // elements of K per stage, 64 per warp
 constexpr int kPitch = kStepK * 2 + 64;
 constexpr int kStageBytes = kTileRows * kPitch;
 constexpr int kStages = 13;
-constexpr int kMaxTiles = 12;        // row tiles that a warp holds sums of at once (48 registers per 8 tokens)
+constexpr int kMaxTiles = 12;        // row tiles that a warp holds sums of at once (48 registers)
 constexpr int kSumFloats = 5376;     // shared memory in which the warps' sums meet (it follows the ring: a fragment's rows
                                      // past the last stage's lie in it, and belong to no result)
 constexpr uint32_t kBarrierPolls = 1u << 22;
 constexpr int kMaxPhases = 4;
-constexpr int kMaxTokens = 8;
+constexpr int kMaxTokens = 8;        // the columns of a fragment, and one token a warp where the norm's factors are worked out
 constexpr int kMaxBlocks = 160;      // a multiple of 32
+constexpr int kGroup = kSumFloats / (kWarps * kTileRows * kMaxTokens);  // row tiles whose sums meet at once
 
 enum Epilogue : int { kResidual = 0, kSwiglu = 1, kPlain = 2 };
 
@@ -167,18 +168,14 @@ __device__ void load_matrices(const Chain& c, Shared& s, uint32_t ring, int load
   }
 }
 
-// 64 elements of K (this warp's share of a step) of the lane's tokens: element group lane % 4 of each half.
-template <int NT>
-__device__ __forceinline__ void load_tokens(uint4 (&x)[NT][2], const Phase& ph, int tokens, int k, int lane) {
-#pragma unroll
-  for (int nt = 0; nt < NT; ++nt) {
-    const int t = nt * 8 + (lane >> 2);
-    const __nv_bfloat16* at = ph.x + (size_t)t * ph.k + k + (lane & 3) * 8;
-    x[nt][0] = x[nt][1] = make_uint4(0, 0, 0, 0);
-    if (t < tokens) {
-      x[nt][0] = __ldcg(reinterpret_cast<const uint4*>(at));
-      x[nt][1] = __ldcg(reinterpret_cast<const uint4*>(at + 32));
-    }
+// 64 elements of K (this warp's share of a step) of the lane's token: element group lane % 4 of each half.
+__device__ __forceinline__ void load_tokens(uint4 (&x)[2], const Phase& ph, int tokens, int k, int lane) {
+  const int t = lane >> 2;
+  const __nv_bfloat16* at = ph.x + (size_t)t * ph.k + k + (lane & 3) * 8;
+  x[0] = x[1] = make_uint4(0, 0, 0, 0);
+  if (t < tokens) {
+    x[0] = __ldcg(reinterpret_cast<const uint4*>(at));
+    x[1] = __ldcg(reinterpret_cast<const uint4*>(at + 32));
   }
 }
 
@@ -192,19 +189,15 @@ __device__ __forceinline__ void load_gains(float4 (&g)[2][2], const Phase& ph, i
   }
 }
 
-template <int NT>
-__device__ __forceinline__ void scale_tokens(uint4 (&x)[NT][2], const float4 (&gains)[2][2]) {
+__device__ __forceinline__ void scale_tokens(uint4 (&x)[2], const float4 (&gains)[2][2]) {
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     const float* g = reinterpret_cast<const float*>(&gains[h]);
+    __nv_bfloat162* v = reinterpret_cast<__nv_bfloat162*>(&x[h]);
 #pragma unroll
-    for (int nt = 0; nt < NT; ++nt) {
-      __nv_bfloat162* v = reinterpret_cast<__nv_bfloat162*>(&x[nt][h]);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float2 f = __bfloat1622float2(v[i]);
-        v[i] = __floats2bfloat162_rn(f.x * g[2 * i], f.y * g[2 * i + 1]);
-      }
+    for (int i = 0; i < 4; ++i) {
+      const float2 f = __bfloat1622float2(v[i]);
+      v[i] = __floats2bfloat162_rn(f.x * g[2 * i], f.y * g[2 * i + 1]);
     }
   }
 }
@@ -213,7 +206,6 @@ struct Walk {
   int stage, parity;
 };
 
-template <int NT>
 __device__ void multiply_phase(const Chain& c, const Phase& ph, Shared& s, uint32_t ring, float* sums, Walk& walk, float4 (&gains)[2][2],
                                int warp, int lane) {
   const int T = c.tokens, tid = warp * 32 + lane;
@@ -221,19 +213,16 @@ __device__ void multiply_phase(const Chain& c, const Phase& ph, Shared& s, uint3
   // the order of a token's sum is then the same whatever else is in the step (and a block has few rows there: 14 to 18 pairs).
   int columns = ph.epilogue == kResidual ? kMaxTokens : 1;
   while (columns < T) columns *= 2;
-  constexpr int TP = NT * 8;                                      // token columns
-  constexpr int kGroup = kSumFloats / (kWarps * kTileRows * TP);  // row tiles whose sums meet at once
-  constexpr int kOwnTokens = (TP + kWarps - 1) / kWarps;
-  uint4 next[NT][2];
-  load_tokens<NT>(next, ph, T, warp * 64, lane);
-  // The norm's factor of a token multiplies its sums: it is worked out beside the first K step. (This warp's tokens.)
-  float shares[kOwnTokens][kMaxBlocks / 32];
+  constexpr int TP = kMaxTokens;  // token columns
+  static_assert(kMaxTokens <= kWarps, "a warp works out one token's factor");
+  uint4 next[2];
+  load_tokens(next, ph, T, warp * 64, lane);
+  // The norm's factor of a token multiplies its sums: it is worked out beside the first K step. (This warp's token.)
+  float shares[kMaxBlocks / 32];
   if (ph.gain) {
 #pragma unroll
-    for (int j = 0; j < kOwnTokens; ++j)
-#pragma unroll
-      for (int i = 0; i < kMaxBlocks / 32; ++i)
-        shares[j][i] = warp + j * kWarps < T && i * 32 + lane < gridDim.x ? __ldcg(ph.squares_in + (size_t)(warp + j * kWarps) * gridDim.x + i * 32 + lane) : 0.f;
+    for (int i = 0; i < kMaxBlocks / 32; ++i)
+      shares[i] = warp < T && i * 32 + lane < gridDim.x ? __ldcg(ph.squares_in + (size_t)warp * gridDim.x + i * 32 + lane) : 0.f;
   }
   const int begin = first_row(ph.rows, blockIdx.x, gridDim.x), end = first_row(ph.rows, blockIdx.x + 1, gridDim.x);
   const int step = pass_rows(end - begin);
@@ -244,22 +233,18 @@ __device__ void multiply_phase(const Chain& c, const Phase& ph, Shared& s, uint3
   float squares = 0.f;  // of this thread's token, tid % columns
   for (int r0 = begin; r0 < end; r0 += step) {
     const int own = min(end, r0 + step) - r0, tiles = (own + kTileRows - 1) / kTileRows;
-    float acc[kMaxTiles][NT][4];
+    float acc[kMaxTiles][4];
 #pragma unroll
-    for (int m = 0; m < kMaxTiles; ++m)
-#pragma unroll
-      for (int nt = 0; nt < NT; ++nt) acc[m][nt][0] = acc[m][nt][1] = acc[m][nt][2] = acc[m][nt][3] = 0.f;
+    for (int m = 0; m < kMaxTiles; ++m) acc[m][0] = acc[m][1] = acc[m][2] = acc[m][3] = 0.f;
     if (r0 != begin) {
-      load_tokens<NT>(next, ph, T, warp * 64, lane);
+      load_tokens(next, ph, T, warp * 64, lane);
       if (ph.gain) load_gains(gains, ph, warp * 64, lane);
     }
     for (int k0 = 0; k0 < ph.k; k0 += kStepK) {
-      uint4 x[NT][2];
-#pragma unroll
-      for (int nt = 0; nt < NT; ++nt) x[nt][0] = next[nt][0], x[nt][1] = next[nt][1];
-      if (k0 + kStepK < ph.k) load_tokens<NT>(next, ph, T, k0 + kStepK + warp * 64, lane);
+      uint4 x[2] = {next[0], next[1]};
+      if (k0 + kStepK < ph.k) load_tokens(next, ph, T, k0 + kStepK + warp * 64, lane);
       if (ph.gain) {
-        scale_tokens<NT>(x, gains);
+        scale_tokens(x, gains);
         if (k0 + kStepK < ph.k) load_gains(gains, ph, k0 + kStepK + warp * 64, lane);
       }
 #pragma unroll
@@ -272,25 +257,19 @@ __device__ void multiply_phase(const Chain& c, const Phase& ph, Shared& s, uint3
           uint32_t a[4], b[4];  // rows lane / 4 and 8 further on, eight elements of K each: two K steps of the mma
           lds128(a, at + h * 64);
           lds128(b, at + h * 64 + 8 * kPitch);
-#pragma unroll
-          for (int nt = 0; nt < NT; ++nt) {
-            mma16816(acc[m][nt], a[0], b[0], a[1], b[1], x[nt][h].x, x[nt][h].y);
-            mma16816(acc[m][nt], a[2], b[2], a[3], b[3], x[nt][h].z, x[nt][h].w);
-          }
+          mma16816(acc[m], a[0], b[0], a[1], b[1], x[h].x, x[h].y);
+          mma16816(acc[m], a[2], b[2], a[3], b[3], x[h].z, x[h].w);
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&s.empty[walk.stage]));
         if (++walk.stage == kStages) walk.stage = 0, walk.parity ^= 1;
       }
       if (k0 == 0 && r0 == begin && ph.gain) {
+        float v = 0.f;
 #pragma unroll
-        for (int j = 0; j < kOwnTokens; ++j) {
-          float v = 0.f;
-#pragma unroll
-          for (int i = 0; i < kMaxBlocks / 32; ++i) v += shares[j][i];
-          v = asb::warp_sum(v);
-          if (lane == 0 && warp + j * kWarps < T) s.rstd[warp + j * kWarps] = rsqrtf(v / (float)ph.k + ph.eps);
-        }
+        for (int i = 0; i < kMaxBlocks / 32; ++i) v += shares[i];
+        v = asb::warp_sum(v);
+        if (lane == 0 && warp < T) s.rstd[warp] = rsqrtf(v / (float)ph.k + ph.eps);
       }
     }
     // the warps' sums, kGroup row tiles at a time: [warp][row][token]
@@ -302,12 +281,9 @@ __device__ void multiply_phase(const Chain& c, const Phase& ph, Shared& s, uint3
 #pragma unroll
       for (int g = 0; g < kGroup; ++g) {
         if (m0 + g < kMaxTiles) {
-#pragma unroll
-          for (int nt = 0; nt < NT; ++nt) {
-            float* at = mine + (g * kTileRows + (lane >> 2)) * TP + nt * 8 + (lane & 3) * 2;
-            *reinterpret_cast<float2*>(at) = make_float2(acc[m0 + g][nt][0], acc[m0 + g][nt][1]);
-            if ((lane >> 2) + 8 < kTileRows) *reinterpret_cast<float2*>(at + 8 * TP) = make_float2(acc[m0 + g][nt][2], acc[m0 + g][nt][3]);
-          }
+          float* at = mine + (g * kTileRows + (lane >> 2)) * TP + (lane & 3) * 2;
+          *reinterpret_cast<float2*>(at) = make_float2(acc[m0 + g][0], acc[m0 + g][1]);
+          if ((lane >> 2) + 8 < kTileRows) *reinterpret_cast<float2*>(at + 8 * TP) = make_float2(acc[m0 + g][2], acc[m0 + g][3]);
         }
       }
       sync_multipliers();
@@ -376,7 +352,6 @@ __device__ void grid_barrier(const Chain& c, Shared& s, int index, int tid) {
   sync_multipliers();
 }
 
-template <int NT>
 __global__ void __launch_bounds__(kThreads, 1) decode_chain_kernel(const __grid_constant__ Chain c) {
   extern __shared__ __align__(128) unsigned char memory[];
   float* sums = reinterpret_cast<float*>(memory + kStages * kStageBytes);
@@ -393,6 +368,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_chain_kernel(const __grid_
   }
   __syncthreads();
   if (warp >= kWarps) {
+    // (128 x 40 + 256 x 224 = 62,464 registers, of the 384 x 168 = 64,512 that the block is launched with)
     asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
     load_matrices(c, s, ring, warp - kWarps, lane);  // weights: no kernel writes them, so nothing is waited for
   } else {
@@ -409,7 +385,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_chain_kernel(const __grid_
       float4 gains[2][2];  // of the first K step: they wait for no other block
       if (c.phase[p].gain) load_gains(gains, c.phase[p], warp * 64, lane);
       if (p) grid_barrier(c, s, p - 1, threadIdx.x);
-      multiply_phase<NT>(c, c.phase[p], s, ring, sums, walk, gains, warp, lane);
+      multiply_phase(c, c.phase[p], s, ring, sums, walk, gains, warp, lane);
     }
   }
   __syncthreads();
@@ -467,9 +443,8 @@ extern "C" int asb_decode_chain(const void* attn, const void* wo, const void* x,
   c.tokens = tokens;
   c.arrived = arrived;
   c.status = status;
-  auto kernel = decode_chain_kernel<1>;
-  const cudaError_t set = cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSharedBytes);
+  const cudaError_t set = cudaFuncSetAttribute((const void*)decode_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSharedBytes);
   if (set != cudaSuccess) return asb::fail("decode_chain: %s", cudaGetErrorString(set));
-  if (const int refused = asb::launch_cooperative(kernel, blocks, kThreads, kSharedBytes, stream, c)) return refused;
+  if (const int refused = asb::launch_cooperative(decode_chain_kernel, blocks, kThreads, kSharedBytes, stream, c)) return refused;
   return asb::check_launch("decode_chain");
 }

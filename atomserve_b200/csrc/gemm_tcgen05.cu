@@ -592,44 +592,6 @@ int stage_room(int bn_kernel) {
   }
 }
 
-// How a shape is run. One block runs per SM (or one pair of blocks per pair of SMs).
-//
-// Up to 128 tokens the operands swap (weights fill the 128-row MMA, tokens are its N = 16..256)
-// always for up to 32 tokens, and beyond where the unswapped tiles of 128 x 256 would leave over
-// half of the SMs idle (few weight rows: qkv, o, down); where they fill the machine (gate/up, the
-// head) whole unswapped tiles win from 33 tokens on (measured on the 8B and 14B shapes).
-//
-// With more than 128 tokens the forms are compared by an estimate of their time in microseconds,
-// a fixed part plus rounds of tiles times K blocks times the form's time per K block, with
-// constants fitted to the twelve projection shapes of Qwen3-8B, -14B and -32B at 200 to 2,048
-// tokens (over those 84 cases the estimate's choice is within 0.1 % of the best form's time
-// summed, and never more than 2 % behind it on one):
-//   unswapped tiles of 128 tokens by bn weight rows, bn a multiple of 32 from 64 to 256 (the
-//     epilogue reads 32 columns at a time): up to 128 rows in the 128-column kernel (six stages),
-//     wider ones in the 256-column kernel with as many stages as fit; an SM's time per K block
-//     goes with the bytes it takes in, so narrower tiles that occupy more SMs win where wide
-//     ones leave SMs idle, as long as they need no further round;
-//   tiles of 256 tokens by 128 to 256 weight rows (in steps of 32) on pairs of SMs (gemm_tcgen05_pair.cu), whose
-//     last round can be cut along K: twice the arithmetic per byte taken in, so with enough
-//     tiles to fill the device the 256-row tile wins (gate/up at 2,048 tokens: 339 -> 268 us, the
-//     vendor library 284), and the 128-row tile where there are few weight rows and a few
-//     hundred tokens (o at 512 tokens on the 14B shape: 34.5 -> 27.6 us);
-//   tiles of 256 weight rows by 32 to 256 tokens on pairs of SMs (gemm_tcgen05_pair.cu, swapped), where one round holds
-//     all tiles: tokens are rounded up to 32 a tile only, and few tiles are cut along K. Qwen3-8B: down at 302 tokens
-//     44.5 -> 33.4 us, at 384 45.1 -> 36.6; o at 160 17.5 -> 14.1. (More rounds would pay for an
-//     epilogue that writes 64 bytes a token and warp: gate/up at 302 tokens 66.2 us in three rounds, 67.9 without.)
-//   swapped operands with the flattened K-block sequence cut into equal ranges, up to 512 tokens:
-//     the partial sums cost about 14 us, which only long K over few tokens repays (down at 200).
-// With 17 to 32 tokens and more than one round of those pair tiles whose rest can be cut (gate/up), the pair tiles also
-// take the place of the swapped single-SM form: gate/up of Qwen3-8B at 32 tokens 41.9 -> 39.2 us, 151,936 rows of 2,048 110.3
-// -> 101.0 (at 16 tokens nothing is gained). With 33 to 64 tokens they do so only for the activated form (`glu`), whose
-// epilogue the narrow unswapped tiles take longer over, from 5/4 rounds of tiles and 4,096 elements of K on: 24,576 rows
-// of 4,096 at 48 tokens 42.0 -> 40.2 us (a step of Qwen3-8B with 64 requests 6,660 -> 6,525), 32,768 of 5,120 60.0 -> 57.3.
-// Below, the unswapped tiles are narrower still (20,480 of 4,096 at 64: 37.4 against 40.2 us; 24,576 of 2,048: 25.7, 28.0), and without
-// the activation they win throughout (20,480 of 4,096: 33.0 against 36.3; 24,576: 36.7 against 39.5).
-// With swapped operands, whole tiles are dealt round-robin unless cutting the flattened K-block
-// sequence into equal ranges shortens the busiest SM's share of the operand stream by more than
-// the partial sums cost to write and read back; unswapped single-SM tiles are never cut.
 // What a product with the activated epilogue takes in a form, in microseconds, as fitted to the calls of a sweep of every
 // form and width (gate/up of 12,288 to 51,200 rows, the other projections with an epilogue of their own, 136 to 2,048
 // tokens; off by 7 % in the mean): a start, the busiest SM's K blocks, what each round's epilogue adds, and where the last
@@ -666,6 +628,45 @@ double activated_us(bool swapped, bool pair, int bn, int M, int N, int K) {
   return us > memory ? us : memory;
 }
 
+// How a shape is run. One block runs per SM (or one pair of blocks per pair of SMs).
+//
+// Up to 128 tokens the operands swap (weights fill the 128-row MMA, tokens are its N = 16..256)
+// always for up to 32 tokens, and beyond where the unswapped tiles of 128 x 256 would leave over
+// half of the SMs idle (few weight rows: qkv, o, down); where they fill the machine (gate/up, the
+// head) whole unswapped tiles win from 33 tokens on (measured on the 8B and 14B shapes).
+//
+// With more than 128 tokens the forms are compared by an estimate of their time in microseconds,
+// a fixed part plus rounds of tiles times K blocks times the form's time per K block, with
+// constants fitted to the twelve projection shapes of Qwen3-8B, -14B and -32B at 200 to 2,048
+// tokens (over those 84 cases the estimate's choice is within 0.1 % of the best form's time
+// summed, and never more than 2 % behind it on one):
+//   unswapped tiles of 128 tokens by bn weight rows, bn a multiple of 32 from 64 to 256 (the
+//     epilogue reads 32 columns at a time): up to 128 rows in the 128-column kernel (six stages),
+//     wider ones in the 256-column kernel with as many stages as fit; an SM's time per K block
+//     goes with the bytes it takes in, so narrower tiles that occupy more SMs win where wide
+//     ones leave SMs idle, as long as they need no further round;
+//   tiles of 256 tokens by 128 to 256 weight rows (in steps of 32) on pairs of SMs (gemm_tcgen05_pair.cu), whose
+//     last round can be cut along K: twice the arithmetic per byte taken in, so with enough
+//     tiles to fill the device the 256-row tile wins (gate/up at 2,048 tokens: 339 -> 268 us, the
+//     vendor library 284), and the 128-row tile where there are few weight rows and a few
+//     hundred tokens (o at 512 tokens on the 14B shape: 34.5 -> 27.6 us);
+//   tiles of 256 weight rows by 32 to 256 tokens on pairs of SMs (gemm_tcgen05_pair.cu, swapped), where one round holds
+//     all tiles: tokens are rounded up to 32 a tile only, and few tiles are cut along K. Qwen3-8B: down at 302 tokens
+//     44.5 -> 33.4 us, at 384 45.1 -> 36.6; o at 160 17.5 -> 14.1. (More rounds pay for an epilogue that writes 64 bytes a
+//     token and warp: gate/up at 302 tokens 66.2 us in three rounds, 67.9 without. Activated products of matrices that no one
+//     round holds take them where activated_us says so.)
+//   swapped operands with the flattened K-block sequence cut into equal ranges, up to 512 tokens:
+//     the partial sums cost about 14 us, which only long K over few tokens repays (down at 200).
+// With 17 to 32 tokens and more than one round of those pair tiles whose rest can be cut (gate/up), the pair tiles also
+// take the place of the swapped single-SM form: gate/up of Qwen3-8B at 32 tokens 41.9 -> 39.2 us, 151,936 rows of 2,048 110.3
+// -> 101.0 (at 16 tokens nothing is gained). With 33 to 64 tokens they do so only for the activated form (`glu`), whose
+// epilogue the narrow unswapped tiles take longer over, from 5/4 rounds of tiles and 4,096 elements of K on: 24,576 rows
+// of 4,096 at 48 tokens 42.0 -> 40.2 us (a step of Qwen3-8B with 64 requests 6,660 -> 6,525), 32,768 of 5,120 60.0 -> 57.3.
+// Below, the unswapped tiles are narrower still (20,480 of 4,096 at 64: 37.4 against 40.2 us; 24,576 of 2,048: 25.7, 28.0), and without
+// the activation they win throughout (20,480 of 4,096: 33.0 against 36.3; 24,576: 36.7 against 39.5).
+// With swapped operands, whole tiles are dealt round-robin unless cutting the flattened K-block
+// sequence into equal ranges shortens the busiest SM's share of the operand stream by more than
+// the partial sums cost to write and read back; unswapped single-SM tiles are never cut.
 Plan make_plan(int M, int N, int K, bool glu) {
   Plan pl;
   const int sms_now = sm_count();
@@ -743,7 +744,7 @@ Plan make_plan(int M, int N, int K, bool glu) {
   // a product with a residual reads and writes 64 bytes a token and warp in this form; and at 400 tokens gate/up of
   // 32B won 6 % alone and nothing in a step.)
   if (glu && M > BM && M <= kWideTokens && wide_tiles > all_pairs && !pl.swap && g_force_swap < 0) {
-    double best = 0.95 * activated_us(pl.wide > 0, pl.pair > 0, pl.wide ? pl.wide : (pl.pair ? pl.pair : pl.bn), M, N, K);
+    double best = 0.95 * activated_us(false, pl.pair > 0, pl.pair ? pl.pair : pl.bn, M, N, K);  // (one round of pairs holds no such matrix)
     for (int bn = 64; bn <= 256; bn += 32) {
       const double us = activated_us(true, false, bn, M, N, K);
       if (us < best) { best = us; pl.pair = 0; pl.wide = bn; }

@@ -64,6 +64,7 @@ __device__ __forceinline__ uint32_t mbar_try(uint32_t bar, uint32_t parity) {
 // not with a lane's number: the instructions take warp-uniform operands, and here the compiler knows that one lane runs. With
 // a branch on the lane the products bound by their issuing thread took longer: o [4096, 4096] on pairs at 512 tokens 18.3
 // -> 16.5 us, down [4096, 12288] 45.9 -> 42.7, gate/up [51200, 5120] at 302 172.6 -> 158.9; the others stay as they were.
+// (The attention kernels' loader warps issue a tile's copies from several lanes at once and wait in one that shares its result.)
 __device__ __forceinline__ bool elect_one() {
   uint32_t elected;
   asm volatile(

@@ -357,6 +357,62 @@ def time_gemms(which: str, tokens: list[int], steps: int) -> None:
         del ws
 
 
+def time_chain(sizes: list[tuple[int, int, int, int]], tokens: list[int], pk: dict) -> None:
+    """Device time of a layer's products from attention's output to the next layer's qkv, as one kernel (`ops.decode_chain`)
+    and as separate ones, from a CUDA graph of 32 layers over four layers' matrices in turn (more than L2 holds from a hidden
+    size of 1,536 on). sizes: (hidden, attention's width, feed-forward, rows of the next product). One JSON line a case."""
+    import torch
+
+    from atomserve_b200 import ops
+    from atomserve_b200.ops.linear import check_gemm_status
+    from atomserve_b200.parts.norms import RMSNorm
+
+    layers, copies = 32, 4
+    for hidden, attn_k, ff, rows in sizes:
+        def matrix(n, k):
+            return (torch.randn(n, k, device="cuda") * k**-0.5).bfloat16()
+
+        weights = [(matrix(hidden, attn_k), matrix(2 * ff, hidden), matrix(hidden, ff), matrix(rows, hidden)) for _ in range(copies)]
+        norm = RMSNorm(hidden, "", 1e-6)
+        norm.gain = torch.ones(hidden, device="cuda")
+        for T in tokens:
+            attn, x = (torch.randn(T, n, device="cuda").bfloat16() for n in (attn_k, hidden))
+
+            def separate():
+                for i in range(layers):
+                    o, gate_up, down, proj = weights[i % copies]
+                    x1, h = norm.after_linear(attn, o, x)
+                    _, h = norm.after_linear(ops.linear_swiglu(h, gate_up), down, x1)
+                    ops.linear_partial(h, proj)  # (the rotary kernel adds its sums up)
+
+            def chain():
+                arrived = torch.zeros(layers, 4, dtype=torch.int32, device="cuda")
+                for i in range(layers):
+                    o, gate_up, down, proj = weights[i % copies]
+                    ops.decode_chain(attn, o, x, norm.gain, norm.eps, gate_up, down, arrived[i], norm.gain, norm.eps, proj)
+
+            line = {"chain": [hidden, attn_k, ff, rows], "tokens": T}
+            for name, fn in (("separate_us", separate), ("chain_us", chain)):
+                fn()
+                torch.cuda.synchronize()
+                graph = torch.cuda.CUDAGraph()
+                with torch.cuda.graph(graph):
+                    fn()
+                times = []
+                for _ in range(6):
+                    start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+                    start.record()
+                    graph.replay()
+                    end.record()
+                    torch.cuda.synchronize()
+                    times.append(start.elapsed_time(end) * 1000 / layers)
+                check_gemm_status()
+                line[name] = round(sorted(times[1:])[2], 1)
+            line["matrices_us"] = round(2 * (hidden * attn_k + 3 * ff * hidden + rows * hidden) / pk["hbm_gbs"] / 1e3, 1)
+            print(json.dumps(line))
+        del weights
+
+
 def attention_range_sweep(batches: list[int], contexts: list[int]) -> None:
     """Device time of the decode attention kernel plus its merge against the number of ranges that all rows' keys are cut
     into (0: whole rows, no merge), per (batch, context), at the 8B shape's heads; one JSON line each, with what the
@@ -1421,15 +1477,15 @@ def main() -> int:
                         help="fewer layers than the model has (same layer sizes), where time or memory needs it")  # fmt: skip
     parser.add_argument("--batch", type=int, default=8)
     parser.add_argument("--impl", default="ours", choices=["ours", "reference"])
-    parser.add_argument("--only", choices=["decode", "prefill", "gemm", "serve", "attention", "sampling", "designs", "zogepel", "tigesun", "nipurax", "lidizen", "vilulix"], help="time just this (for profiling small cases and the other shapes)")
-    parser.add_argument("--shape", default="8b", choices=sorted(SHAPES), help="with --only decode/prefill/serve: layer sizes of Qwen3-8B, -14B or -32B")
+    parser.add_argument("--only", choices=["decode", "prefill", "gemm", "chain", "serve", "attention", "sampling", "designs", "zogepel", "tigesun", "nipurax", "lidizen", "vilulix"], help="time just this (for profiling small cases and the other shapes)")
+    parser.add_argument("--shape", default="8b", choices=sorted(SHAPES), help="with --only decode/prefill/serve/chain: layer sizes of Qwen3-8B, -14B or -32B")
     parser.add_argument("--context", type=int, default=PROMPT_TOKENS, help="with --only decode: tokens each request holds when decoding starts")
     parser.add_argument("--requests", type=int, default=32, help="with --only serve: requests submitted at once")
     parser.add_argument("--decode-tokens", type=int, default=256, help="with --only serve: tokens generated per request")
     parser.add_argument("--budget", type=int, default=512, help="with --only serve: the scheduler's token budget per step")
     parser.add_argument("--gemm-shape", default="all", help="with --only gemm: qkv, o, gate_up, down, lm_head or all")
-    parser.add_argument("--gemm-tokens", default="1,8,64,2048", help="with --only gemm: token counts, comma-separated")
-    parser.add_argument("--widths", default="2048,4096", help="with --only designs, zogepel, tigesun, nipurax, lidizen or vilulix: model widths, comma-separated")
+    parser.add_argument("--gemm-tokens", default="1,8,64,2048", help="with --only gemm or chain (up to 8): token counts, comma-separated")
+    parser.add_argument("--widths", default="2048,4096", help="with --only chain (in the shape's place: attention as wide, three times that between), designs, zogepel, tigesun, nipurax, lidizen or vilulix: model widths, comma-separated")
     parser.add_argument("--timeline", action="store_true", help="with --only gemm: where a decode-size call's time goes")
     args = parser.parse_args()
     args.layers_given = any(a == "--layers" or a.startswith("--layers=") for a in sys.argv[1:])
@@ -1469,6 +1525,15 @@ def main() -> int:
         return 0
     if args.only == "vilulix":
         time_vilulix([int(w) for w in args.widths.split(",")], args.layers if args.layers_given else 4, max(args.steps // 4, 8), warmup, pk)
+        return 0
+    if args.only == "chain":
+        c, widths = SHAPES[args.shape], []
+        if any(a == "--widths" or a.startswith("--widths=") for a in sys.argv[1:]):
+            widths = [int(w) for w in args.widths.split(",")]
+        heads, hd = c["num_attention_heads"], c["head_dim"]
+        sizes = [(w, w, 3 * w, w * 3 // 2) for w in widths] or [
+            (c["hidden_size"], heads * hd, c["intermediate_size"], (heads + 2 * c["num_key_value_heads"]) * hd)]
+        time_chain(sizes, [t for t in map(int, args.gemm_tokens.split(",")) if t <= 8], pk)
         return 0
     if args.only == "gemm" and args.timeline:
         gemm_timelines(args.gemm_shape, [int(t) for t in args.gemm_tokens.split(",")])
