@@ -94,13 +94,10 @@ class Sampler:
                 self._dev = torch.empty(max(4 * n, 1024), dtype=torch.int64, device=self.device)
             # (filled through numpy: a small tensor a setting, and its copy, took the host 40 us a step)
             host, dev = self._host[turn][: 4 * n], self._dev[: 4 * n]
-            words = host.numpy().reshape(4, n)
-            floats, ints = words[2].view(np.float32), words[3].view(np.int32)
-            words[0] = _numbers("q", [self.seed_of(s) for s in seqs])
-            words[1] = _numbers("q", [len(s.token_ids) - s.num_prompt_tokens + ahead for s in seqs])
-            floats[:n] = _numbers("f", [s.params.temperature for s in seqs])
-            floats[n:] = _numbers("f", [s.params.top_p for s in seqs])
-            ints[:n] = _numbers("i", [s.params.top_k for s in seqs])
+            words = host.numpy()
+            words[: 2 * n] = _numbers("q", [self.seed_of(s) for s in seqs] + [len(s.token_ids) - s.num_prompt_tokens + ahead for s in seqs])
+            words[2 * n : 3 * n].view(np.float32)[:] = _numbers("f", [s.params.temperature for s in seqs] + [s.params.top_p for s in seqs])
+            words[3 * n :].view(np.int32)[:n] = _numbers("i", [s.params.top_k for s in seqs])
             dev.copy_(host, non_blocking=True)
             dev_floats, dev_ints = dev[2 * n : 3 * n].view(torch.float32), dev[3 * n :].view(torch.int32)
             out = ops.sample_rows(logits, dev_floats[:n], dev_ints[:n], dev_floats[n:], dev[:n], dev[n : 2 * n])
