@@ -25,8 +25,8 @@
 // blocks in one order, so that each token's factor is the same everywhere, and the same for any number of tokens.
 //
 // Measured in a CUDA graph of such layers, 1 and 8 tokens, in us, as separate kernels and as one, beside the matrices' time
-// at 6,546 GB/s: Qwen3-8B's sizes 80.3, 82.5 -> 70.9, 73.7 (59.0); 14B's 120.3, 123.3 -> 107.1, 110.7 (100.9); 32B's 165.9,
-// 169.7 -> 151.3, 157.6 (149.0); a hidden size of 512 (1.0) 20.7, 20.9 -> 13.9, 14.5: no size in between was slower, so
+// at 6,549 GB/s: Qwen3-8B's sizes 78.2, 80.5 -> 70.6, 73.4 (58.9); 14B's 118.5, 121.4 -> 106.9, 110.4 (100.9); 32B's 163.5,
+// 167.1 -> 152.3, 157.3 (148.9); a hidden size of 512 (1.0) 18.7, 19.5 -> 13.6, 14.2: no size in between was slower, so
 // the sizes do not decide. What is left: the first product's start, and about 1.5 us at each barrier. Loads held to 84 KB
 // in flight an SM (so that the SMs stay level) were slower, 72 -> 73 us; without the gains' prefetch, the factor's sums
 // beside the first K step and the early residual it took 74.

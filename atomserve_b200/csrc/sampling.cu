@@ -19,15 +19,17 @@
 // leading digit is its exponent and two bits, so that half a row falls into some sixteen bins and its atomics wait for
 // one another, while 2,048 equal steps spread it; and what shares the deciding step is so few (a row of 151,936 has under
 // 200 to a step) that it is gathered and ranked in place of two more passes. Rows with a NaN or an infinity on top, and
-// those with more in one step than the buffer holds, take the digits. 48 rows of 151,936 normal logits, top-p 0.95 alone:
-// 109 -> 83 us, after a top-k of 2,000 139 -> 110; all logits within 0.01 of each other 131 -> 102; only where hundreds of
-// logits are equal at the cut is the histogram of steps one pass more (logits of whole quarters: 205 -> 231).
+// those with more in one step than the buffer holds, take the digits. 48 rows of 151,936 normal logits, top-p 0.95 alone, us:
+// deviation 3 at temperature 0.6 and 0.8 86 -> 64 and 107 -> 80, deviation 1 at 1 132 -> 106, after a top-k of 2,000
+// 140 -> 112; all logits within 0.01 of each other 131 -> 102. Slower: where hundreds of logits are equal at the cut the
+// histogram of steps is one pass more (deviation 1 in whole quarters: 202 -> 228; digits within the deciding step alone
+// took 240), and rows that end in a top-k of 20 by 2 % (40.1 -> 41.0; without their smallest logit 40.7, and the others slower).
 //
 // What bounds it: a row of 151,936 logits is 600 KB, and with one block a row every one of
 // seven passes over it moved at the rate of one SM. Here each block of the cluster brings its share of the row
 // into shared memory once (76 KB, two blocks an SM) and all passes read it there; what is left is the
 // chain of passes with two cluster barriers each. Measured, 1 / 48 rows of 151,936: temperature 0.6, top-k 20, top-p
-// 0.95 122 / 124 -> 17 / 40 us; top-p 0.95 alone 371 / 480 -> 28 / 83 us (the steps included); argmax 8.8 / 8.8 -> 3.8 / 6.5 us. An eighth and not a quarter, because rows in flight on the
+// 0.95 122 / 124 -> 17 / 41 us; top-p 0.95 alone at 0.6 371 / 480 -> 24 / 64 us (the steps included); argmax 8.8 / 8.8 -> 3.8 / 6.5 us. An eighth and not a quarter, because rows in flight on the
 // device are the same (74 KB x 2 against 148 KB x 1 an SM) while a pass takes half as long.
 //
 // Random numbers are Philox-4x32-10 keyed by the row's seed; the counter is (token id, the
