@@ -25,16 +25,22 @@ def chain_limits() -> tuple[int, int]:
 
 def decode_chain_takes(x: torch.Tensor, *weights: torch.Tensor) -> bool:
     """Whether `decode_chain` runs for this residual stream and these weights: matrices (the output, gated and down projections,
-    and any that follow) and norms' gains. Its loads are of 16 bytes; what is laid out otherwise, the separate kernels take."""
+    and any that follow) and norms' gains, or for the stream with some weights. Its loads are of 16 bytes; what is laid out
+    otherwise, the separate kernels take."""
     if not CHAIN or not own_kernels() or x.dtype != torch.bfloat16 or not x.is_cuda:
         return False
     tokens, k_multiple = chain_limits()
-    if not 0 < x.shape[0] <= tokens or not all(t.is_contiguous() and t.data_ptr() % 16 == 0 for t in (x, *weights)):
+    if not 0 < x.shape[0] <= tokens or not x.is_contiguous() or x.data_ptr() % 16:
         return False
-    return all(
-        w.dtype == torch.float32 if w.dim() == 1 else w.dim() == 2 and w.dtype == torch.bfloat16 and w.shape[0] % 2 == 0 and w.shape[1] % k_multiple == 0
-        for w in weights
-    )
+    for w in weights:
+        size = w.shape
+        if len(size) == 2:
+            fits = w.dtype == torch.bfloat16 and size[0] % 2 == 0 and size[1] % k_multiple == 0
+        else:
+            fits = len(size) == 1 and w.dtype == torch.float32
+        if not fits or not w.is_contiguous() or w.data_ptr() % 16:
+            return False
+    return True
 
 
 def decode_chain(

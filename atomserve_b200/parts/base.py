@@ -155,17 +155,15 @@ class StepContext:
     # ends or something else comes between
     following: tuple["Block", bool] | None = None
 
-    # zeroed words of this pass for kernels whose blocks count themselves in, and how many rows of them are taken: None at the
-    # start of every pass, so that a captured pass holds their zeroing whatever ran over this context before
-    counters: tuple[torch.Tensor, int] | None = None
+    # zeroed words of this pass for kernels whose blocks count themselves in: none are left over at the start of a pass, so that
+    # a captured pass holds their zeroing whatever ran over this context before
+    counters: list[torch.Tensor] = field(default_factory=list)
 
     def zeroed_counters(self, device: torch.device) -> torch.Tensor:
         """Four int32 zeros on the device for one call of a kernel (zeroed a few dozen calls at a time, in the current stream)."""
-        words, used = self.counters or (None, 0)
-        if words is None or used == len(words):
-            words, used = torch.zeros(64, 4, dtype=torch.int32, device=device), 0
-        self.counters = (words, used + 1)
-        return words[used]
+        if not self.counters:
+            self.counters = list(torch.zeros(64, 4, dtype=torch.int32, device=device).unbind())
+        return self.counters.pop()
 
     def portions_context(self) -> int:
         """The longest context of the requests that bring more than a few tokens (single tokens beside them may have longer
@@ -201,7 +199,8 @@ class Part:
 def runs_own(part: Part, owner: type, *methods: str) -> bool:
     """Whether `part` runs these methods as `owner` wrote them. A class that offers its weights to a kernel which stands in for
     its methods does so for itself alone: a part that derives from it and changes one of them is run by what it has."""
-    return all(getattr(type(part), m) is getattr(owner, m) and m not in vars(part) for m in methods)
+    kind = type(part)
+    return (kind is owner or all(getattr(kind, m) is getattr(owner, m) for m in methods)) and vars(part).keys().isdisjoint(methods)
 
 
 class Norm(Part):

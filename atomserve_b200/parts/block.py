@@ -32,6 +32,8 @@ class PreNormBlock(Block):
     def _chained(self, x: torch.Tensor, normed, ctx: StepContext, cache: CacheView | None, write_cache: bool, then: Norm | None):
         """With few tokens: all products from the mixer's last to the following block's first as one kernel
         (`ops.decode_chain`), where both blocks are of the kind it knows. None where it does not run."""
+        if not ops.decode_chain_takes(x):  # (most steps: nothing more is asked of the parts)
+            return None
         offered = getattr(self.mixer, "output_projection", None)
         gated = getattr(self.feed_forward, "gated_weights", None)
         output, weights = offered() if offered is not None else None, gated() if gated is not None else None

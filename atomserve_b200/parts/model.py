@@ -95,7 +95,7 @@ class DecoderModel:
         """Run the T tokens of the step; float32 logits [len(ctx.logits_rows), vocab], written
         into `logits_out` where the caller brings the buffer (a head whose `forward` takes no
         `out` has its result copied there)."""
-        ctx.counters = None
+        ctx.counters = []
         if hasattr(self.embedding, "forward_step"):  # an embedding that reads more of the step than its token ids
             x = self.embedding.forward_step(ctx, views[len(self.schedule)] if len(views) > len(self.schedule) else None)
         else:
