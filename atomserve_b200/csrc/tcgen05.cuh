@@ -90,11 +90,6 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
       : "memory");
 }
 
-// The same box requested into L2 only: no shared memory, no barrier, nothing to wait for.
-__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int x, int y) {
-  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
-}
-
 // Shared-memory matrix descriptors for tiles in the 128-byte swizzle, rows of 128 bytes (64
 // 16-bit elements), groups of eight rows 1024 bytes apart. (version 1 at bit 46, layout type 2 =
 // SWIZZLE_128B at bit 61.)
