@@ -25,10 +25,10 @@
 // blocks in one order, so that each token's factor is the same everywhere, and the same for any number of tokens.
 //
 // Measured in a CUDA graph of such layers, 1 and 8 tokens, in us, as separate kernels and as one, beside the matrices' time
-// at 6,549 GB/s: Qwen3-8B's sizes 78.2, 80.5 -> 70.6, 73.4 (58.9); 14B's 118.5, 121.4 -> 106.9, 110.4 (100.9); 32B's 163.5,
-// 167.1 -> 152.3, 157.3 (148.9); a hidden size of 512 (1.0) 18.7, 19.5 -> 13.6, 14.2: no size in between was slower, so
+// at 6,549 GB/s: Qwen3-8B's sizes 78.3, 80.8 -> 70.0, 73.0 (58.9); 14B's 118.7, 121.7 -> 106.8, 110.3 (100.9); 32B's 163.6,
+// 167.0 -> 152.6, 156.8 (148.9); a hidden size of 512 (1.0) 19.2, 19.5 -> 13.5, 14.2: no size in between was slower, so
 // the sizes do not decide. What is left: the first product's start, and about 1.5 us at each barrier. Loads held to 84 KB
-// in flight an SM (so that the SMs stay level) were slower, 72 -> 73 us; without the gains' prefetch, the factor's sums
+// in flight an SM (so that the SMs stay level) were slower, 72 -> 73 us; without the gains' early loads, the factor's sums
 // beside the first K step and the early residual it took 74.
 //
 // Waits are bounded; one that runs out reports through the status word and the block goes on to its end without waiting.
