@@ -373,9 +373,8 @@ __global__ void __launch_bounds__(kThreads, 1) decode_chain_kernel(const __grid_
     load_matrices(c, s, ring, warp - kWarps, lane);  // weights: no kernel writes them, so nothing is waited for
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
-    // A load from every line of the gains, for nothing but to have them in L2 before their first product reads them. (Loads and
-    // not prefetches: a kernel that prefetched memory into L2 before its wait, and a process that ran this one so, ended in a
-    // launch failure at a new model's step; no address was out of range. 70.6 -> 70.0 us at Qwen3-8B's sizes.)
+    // A load from every line of the gains, for nothing but to have them in L2 before their first product reads them. (With
+    // prefetches in their place 70.6 us at Qwen3-8B's sizes instead of 70.0.)
     for (int p = 0; p < c.phases; ++p)
       if (c.phase[p].gain)
         for (int i = threadIdx.x * 32; i < c.phase[p].k; i += kWarps * 32 * 32) {
